@@ -621,6 +621,18 @@ struct step_counts
 // that differs between tiles.  Only keys whose home group is full of other keys (or whose claim lost
 // to another key) take the tile-cooperative slow path.
 
+// Ends a warp step: the lanes leave it together.  Without this barrier the lanes that lost a claim, or took the
+// slow path, left the step on their own and the compiler let them run into the next step's code in parts, up to
+// its first shuffle: the instructions after the divergence were issued once per part.  Measured for bulk inserts
+// with and without it (one box, kernel time): 2^20 keys into a set<u32> of capacity 2^21 36 against 65 us, 2.5 M
+// keys into a set<u64> of capacity 2^22 73 against 161 us, 5.2 M keys into a map<u64,u64> of capacity 8 M (DRAM)
+// 174 against 219 us.
+SG_D void
+step_end()
+{
+    __syncwarp();
+}
+
 SG_D unsigned
 tile_nibble(unsigned ballot, int tbase)
 {
@@ -774,6 +786,7 @@ insert_kv_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::
             out_flags[i] = static_cast<uint8_t>(res == 1);
         }
     }
+    step_end();
 }
 
 template <int KIND, bool AOS>
@@ -895,6 +908,7 @@ erase_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::
             out_flags[i] = static_cast<uint8_t>(res);
         }
     }
+    step_end();
 }
 
 // Erase step whose compare-and-swap result is consumed one step later: the swap of step k stays in flight
@@ -994,6 +1008,7 @@ find_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K
             }
         }
     }
+    step_end();
 }
 
 template <int KIND, bool WANT_VALUES>
