@@ -61,9 +61,6 @@ struct unordered_ref
     static constexpr int SPL = C::slots_per_lane;
 
     sg_unordered_view v;
-    // A bulk kernel's per-thread counts: the header counters' changes accumulate here, to be added once per
-    // block, instead of one atomic per key on each counter (nullptr: every call updates the header).
-    detail::call_counts* defer = nullptr;
 
     // d (+-1) added to a header counter by the lanes of the warp that run this call together: one atomic
     // per group of converged lanes instead of one per lane on the same address (the counters' updates are
@@ -84,53 +81,25 @@ struct unordered_ref
     __device__ __forceinline__ void
     add_size(int d) const
     {
-        if (defer != nullptr)
-        {
-            defer->size += d;
-        }
-        else
-        {
-            warp_add(&header()->size, d);
-        }
+        warp_add(&header()->size, d);
     }
 
     __device__ __forceinline__ void
     add_tombs(int d) const
     {
-        if (defer != nullptr)
-        {
-            defer->tombs += d;
-        }
-        else
-        {
-            warp_add(&header()->tombstones, d);
-        }
+        warp_add(&header()->tombstones, d);
     }
 
     __device__ __forceinline__ void
     add_refused() const
     {
-        if (defer != nullptr)
-        {
-            defer->refused += 1;
-        }
-        else
-        {
-            warp_add(&header()->refused, 1);
-        }
+        warp_add(&header()->refused, 1);
     }
 
     __device__ __forceinline__ void
     add_excess(long long d) const
     {
-        if (defer != nullptr)
-        {
-            defer->excess += d;
-        }
-        else
-        {
-            atomicAdd(&header()->excess_used, static_cast<unsigned long long>(d));
-        }
+        atomicAdd(&header()->excess_used, static_cast<unsigned long long>(d));
     }
 
     __device__ __forceinline__ detail::table_header*
@@ -644,11 +613,6 @@ struct unordered_ref
         {
             return 1;
         }
-        if (defer != nullptr)
-        {
-            defer->excess += 1; // a bulk call that cannot reach the end of the list: counted at its end
-            return 0;
-        }
         if (atomicAdd(&header()->excess_used, 1ull) < static_cast<unsigned long long>(v.excess_count))
         {
             return 0;
@@ -891,91 +855,6 @@ struct unordered_ref
         return result;
     }
 
-    // Insert of a bulk call with the accounting on that cannot reach the refusal (the caller checked that the
-    // size and the keys in excess slots stay below their limits whatever the call does) and runs no erase:
-    // no lock, as in the bulk kernels -- only free slots disappear during the launch, and each insert reads
-    // every slot before the one it claims, so a key is stored once.  The stored copy then takes its bucket's
-    // own slot when it is the bucket's first new key (first_new) and the slot is free, else an excess slot.
-    __device__ int64_t
-    insert_slot_quiet(key_type key, mapped_type mapped, int64_t b, bool first_new) const
-    {
-        int64_t slot = -1;
-        if (is_special(key))
-        {
-            const int s = key == C::empty_key ? 0 : 1;
-            if (atomicCAS(&header()->special_state[s], 0u, 2u) != 0u)
-            {
-                return -1;
-            }
-            store_slot(special_slot(key), key, mapped);
-            __threadfence();
-            atomicExch(&header()->special_state[s], 1u);
-            slot = special_slot(key);
-        }
-        else
-        {
-            const int64_t home = detail::group_of_bucket(static_cast<uint64_t>(b), v.bucket_bits, v.num_groups);
-            for (int attempt = 0; attempt < 65536 && slot < 0; ++attempt)
-            {
-                int64_t target = -1;
-                bool target_tomb = false;
-                // the first read with the warp (all lanes arrive here together in a bulk kernel's step)
-                if (attempt == 0 ? scan_for_insert_warp(key, home, target, target_tomb)
-                                 : scan_for_insert(key, home, target, target_tomb))
-                {
-                    return -1; // present
-                }
-                if (target < 0)
-                {
-                    add_refused();
-                    return -1;
-                }
-                uint32_t image[4];
-                if (target_tomb)
-                {
-                    read_slot(target, image);
-                    if (detail::key_in_lane<KIND>(make_uint4(image[0], image[1], image[2], image[3]), 0) != C::tomb_key)
-                    {
-                        continue; // taken since the scan
-                    }
-                }
-                else
-                {
-                    image[0] = image[1] = image[2] = image[3] = ~0u;
-                }
-                key_type old;
-                if (detail::claim_slot_image<KIND>(slot_ptr(target), image, key, mapped, old))
-                {
-                    if (target_tomb)
-                    {
-                        add_tombs(-1);
-                    }
-                    slot = target;
-                }
-                else if (old == key)
-                {
-                    return -1;
-                }
-            }
-            if (slot < 0)
-            {
-                atomicOr(&header()->error, detail::kErrRetry);
-                return -1;
-            }
-        }
-        add_size(1);
-        const unsigned bit = 1u << (b & 31);
-        if (first_new && (atomicOr(v.bucket_heads + (b >> 5), bit) & bit) == 0u)
-        {
-            mark_bucket_slot(slot);
-        }
-        else
-        {
-            add_excess(1);
-        }
-        return slot;
-    }
-
     // insert_slot for a key of bucket b; may_take_bucket as in take_bucket_or_excess (accounting only).
     __device__ int64_t
     insert_slot_bucket(key_type key, mapped_type mapped, int64_t b, bool may_take_bucket = true) const
@@ -1126,43 +1005,6 @@ struct unordered_ref
     erase_hashed(key_type key, uint64_t hash) const
     {
         return erase_bucket(key, static_cast<int64_t>(detail::fibonacci_bucket(hash, v.bucket_bits)));
-    }
-
-    // Erase of a bulk erase call with the accounting on: no insert runs in the launch, so no lock -- the slot's
-    // bit is read after the swap that erased the key, which only one erase of a key wins.
-    __device__ int64_t
-    erase_quiet(key_type key, int64_t b) const
-    {
-        const int64_t slot = find_slot_warp(
-                key, detail::group_of_bucket(static_cast<uint64_t>(b), v.bucket_bits, v.num_groups), nullptr);
-        if (slot < 0)
-        {
-            return 0;
-        }
-        if (is_special(key))
-        {
-            if (atomicCAS(&header()->special_state[key == C::empty_key ? 0 : 1], 1u, 0u) != 1u)
-            {
-                return 0;
-            }
-        }
-        else if (cas_key(slot, key, C::tomb_key) == key)
-        {
-            add_tombs(1);
-        }
-        else
-        {
-            return 0;
-        }
-        add_size(-1);
-        release(b, unmark_bucket_slot(slot));
-        return 1;
-    }
-
-    __device__ __forceinline__ int64_t
-    erase_quiet_hashed(key_type key, uint64_t hash) const
-    {
-        return erase_quiet(key, static_cast<int64_t>(detail::fibonacci_bucket(hash, v.bucket_bits)));
     }
 
     // erase under the accounting: the stripe lock of the key's home group, then the slot's bits.

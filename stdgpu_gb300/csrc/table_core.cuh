@@ -413,14 +413,15 @@ group_mask(unsigned sector_mask, int q, unsigned mask)
 
 // Insert of one key by one tile (all 4 lanes call it with the same key; w is this lane's sector of the
 // key's home group).  Returns 1 inserted, 0 already present, 2 refused (no free slot in the table),
-// 3 retry limit.  With REUSE, erased slots are claimed too: the tile scans to the first group holding a
+// 3 retry limit; where is the slot it was inserted in.  With REUSE, erased slots are claimed too: the tile scans to the first group holding a
 // never-used slot (so a copy of the key stored beyond an erased slot is seen) and claims the first free
 // slot of the probe sequence.  Free slots only disappear during an insert launch, so two inserts of one
 // key cannot both succeed: each has read every slot before the one it claims.
 template <int KIND, bool REUSE>
 SG_D int
 tile_insert(const dview& t, typename kind_consts<KIND>::K key, typename kind_consts<KIND>::V val, uint32_t home,
-            uint32_t (&w)[8], unsigned tmask, int tbase, int q, unsigned int& tombs_reused, uint32_t rot)
+            uint32_t (&w)[8], unsigned tmask, int tbase, int q, unsigned int& tombs_reused, uint32_t rot,
+            uint32_t& where)
 {
     using C = kind_consts<KIND>;
     using K = typename C::K;
@@ -490,6 +491,7 @@ tile_insert(const dview& t, typename kind_consts<KIND>::K key, typename kind_con
         old = __shfl_sync(tmask, old, tbase);
         if (old == expected)
         {
+            where = target;
             return 1;
         }
         if (old == key)
@@ -659,13 +661,14 @@ load_homes(const dview& t, const tile_lanes& L, uint64_t hash, bool probe, uint3
 // slot of the group (when the group also has a never-used slot) else of the first never-used slot, made
 // by the key's own lane with one compare-and-swap -- 32 claims in flight per warp.
 // The step over keys already in registers (key / val of lane element i, meaningful when valid; hashes as
-// in the loading steps below).
+// in the loading steps below).  Returns what became of the lane's key: 1 inserted (into slot), 0 present,
+// 2 refused, 3 retry limit.
 // GIVEN: the caller passes the key's hash in given_hash (a staged element that carries it).
-template <int KIND, bool GIVEN = false>
-SG_D void
-insert_kv_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K key,
-               typename kind_consts<KIND>::V val, int64_t i, bool valid, uint8_t* out_flags, step_counts& c,
-               const uint64_t* hashes = nullptr, uint64_t given_hash = 0)
+template <int KIND, bool GIVEN>
+SG_D int
+insert_kv_place(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K key,
+                typename kind_consts<KIND>::V val, int64_t i, bool valid, step_counts& c, const uint64_t* hashes,
+                uint64_t given_hash, uint32_t& slot)
 {
     using C = kind_consts<KIND>;
     using K = typename C::K;
@@ -678,7 +681,12 @@ insert_kv_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::
         val = V{};
     }
     const bool special = valid && key >= C::tomb_key;
-    int res = special ? special_insert<KIND>(t, key, val) : 0;
+    int res = 0;
+    if (special)
+    {
+        res = special_insert<KIND>(t, key, val);
+        slot = t.num_groups * G + (key == C::empty_key ? 0u : 1u);
+    }
     const bool probe = valid && !special;
     uint32_t hr[kTile];
     uint32_t pre[kTile][8];
@@ -721,6 +729,7 @@ insert_kv_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::
         {
             c.reused += my_tomb ? 1u : 0u;
             res = 1;
+            slot = my_target;
         }
         else if (old != key)
         {
@@ -736,11 +745,12 @@ insert_kv_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::
                 while (rest != 0u)
                 {
                     const uint32_t s = static_cast<uint32_t>(first_from<G>(rest, my_rot));
-                    const uint32_t slot = gbase + s;
+                    const uint32_t next = gbase + s;
                     rest &= ~(1u << s);
-                    if (claim_slot<KIND>(t, slot, false, key, val, old))
+                    if (claim_slot<KIND>(t, next, false, key, val, old))
                     {
                         res = 1;
+                        slot = next;
                         again = false;
                         break;
                     }
@@ -768,14 +778,28 @@ insert_kv_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::
                 uint32_t w[8];
                 load_sector(t, hr[r], L.q, w);
                 const uint32_t rot = __shfl_sync(L.tmask, my_rot, L.tbase + r);
-                const int x = tile_insert<KIND, true>(t, kr, vr, hr[r], w, L.tmask, L.tbase, L.q, c.reused, rot);
+                uint32_t where = 0;
+                const int x =
+                        tile_insert<KIND, true>(t, kr, vr, hr[r], w, L.tmask, L.tbase, L.q, c.reused, rot, where);
                 if (L.q == r)
                 {
                     res = x;
+                    slot = where;
                 }
             }
         }
     }
+    return res;
+}
+
+template <int KIND, bool GIVEN = false>
+SG_D void
+insert_kv_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K key,
+               typename kind_consts<KIND>::V val, int64_t i, bool valid, uint8_t* out_flags, step_counts& c,
+               const uint64_t* hashes = nullptr, uint64_t given_hash = 0)
+{
+    uint32_t slot = 0;
+    const int res = insert_kv_place<KIND, GIVEN>(t, L, key, val, i, valid, c, hashes, given_hash, slot);
     if (valid)
     {
         c.done += (res == 1);

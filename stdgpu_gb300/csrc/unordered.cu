@@ -43,11 +43,36 @@ bit_set(const uint32_t* words, int64_t i)
 
 // ---------------------------------------------------------------- kernels
 
+// The arrays of the excess-list accounting that an empty table starts from (units 0: the accounting is off).
+struct accounting_init
+{
+    uint4* zeros; // bucket_heads and slot_heads, one after the other: no slot taken
+    int64_t zero_units;
+    uint4* ones; // bucket_cand: no candidate
+    int64_t one_units;
+};
+
+// Words of a counted bulk insert (k_counted_*), in the 256 bytes that the device header is given of its own,
+// behind its fields.  All zero between calls.
+struct counted_control
+{
+    unsigned long long absent; // keys of the call that are not stored
+    unsigned long long heads;  // buckets that get their first new key while their own slot is free
+    unsigned int done_blocks;  // blocks of the candidate pass that have added theirs
+    unsigned int mode;         // how the call inserts (kCounted*)
+};
+constexpr size_t kCountedControlOffset = 128;
+static_assert(sizeof(table_header) <= kCountedControlOffset &&
+                      kCountedControlOffset + sizeof(counted_control) <= 256,
+              "the control words lie behind the header's fields");
+
 // Fills every slot with the never-used marker and the slots at or above total_count with the erased
-// marker; resets the header.  clear(): unordered_base_detail.cuh:1220-1252 (one launch instead of four).
+// marker; resets the header and the accounting's arrays.  clear(): unordered_base_detail.cuh:1220-1252, one
+// launch instead of four.  A small table's clear is bound by its launches: with the accounting's arrays reset by
+// four memsets before this kernel a clear at capacity 1000 took 8.9 us (back to back on the device), now 4.1.
 template <int KIND>
 __global__ void __launch_bounds__(kThreads)
-k_init(dview t)
+k_init(dview t, accounting_init acc)
 {
     using C = kind_consts<KIND>;
     using K = typename C::K;
@@ -74,6 +99,22 @@ k_init(dview t)
                 }
             }
             base[u] = d;
+        }
+    }
+    if (acc.zero_units != 0)
+    {
+        for (int64_t u = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; u < acc.zero_units; u += stride)
+        {
+            acc.zeros[u] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        for (int64_t u = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; u < acc.one_units; u += stride)
+        {
+            acc.ones[u] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+        {
+            *reinterpret_cast<counted_control*>(reinterpret_cast<char*>(t.hdr) + kCountedControlOffset) =
+                    counted_control{};
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -832,112 +873,199 @@ k_erase(dview t, const void* keys, int64_t n, uint8_t* out_flags, const uint64_t
     block_add<2>(v, dst);
 }
 
-// Bulk insert / erase of a table with the reference's excess-list accounting on: one thread per key through
-// the device calls (sg::unordered_ref), which order the keys of one bucket under its stripe lock -- the
-// reference's per-key path (insert_value / erase_from_key, unordered_base_detail.cuh:470-522).  The result
-// is the reference's on one thread, which takes the keys in input order:
-//  * k_counted_candidates first finds, per bucket, the smallest input index of a key not stored yet -- in
+// Bulk insert / erase of a table with the reference's excess-list accounting on (insert_value /
+// erase_from_key, unordered_base_detail.cuh:470-522).  The result is the reference's on one thread, which takes
+// the keys in input order:
+//  * the candidate pass first finds, per bucket, the smallest input index of a key not stored yet -- in
 //    input order the first new key of that bucket, the one that takes the bucket's own slot if it is free;
-//    every other new key takes an excess slot (and a later pass resets the candidates);
-//  * a call of at most kCountedInOrderMax keys runs as one block, and when it could reach the refusal (the
-//    excess list or the table could run out within it), one thread takes its keys in input order, so which
-//    keys are refused is the same too.  A larger call that could reach it refuses keys in launch order.
+//    every other new key takes an excess slot (and a last pass resets the candidates);
+//  * the pass also bounds what the call can add.  A call that cannot reach the refusal (the excess list or the
+//    table running out) inserts as the other bulk calls do, with the warp steps of table_core.cuh: no locks,
+//    since in an insert-only launch free slots only disappear.  Each new key then takes its bucket's own slot or
+//    an excess slot, and the counters are added once per block;
+//  * a call that could reach it goes one thread per key through the device calls (sg::unordered_ref), which order
+//    the keys of one bucket under its stripe lock.  Of at most kCountedInOrderMax keys, one thread takes all in
+//    input order, so which keys are refused is the same too; a larger call refuses keys in launch order.
 constexpr int64_t kCountedInOrderMax = 4096;
 constexpr uint32_t kNoCandidate = 0xFFFFFFFFu;
+constexpr unsigned int kCountedQuiet = 0u;     // warp steps, no locks
+constexpr unsigned int kCountedImmediate = 1u; // one thread per key, stripe locks
+constexpr unsigned int kCountedInOrder = 2u;   // one thread
 
-template <int KIND>
-SG_D int64_t
-counted_bucket(const sg_unordered_view& v, typename kind_consts<KIND>::K key, const uint64_t* hashes, int64_t i)
+// A call of at most this many keys runs its three passes in one launch, a cluster of blocks with hardware
+// barriers between the passes: such a call is bound by its launches (4.1 us each, back to back) and by the chain
+// of dependent reads.  700 keys, capacity 1000: one cluster 10.2 us; a memset and three launches, the inserts one
+// thread per key in one block and every key racing for its group's first free slot, 21.0 us.  Above it, the three
+// launches: 45 K keys of a map<u32,u32> 16.4 us, 22.2 us before with the memset and one thread per key.  The line
+// is the size up to which a call that could reach the refusal takes its keys in input order; the largest call
+// below it gives each thread of the cluster two keys.
+constexpr int kCountedClusterBlocks = 8;
+constexpr int64_t kCountedClusterMax = 4096;
+
+SG_D counted_control*
+counted_words(table_header* h)
 {
-    const uint64_t h = hashes != nullptr ? __ldg(hashes + i) : identity_word_hash{}(key);
-    return static_cast<int64_t>(fibonacci_bucket(h, v.bucket_bits));
+    return reinterpret_cast<counted_control*>(reinterpret_cast<char*>(h) + kCountedControlOffset);
 }
 
-// reset false: candidate per bucket (atomic minimum of the input indices of keys not stored); true: back to none.
+SG_D void
+cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Hash of input element i (the caller's, or the key word).
+template <int KIND>
+SG_D uint64_t
+counted_hash(typename kind_consts<KIND>::K key, const uint64_t* hashes, int64_t i)
+{
+    return hashes != nullptr ? __ldg(hashes + i) : identity_word_hash{}(key);
+}
+
+// Pass 1: candidate per bucket (atomic minimum of the input indices of keys not stored) and the call's bounds.
 template <int KIND, bool AOS>
-__global__ void __launch_bounds__(kThreads)
-k_counted_candidates(sg_unordered_view v, const void* in0, const void* in1, int64_t n, const uint64_t* hashes,
-                     uint32_t* cand, bool reset)
+SG_D void
+counted_candidates(const dview& t, const sg_unordered_view& v, const void* in0, const void* in1, int64_t n,
+                   const uint64_t* hashes, uint32_t* cand)
 {
     using C = kind_consts<KIND>;
-    const sg::unordered_ref<KIND> ref{ v };
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    const tile_lanes L;
+    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     unsigned long long absent = 0, heads = 0;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+    for (int64_t base = warp * 32; base < n; base += nwarps * 32)
     {
-        typename C::K key;
-        typename C::V val;
-        load_input<KIND, AOS>(in0, in1, i, key, val);
-        const int64_t b = counted_bucket<KIND>(v, key, hashes, i);
-        if (reset)
+        const int64_t i = base + L.lane;
+        const bool valid = i < n;
+        typename C::K key = C::empty_key;
+        typename C::V val{};
+        uint64_t hash = 0;
+        if (valid)
         {
-            cand[b] = kNoCandidate;
+            load_input<KIND, AOS>(in0, in1, i, key, val);
+            hash = counted_hash<KIND>(key, hashes, i);
         }
-        else if (ref.find_slot_home(key, group_of_bucket(static_cast<uint64_t>(b), v.bucket_bits, v.num_groups)) < 0)
+        const bool special = valid && key >= C::tomb_key;
+        typename C::V found{};
+        const int32_t slot = locate_step<KIND, false>(t, L, key, hash, valid && !special, found);
+        if (valid && (special ? !special_find<KIND>(t, key, found) : slot < 0))
         {
-            // bounds for k_insert_counted: keys not stored (copies counted each), buckets that get a first new
-            // key while their own slot is free
+            // keys not stored (copies counted each), buckets that get a first new key while their own slot is free
+            const int64_t b = static_cast<int64_t>(fibonacci_bucket(hash, v.bucket_bits));
             ++absent;
             if (atomicMin(cand + b, static_cast<uint32_t>(i)) == kNoCandidate && !bit_set(v.bucket_heads, b))
             {
                 ++heads;
             }
         }
+        step_end();
     }
-    if (!reset)
-    {
-        unsigned long long c[2] = { absent, heads };
-        unsigned long long* const dst[2] = { &ref.header()->count, &ref.header()->scratch };
-        block_add<2>(c, dst);
-    }
+    counted_control* w = counted_words(t.hdr);
+    unsigned long long c[2] = { absent, heads };
+    unsigned long long* const dst[2] = { &w->absent, &w->heads };
+    block_add<2>(c, dst);
 }
 
-// The header counters' changes of a block's threads, added once.
-SG_D void
-flush_counts(table_header* h, const call_counts& c)
+// How a call whose candidate pass is complete inserts (one thread of a block; single: at most
+// kCountedInOrderMax keys).
+SG_D unsigned int
+counted_mode(const sg_unordered_view& v, const table_header* h, bool single)
 {
-    unsigned long long v[4] = { static_cast<unsigned long long>(c.size), static_cast<unsigned long long>(c.tombs),
-                                static_cast<unsigned long long>(c.refused), static_cast<unsigned long long>(c.excess) };
-    unsigned long long* const dst[4] = { &h->size, &h->tombstones, &h->refused, &h->excess_used };
-    block_add<4>(v, dst);
+    const counted_control* w = counted_words(const_cast<table_header*>(h));
+    const unsigned long long used = __ldcg(&h->excess_used);
+    const unsigned long long size = __ldcg(&h->size);
+    const unsigned long long absent = __ldcg(&w->absent), heads = __ldcg(&w->heads);
+    const bool quiet = used + (absent - heads) < static_cast<unsigned long long>(v.excess_count) &&
+                       size + absent < static_cast<unsigned long long>(v.total_count);
+    return quiet ? kCountedQuiet : (single ? kCountedInOrder : kCountedImmediate);
 }
 
+// Whether the key is its bucket's candidate (any copy of it): the bucket's own slot is for that key.
 template <int KIND, bool AOS>
-__global__ void __launch_bounds__(kThreads)
-k_insert_counted(sg_unordered_view v, const void* in0, const void* in1, int64_t n, uint8_t* out_flags,
-                 const uint64_t* hashes, const uint32_t* cand)
+SG_D bool
+counted_first_new(const void* in0, const void* in1, const uint32_t* cand, int64_t b, typename kind_consts<KIND>::K key)
+{
+    const uint32_t c = __ldcg(cand + b);
+    if (c == kNoCandidate)
+    {
+        return false;
+    }
+    typename kind_consts<KIND>::K ck;
+    typename kind_consts<KIND>::V cv;
+    load_input<KIND, AOS>(in0, in1, static_cast<int64_t>(c), ck, cv);
+    return ck == key;
+}
+
+// Header changes of a thread of pass 2.
+struct counted_changes
+{
+    step_counts c;
+    unsigned int excess = 0; // new keys in excess slots
+};
+
+// Pass 2.  Quiet: every key of the block's warps through the warp step; the changes are left to the caller to add
+// (counted_flush), after every block has read the header.
+template <int KIND, bool AOS>
+SG_D counted_changes
+counted_insert(const dview& t, const sg_unordered_view& v, const void* in0, const void* in1, int64_t n,
+               uint8_t* out_flags, const uint64_t* hashes, const uint32_t* cand, unsigned int mode)
 {
     using C = kind_consts<KIND>;
-    sg::unordered_ref<KIND> ref{ v };
-    // quiet: the call cannot reach the refusal -- it adds at most `absent` keys (k_counted_candidates), of which
-    // at least `heads` take their buckets' own slots -- so it needs no lock and adds the counters at each
-    // block's end (a block that starts after another block's flush sees larger counters and may take the
-    // immediate path, which is always right)
-    __shared__ int mode; // 0 quiet, 1 immediate, 2 in input order (one thread)
-    if (threadIdx.x == 0)
+    counted_changes ch;
+    if (mode == kCountedQuiet)
     {
-        const table_header* h = ref.header();
-        const unsigned long long used = *reinterpret_cast<const volatile unsigned long long*>(&h->excess_used);
-        const unsigned long long size = *reinterpret_cast<const volatile unsigned long long*>(&h->size);
-        const unsigned long long absent = h->count, heads = h->scratch;
-        const bool quiet = used + (absent - heads) < static_cast<unsigned long long>(v.excess_count) &&
-                           size + absent < static_cast<unsigned long long>(v.total_count);
-        mode = quiet ? 0 : (gridDim.x == 1 ? 2 : 1);
+        const tile_lanes L;
+        const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+        const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+        for (int64_t base = warp * 32; base < n; base += nwarps * 32)
+        {
+            const int64_t i = base + L.lane;
+            const bool valid = i < n;
+            typename C::K key = C::empty_key;
+            typename C::V val{};
+            uint64_t hash = 0;
+            if (valid)
+            {
+                load_input<KIND, AOS>(in0, in1, i, key, val);
+                hash = counted_hash<KIND>(key, hashes, i);
+            }
+            uint32_t slot = 0;
+            const int res = insert_kv_place<KIND, true>(t, L, key, val, i, valid, ch.c, nullptr, hash, slot);
+            if (valid)
+            {
+                ch.c.done += (res == 1);
+                ch.c.refused += (res == 2);
+                ch.c.retry += (res == 3);
+                if (out_flags != nullptr)
+                {
+                    out_flags[i] = static_cast<uint8_t>(res == 1);
+                }
+                if (res == 1)
+                {
+                    // the stored copy takes its bucket's own slot or an excess slot
+                    const int64_t b = static_cast<int64_t>(fibonacci_bucket(hash, v.bucket_bits));
+                    const unsigned bit = 1u << (b & 31);
+                    if (counted_first_new<KIND, AOS>(in0, in1, cand, b, key) &&
+                        (atomicOr(v.bucket_heads + (b >> 5), bit) & bit) == 0u)
+                    {
+                        atomicOr(v.slot_heads + (slot >> 5), 1u << (slot & 31));
+                    }
+                    else
+                    {
+                        ch.excess += 1;
+                    }
+                }
+            }
+            step_end();
+        }
+        return ch;
     }
-    __syncthreads();
+    sg::unordered_ref<KIND> ref{ v };
     int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    call_counts counts;
-    if (mode == 0)
+    if (mode == kCountedInOrder)
     {
-        ref.defer = &counts;
-    }
-    if (mode == 2)
-    {
-        if (threadIdx.x != 0)
-        {
-            return;
-        }
+        first = first == 0 ? 0 : n;
         stride = 1;
     }
     for (int64_t i = first; i < n; i += stride)
@@ -945,52 +1073,184 @@ k_insert_counted(sg_unordered_view v, const void* in0, const void* in1, int64_t 
         typename C::K key;
         typename C::V val;
         load_input<KIND, AOS>(in0, in1, i, key, val);
-        const int64_t b = counted_bucket<KIND>(v, key, hashes, i);
-        // the bucket's own slot is for its candidate key (any copy of it)
-        const uint32_t c = cand[b];
-        bool first_new = false;
-        if (c != kNoCandidate)
-        {
-            typename C::K ck;
-            typename C::V cv;
-            load_input<KIND, AOS>(in0, in1, static_cast<int64_t>(c), ck, cv);
-            first_new = ck == key;
-        }
-        const int64_t slot = mode == 0 ? ref.insert_slot_quiet(key, val, b, first_new)
-                                       : ref.insert_slot_bucket(key, val, b, first_new);
+        const int64_t b = static_cast<int64_t>(fibonacci_bucket(counted_hash<KIND>(key, hashes, i), v.bucket_bits));
+        const int64_t slot =
+                ref.insert_slot_bucket(key, val, b, counted_first_new<KIND, AOS>(in0, in1, cand, b, key));
         if (out_flags != nullptr)
         {
             out_flags[i] = static_cast<uint8_t>(slot >= 0);
         }
     }
-    if (mode == 0)
-    {
-        flush_counts(ref.header(), counts);
-    }
+    return ch;
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(kThreads)
-k_erase_counted(sg_unordered_view v, const void* keys, int64_t n, uint8_t* out_flags, const uint64_t* hashes)
+SG_D void
+counted_flush(table_header* h, const counted_changes& ch)
 {
-    using K = typename kind_consts<KIND>::K;
-    // an erase-only launch: no lock (erase_quiet), and no insert reads the counters meanwhile, so they are
-    // added at the block's end
-    call_counts counts;
-    sg::unordered_ref<KIND> ref{ v };
-    ref.defer = &counts;
+    if (ch.c.retry != 0)
+    {
+        atomicOr(&h->error, kErrRetry);
+    }
+    unsigned long long x[4] = { ch.c.done, 0ull - ch.c.reused, ch.c.refused, ch.excess };
+    unsigned long long* const dst[4] = { &h->size, &h->tombstones, &h->refused, &h->excess_used };
+    block_add<4>(x, dst);
+}
+
+// Pass 3: no candidates, the control words zero (one block's thread).
+template <int KIND, bool AOS>
+SG_D void
+counted_reset(const sg_unordered_view& v, table_header* h, const void* in0, const void* in1, int64_t n,
+              const uint64_t* hashes, uint32_t* cand)
+{
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
     {
-        const K key = __ldg(static_cast<const K*>(keys) + i);
-        const int64_t r = hashes != nullptr ? ref.erase_quiet_hashed(key, __ldg(hashes + i))
-                                            : ref.erase_quiet(key, ref.bucket(key));
-        if (out_flags != nullptr)
+        typename kind_consts<KIND>::K key;
+        typename kind_consts<KIND>::V val;
+        load_input<KIND, AOS>(in0, in1, i, key, val);
+        cand[fibonacci_bucket(counted_hash<KIND>(key, hashes, i), v.bucket_bits)] = kNoCandidate;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        *counted_words(h) = counted_control{};
+    }
+}
+
+// The three passes as launches of their own.
+template <int KIND, bool AOS>
+__global__ void __launch_bounds__(kThreads, SG_BULK_MIN_BLOCKS)
+k_counted_candidates(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n, const uint64_t* hashes,
+                     uint32_t* cand)
+{
+    counted_candidates<KIND, AOS>(t, v, in0, in1, n, hashes, cand);
+    // block_add's additions come from threads 0 and 1; the block that is last to add decides for the call
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        __threadfence();
+        counted_control* w = counted_words(t.hdr);
+        if (atomicAdd(&w->done_blocks, 1u) == gridDim.x - 1)
         {
-            out_flags[i] = static_cast<uint8_t>(r);
+            __threadfence();
+            w->mode = counted_mode(v, t.hdr, n <= kCountedInOrderMax);
         }
     }
-    flush_counts(ref.header(), counts);
+}
+
+template <int KIND, bool AOS>
+__global__ void __launch_bounds__(kThreads, 3)
+k_insert_counted(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n, uint8_t* out_flags,
+                 const uint64_t* hashes, const uint32_t* cand)
+{
+    const unsigned int mode = __ldcg(&counted_words(t.hdr)->mode);
+    const counted_changes ch = counted_insert<KIND, AOS>(t, v, in0, in1, n, out_flags, hashes, cand, mode);
+    if (mode == kCountedQuiet)
+    {
+        counted_flush(t.hdr, ch);
+    }
+}
+
+template <int KIND, bool AOS>
+__global__ void __launch_bounds__(kThreads)
+k_counted_reset(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n, const uint64_t* hashes,
+                uint32_t* cand)
+{
+    counted_reset<KIND, AOS>(v, t.hdr, in0, in1, n, hashes, cand);
+}
+
+// The three passes of a small call in one launch: one cluster, a barrier between the passes.
+template <int KIND, bool AOS>
+__global__ void __launch_bounds__(kThreads)
+k_insert_counted_cluster(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n,
+                         uint8_t* out_flags, const uint64_t* hashes, uint32_t* cand)
+{
+    __shared__ unsigned int s_mode;
+    counted_candidates<KIND, AOS>(t, v, in0, in1, n, hashes, cand);
+    __syncthreads();
+    __threadfence();
+    cluster_barrier(); // every block's candidates and bounds are there
+    if (threadIdx.x == 0)
+    {
+        s_mode = counted_mode(v, t.hdr, n <= kCountedInOrderMax);
+    }
+    __syncthreads();
+    const unsigned int mode = s_mode;
+    cluster_barrier(); // every block has read the header; the immediate path changes it from here on
+    const counted_changes ch = counted_insert<KIND, AOS>(t, v, in0, in1, n, out_flags, hashes, cand, mode);
+    __syncwarp();
+    cluster_barrier(); // every block has read its candidates
+    if (mode == kCountedQuiet)
+    {
+        counted_flush(t.hdr, ch);
+    }
+    counted_reset<KIND, AOS>(v, t.hdr, in0, in1, n, hashes, cand);
+}
+
+// Bulk erase with the accounting on: an erase-only launch, so no lock, and no insert reads the counters meanwhile.
+// A slot's bit is read after the swap that erased its key, which one erase of a key wins.
+template <int KIND>
+__global__ void __launch_bounds__(kThreads, SG_BULK_MIN_BLOCKS)
+k_erase_counted(dview t, sg_unordered_view v, const void* keys, int64_t n, uint8_t* out_flags, const uint64_t* hashes)
+{
+    using C = kind_consts<KIND>;
+    using K = typename C::K;
+    const tile_lanes L;
+    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    step_counts c;
+    unsigned long long excess = 0;
+    for (int64_t base = warp * 32; base < n; base += nwarps * 32)
+    {
+        const int64_t i = base + L.lane;
+        const bool valid = i < n;
+        K key = C::empty_key;
+        uint64_t hash = 0;
+        if (valid)
+        {
+            key = __ldg(static_cast<const K*>(keys) + i);
+            hash = counted_hash<KIND>(key, hashes, i);
+        }
+        const bool special = valid && key >= C::tomb_key;
+        typename C::V dummy{};
+        int32_t slot = locate_step<KIND, false>(t, L, key, hash, valid && !special, dummy);
+        int res = 0;
+        if (special)
+        {
+            res = special_erase<KIND>(t, key);
+            c.oob += static_cast<unsigned int>(res);
+            slot = static_cast<int32_t>(t.num_groups * C::slots_per_group + (key == C::empty_key ? 0u : 1u));
+        }
+        else if (slot >= 0)
+        {
+            res = cas_key<KIND>(t, static_cast<uint32_t>(slot), key, C::tomb_key) == key ? 1 : 0;
+        }
+        if (valid)
+        {
+            c.done += static_cast<unsigned int>(res);
+            if (out_flags != nullptr)
+            {
+                out_flags[i] = static_cast<uint8_t>(res);
+            }
+            if (res == 1)
+            {
+                // the bucket's own slot becomes free, or the key's excess slot goes back
+                const unsigned sbit = 1u << (slot & 31);
+                if ((atomicAnd(v.slot_heads + (slot >> 5), ~sbit) & sbit) != 0u)
+                {
+                    const int64_t b = static_cast<int64_t>(fibonacci_bucket(hash, v.bucket_bits));
+                    atomicAnd(v.bucket_heads + (b >> 5), ~(1u << (b & 31)));
+                }
+                else
+                {
+                    ++excess;
+                }
+            }
+        }
+        step_end();
+    }
+    unsigned long long x[3] = { 0ull - c.done, c.done - c.oob, 0ull - excess };
+    unsigned long long* const dst[3] = { &t.hdr->size, &t.hdr->tombstones, &t.hdr->excess_used };
+    block_add<3>(x, dst);
 }
 
 // Bulk find / contains (device-only find/contains in the reference, :619-706).
@@ -1617,7 +1877,17 @@ struct do_init
     {
         static const int max_grid = persistent_grid(k_init<KIND>, kThreads);
         const int64_t units = (t->num_groups + 1) * (kGroupBytes / 16);
-        k_init<KIND><<<grid_for(units, kThreads, max_grid), kThreads, 0, s>>>(view_of(t));
+        accounting_init acc{};
+        if (t->bucket_heads != nullptr)
+        {
+            acc.zeros = reinterpret_cast<uint4*>(t->bucket_heads);
+            acc.zero_units = static_cast<int64_t>(bucket_heads_bytes(t->bucket_count) +
+                                                  slot_heads_bytes(t->num_groups, t->slot_bytes)) /
+                             16;
+            acc.ones = reinterpret_cast<uint4*>(t->bucket_cand);
+            acc.one_units = static_cast<int64_t>(bucket_cand_bytes(t->bucket_count)) / 16;
+        }
+        k_init<KIND><<<grid_for(units, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), acc);
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -1755,17 +2025,42 @@ insert_counted(sg_unordered* t, const void* in0, const void* in1, int64_t n, uin
     {
         return SG_ERR_BAD_ARG; // candidates are 32-bit input indices
     }
+    const dview d = view_of(t);
     const sg_unordered_view v = public_view(t);
+    if (n <= kCountedClusterMax)
+    {
+        int blocks = 1;
+        while (blocks < kCountedClusterBlocks && static_cast<int64_t>(blocks) * kThreads < n)
+        {
+            blocks <<= 1;
+        }
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = static_cast<unsigned>(blocks);
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+        cfg.blockDim = dim3(kThreads);
+        cfg.stream = s;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        SG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_insert_counted_cluster<KIND, AOS>, d, v, in0, in1, n, flags, hashes,
+                                       t->bucket_cand));
+        SG_LAUNCH_CHECK();
+        return SG_OK;
+    }
     static const int g_cand = persistent_grid(k_counted_candidates<KIND, AOS>, kThreads);
     static const int g_ins = persistent_grid(k_insert_counted<KIND, AOS>, kThreads);
-    const int grid_cand = grid_for(n, kThreads, g_cand);
-    SG_CUDA_TRY(cudaMemsetAsync(&t->hdr->count, 0, 2 * sizeof(unsigned long long), s));
-    k_counted_candidates<KIND, AOS><<<grid_cand, kThreads, 0, s>>>(v, in0, in1, n, hashes, t->bucket_cand, false);
+    static const int g_reset = persistent_grid(k_counted_reset<KIND, AOS>, kThreads);
+    k_counted_candidates<KIND, AOS><<<grid_for(n, kThreads, g_cand), kThreads, 0, s>>>(d, v, in0, in1, n, hashes,
+                                                                                      t->bucket_cand);
     SG_LAUNCH_CHECK();
-    const int grid = n <= kCountedInOrderMax ? 1 : grid_for(n, kThreads, g_ins);
-    k_insert_counted<KIND, AOS><<<grid, kThreads, 0, s>>>(v, in0, in1, n, flags, hashes, t->bucket_cand);
+    k_insert_counted<KIND, AOS><<<grid_for(n, kThreads, g_ins), kThreads, 0, s>>>(d, v, in0, in1, n, flags, hashes,
+                                                                                 t->bucket_cand);
     SG_LAUNCH_CHECK();
-    k_counted_candidates<KIND, AOS><<<grid_cand, kThreads, 0, s>>>(v, in0, in1, n, hashes, t->bucket_cand, true);
+    k_counted_reset<KIND, AOS><<<grid_for(n, kThreads, g_reset), kThreads, 0, s>>>(d, v, in0, in1, n, hashes,
+                                                                                  t->bucket_cand);
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -1863,8 +2158,8 @@ struct do_erase
         if (t->bucket_heads != nullptr)
         {
             static const int max_grid = persistent_grid(k_erase_counted<KIND>, kThreads);
-            k_erase_counted<KIND><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(public_view(t), keys, n, flags,
-                                                                                      hashes);
+            k_erase_counted<KIND><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), public_view(t), keys,
+                                                                                      n, flags, hashes);
             SG_LAUNCH_CHECK();
             return SG_OK;
         }
@@ -2120,6 +2415,7 @@ reset_accounting(sg_unordered* t, cudaStream_t s)
     SG_CUDA_TRY(cudaMemsetAsync(t->slot_heads, 0, slot_heads_bytes(t->num_groups, t->slot_bytes), s));
     SG_CUDA_TRY(cudaMemsetAsync(t->bucket_cand, 0xFF, bucket_cand_bytes(t->bucket_count), s));
     SG_CUDA_TRY(cudaMemsetAsync(&t->hdr->excess_used, 0, sizeof(unsigned long long), s));
+    SG_CUDA_TRY(cudaMemsetAsync(reinterpret_cast<char*>(t->hdr) + kCountedControlOffset, 0, sizeof(counted_control), s));
     return SG_OK;
 }
 
@@ -2188,10 +2484,6 @@ create_table(int32_t kind, int64_t capacity, const object_allocator& oa, void* s
     if (e == cudaSuccess)
     {
         e = cudaMemsetAsync(t->locks, 0, static_cast<size_t>(t->lock_count) * sizeof(unsigned int), as_stream(stream));
-    }
-    if (e == cudaSuccess && accounting && reset_accounting(t, as_stream(stream)) != SG_OK)
-    {
-        e = cudaErrorUnknown;
     }
     if (e != cudaSuccess)
     {
@@ -2605,8 +2897,7 @@ sg_unordered_clear(sg_unordered* t, void* stream)
     {
         return SG_ERR_BAD_ARG;
     }
-    const sg_status st = reset_accounting(t, as_stream(stream));
-    return st != SG_OK ? st : dispatch<do_init>(t->kind, t, as_stream(stream));
+    return dispatch<do_init>(t->kind, t, as_stream(stream));
 }
 
 sg_status
