@@ -238,6 +238,11 @@ SG_API sg_status sg_unordered_erase(sg_unordered* table, const void* keys, int64
 SG_API sg_status sg_unordered_find(sg_unordered* table, const void* keys, int64_t n, void* out_mapped, uint8_t* out_found,
                             void* stream);
 
+/* sg_unordered_find (hashes NULL) or sg_unordered_find_hashed (hashes of a custom-hash table) with 0 written as
+ * the mapped value of every absent key: a caller that wants that needs no pass over out_mapped of its own. */
+SG_API sg_status sg_unordered_find_zero(sg_unordered* table, const void* keys, const uint64_t* hashes, int64_t n,
+                            void* out_mapped, uint8_t* out_found, void* stream);
+
 /* Bulk form of the device-only contains(key) / count(key): unordered_base_detail.cuh:595-617, 684-706. */
 SG_API sg_status sg_unordered_contains(sg_unordered* table, const void* keys, int64_t n, uint8_t* out_flags, void* stream);
 

@@ -249,9 +249,9 @@ class unordered_base:
             found = torch.empty(keys.numel(), dtype=torch.uint8, device=keys.device)
             vals = None
             if self.mapped_bytes:
-                vals = torch.zeros(keys.numel(), dtype=_INT_DTYPE[self.mapped_bytes], device=keys.device)
-            N.check(N.load().sg_unordered_find_hashed(self._h, _ptr(keys), self._hashes(hashes, keys.numel()),
-                                                      keys.numel(), _ptr(vals), _ptr(found), _stream(stream)), "find")
+                vals = torch.empty(keys.numel(), dtype=_INT_DTYPE[self.mapped_bytes], device=keys.device)
+            N.check(N.load().sg_unordered_find_zero(self._h, _ptr(keys), self._hashes(hashes, keys.numel()),
+                                                    keys.numel(), _ptr(vals), _ptr(found), _stream(stream)), "find")
             return vals, found
         if not keys.is_cuda:
             st = stager or default_stager()
@@ -264,9 +264,9 @@ class unordered_base:
         found = torch.empty(keys.numel(), dtype=torch.uint8, device=keys.device)
         vals = None
         if self.mapped_bytes:
-            vals = torch.zeros(keys.numel(), dtype=_INT_DTYPE[self.mapped_bytes], device=keys.device)
-        N.check(N.load().sg_unordered_find(self._h, _ptr(keys), keys.numel(), _ptr(vals), _ptr(found),
-                                           _stream(stream)), "find")
+            vals = torch.empty(keys.numel(), dtype=_INT_DTYPE[self.mapped_bytes], device=keys.device)
+        N.check(N.load().sg_unordered_find_zero(self._h, _ptr(keys), None, keys.numel(), _ptr(vals), _ptr(found),
+                                                _stream(stream)), "find")
         return vals, found
 
     def size(self, stream=None) -> int:

@@ -386,15 +386,9 @@ sg_unordered_find_host(sg_unordered* t, sg_stager* sg, const void* keys, int64_t
     }
     void* mo = mb > 0 ? out_mapped : nullptr;
     return staged(sg, sg::detail::as_stream(stream), n, { keys, kb }, { nullptr, 0 }, { mo, mb }, { out_found, 1 },
-                  [t, mb](void* in0, void*, void* out0, uint8_t* out1, int64_t m, cudaStream_t s)
-                  {
-                      // the staging buffer holds an earlier chunk's values: absent keys read back as 0
-                      if (out0 != nullptr)
-                      {
-                          SG_CUDA_TRY(cudaMemsetAsync(out0, 0, static_cast<size_t>(m) * mb, s));
-                      }
-                      return sg_unordered_find(t, in0, m, out0, out1, s);
-                  });
+                  // the staging buffer holds an earlier chunk's values: absent keys read back as 0
+                  [t](void* in0, void*, void* out0, uint8_t* out1, int64_t m, cudaStream_t s)
+                  { return sg_unordered_find_zero(t, in0, nullptr, m, out0, out1, s); });
 }
 
 sg_status

@@ -993,11 +993,13 @@ erase_step(const dview& t, const tile_lanes& L, const void* keys, int64_t i, boo
     erase_key_step<KIND>(t, L, key, i, valid, out_flags, c, hashes);
 }
 
-// Find / contains step.
+// Find / contains step.  zero_absent: an absent key's mapped value is written as 0 (else left alone), so a caller
+// that wants it so needs no pass over the output before the call (which cost 70 us of a 3.73 ms find of 2^27
+// queries, and a launch of 4 us and 16 us of host time before a find of 60 K queries).
 template <int KIND, bool WANT_VALUES>
 SG_D void
 find_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K key, int64_t i, bool valid,
-              void* out_vals, uint8_t* out_found, const uint64_t* hashes = nullptr)
+              void* out_vals, uint8_t* out_found, const uint64_t* hashes = nullptr, bool zero_absent = false)
 {
     using C = kind_consts<KIND>;
     using K = typename C::K;
@@ -1026,9 +1028,9 @@ find_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K
         }
         if constexpr (WANT_VALUES && kind_traits<KIND>::is_map)
         {
-            if (found && out_vals != nullptr)
+            if ((found || zero_absent) && out_vals != nullptr)
             {
-                __stcs(reinterpret_cast<V*>(out_vals) + i, val);
+                __stcs(reinterpret_cast<V*>(out_vals) + i, found ? val : V{});
             }
         }
     }
@@ -1038,11 +1040,11 @@ find_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K
 template <int KIND, bool WANT_VALUES>
 SG_D void
 find_step(const dview& t, const tile_lanes& L, const void* keys, int64_t i, bool valid, void* out_vals,
-          uint8_t* out_found, const uint64_t* hashes = nullptr)
+          uint8_t* out_found, const uint64_t* hashes = nullptr, bool zero_absent = false)
 {
     using K = typename kind_consts<KIND>::K;
     const K key = valid ? __ldcs(reinterpret_cast<const K*>(keys) + i) : kind_consts<KIND>::empty_key;
-    find_key_step<KIND, WANT_VALUES>(t, L, key, i, valid, out_vals, out_found, hashes);
+    find_key_step<KIND, WANT_VALUES>(t, L, key, i, valid, out_vals, out_found, hashes, zero_absent);
 }
 
 } // namespace detail

@@ -1256,7 +1256,8 @@ k_erase_counted(dview t, sg_unordered_view v, const void* keys, int64_t n, uint8
 // Bulk find / contains (device-only find/contains in the reference, :619-706).
 template <int KIND, bool WANT_VALUES>
 __global__ void __launch_bounds__(kThreads, SG_FIND_MIN_BLOCKS)
-k_find(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found, const uint64_t* hashes)
+k_find(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found, const uint64_t* hashes,
+       bool zero_absent)
 {
     const tile_lanes L;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -1264,7 +1265,7 @@ k_find(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found,
     for (int64_t base = warp * 32; base < n; base += nwarps * 32)
     {
         const int64_t i = base + L.lane;
-        find_step<KIND, WANT_VALUES>(t, L, keys, i, i < n, out_vals, out_found, hashes);
+        find_step<KIND, WANT_VALUES>(t, L, keys, i, i < n, out_vals, out_found, hashes, zero_absent);
     }
 }
 
@@ -1281,7 +1282,7 @@ k_find(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found,
 
 template <int KIND, bool WANT_VALUES>
 __global__ void __launch_bounds__(kThreads, SG_FIND_MIN_BLOCKS)
-k_find_staged(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found)
+k_find_staged(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found, bool zero_absent)
 {
     using C = kind_consts<KIND>;
     using K = typename C::K;
@@ -1361,7 +1362,7 @@ k_find_staged(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out
             fence_async_shared();
             issue(it + ST, st);
         }
-        find_key_step<KIND, WANT_VALUES>(t, L, key, i, valid, out_vals, out_found);
+        find_key_step<KIND, WANT_VALUES>(t, L, key, i, valid, out_vals, out_found, nullptr, zero_absent);
     }
 }
 
@@ -2219,7 +2220,7 @@ struct do_find
 {
     static sg_status
     run(sg_unordered* t, const void* keys, int64_t n, void* vals, uint8_t* found, cudaStream_t s,
-        const uint64_t* hashes = nullptr)
+        const uint64_t* hashes = nullptr, bool zero_absent = false)
     {
         if (SG_FIND_STAGE && hashes == nullptr && reinterpret_cast<uintptr_t>(keys) % 16 == 0)
         {
@@ -2227,13 +2228,13 @@ struct do_find
             {
                 static const int max_grid = persistent_grid(k_find_staged<KIND, true>, kThreads);
                 k_find_staged<KIND, true><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), keys, n,
-                                                                                              vals, found);
+                                                                                              vals, found, zero_absent);
             }
             else
             {
                 static const int max_grid = persistent_grid(k_find_staged<KIND, false>, kThreads);
                 k_find_staged<KIND, false><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), keys, n,
-                                                                                               vals, found);
+                                                                                               vals, found, false);
             }
             SG_LAUNCH_CHECK();
             return SG_OK;
@@ -2242,13 +2243,13 @@ struct do_find
         {
             static const int max_grid = persistent_grid(k_find<KIND, true>, kThreads);
             k_find<KIND, true><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), keys, n, vals, found,
-                                                                                   hashes);
+                                                                                   hashes, zero_absent);
         }
         else
         {
             static const int max_grid = persistent_grid(k_find<KIND, false>, kThreads);
             k_find<KIND, false><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), keys, n, vals,
-                                                                                    found, hashes);
+                                                                                    found, hashes, false);
         }
         SG_LAUNCH_CHECK();
         return SG_OK;
@@ -2829,6 +2830,23 @@ sg_unordered_find(sg_unordered* t, const void* keys, int64_t n, void* out_mapped
     }
     const bool is_map = t->kind >= SG_MAP_U64_U32;
     return dispatch<do_find>(t->kind, t, keys, n, is_map ? out_mapped : nullptr, out_found, as_stream(stream));
+}
+
+sg_status
+sg_unordered_find_zero(sg_unordered* t, const void* keys, const uint64_t* hashes, int64_t n, void* out_mapped,
+                       uint8_t* out_found, void* stream)
+{
+    if (t == nullptr || n < 0 || (n > 0 && (keys == nullptr || t->custom_hash != (hashes != nullptr))))
+    {
+        return SG_ERR_BAD_ARG;
+    }
+    if (n == 0)
+    {
+        return SG_OK;
+    }
+    const bool is_map = t->kind >= SG_MAP_U64_U32;
+    return dispatch<do_find>(t->kind, t, keys, n, is_map ? out_mapped : nullptr, out_found, as_stream(stream), hashes,
+                             true);
 }
 
 sg_status

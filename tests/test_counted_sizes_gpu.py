@@ -42,3 +42,34 @@ def test_insert_and_erase_equal_the_oracle(kind, n):
     assert t.size() == 0 and t.t.excess_used() == 0 and t.valid()
     t.close()
     P.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 1000, 70001])
+@pytest.mark.parametrize("kind", [O.MAP_U64_U32, O.MAP_U32_U64, O.MAP_U64_U64])
+def test_absent_keys_read_back_as_zero(kind, n):
+    """find() returns 0 for absent keys whatever its output memory held, the two out-of-band keys included; the C
+    entry point sg_unordered_find leaves them alone."""
+    import torch
+
+    from gpu_util import dev, host
+    from stdgpu_gb300 import _native as N
+
+    kd, vd = O.KEY_DTYPE[kind], O.VAL_DTYPE[kind]
+    t = Table(kind, 4 * n)
+    keys = (np.arange(n).astype(kd) + kd(1)) * kd(2654435761)
+    vals = (keys >> kd(3)).astype(vd)
+    t.insert(keys, vals)
+    top = np.iinfo(kd).max
+    q = np.concatenate([keys[::2], ~keys, np.array([top, top - kd(1)], kd)])
+    stored = np.isin(q, keys)
+    want = np.where(stored, (q >> kd(3)).astype(vd), vd(0)).astype(vd)
+    del_me = torch.full((4 * q.size,), -1, dtype=torch.int64, device="cuda")  # what the allocator hands out next
+    del del_me
+    got, found = t.find(q)
+    assert np.array_equal(found, stored.astype(np.uint8)) and np.array_equal(got, want)
+    out = dev(np.full(q.size, 5, vd))
+    flag = torch.empty(q.size, dtype=torch.uint8, device="cuda")
+    N.check(N.load().sg_unordered_find(t.t._h, dev(q).data_ptr(), q.size, out.data_ptr(), flag.data_ptr(), None), "find")
+    torch.cuda.synchronize()
+    assert np.array_equal(host(out, vd), np.where(stored, want, vd(5)))
+    t.close()
