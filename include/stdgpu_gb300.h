@@ -526,7 +526,8 @@ typedef struct sg_deque_view
  * slot is free (push) or written (pop), the reference's per-slot occupied bit
  * (src/stdgpu/impl/deque_detail.cuh:202-446).  A word of another epoch has not been touched since the last
  * bulk call: its slot is occupied exactly when its ticket lay in [base_begin, base_end) after that call.
- * Device calls set `dirty`; the next bulk call first rebuilds the turn words its own kernels wait on. */
+ * `dirty` is set while the turn words are not kept (by device calls and by most bulk calls); a bulk call whose
+ * kernel waits on them first rebuilds them. */
 typedef struct sg_deque_sync
 {
     uint32_t epoch; /* 1 .. 32767 */
@@ -544,9 +545,17 @@ SG_API sg_status sg_deque_create_with_allocator(int32_t elem_bytes, int64_t capa
 SG_API sg_status sg_deque_destroy(sg_deque* dq);
 /* Mixed launch: element i does push_back(values[i]) when is_push[i] != 0, else pop_front().
  * deque_detail.cuh:202-258 (push_back) and :388-446 (pop_front).  out_popped / out_ok nullable.
- * is_push == NULL means all push_back. */
+ * is_push == NULL means all push_back.  The pushes and pops of a call act in some order that the reference's
+ * concurrent threads could take. */
 SG_API sg_status sg_deque_ops(sg_deque* dq, const uint8_t* is_push, const void* values, int64_t n, void* out_popped,
                        uint8_t* out_ok, void* stream);
+/* sg_deque_ops with 0 written to out_popped for every element that popped nothing: a caller that wants that needs
+ * no pass over out_popped of its own. */
+SG_API sg_status sg_deque_ops_zero(sg_deque* dq, const uint8_t* is_push, const void* values, int64_t n,
+                                   void* out_popped, uint8_t* out_ok, void* stream);
+/* pop_front() n times: element i acts as the i-th of a sequence of calls; 0 is written to out_popped where the
+ * deque held no more.  out_popped / out_ok nullable. */
+SG_API sg_status sg_deque_pop_front(sg_deque* dq, int64_t n, void* out_popped, uint8_t* out_ok, void* stream);
 /* size() (clamped): src/stdgpu/impl/deque_detail.cuh:486-520; SG_ERR_RETRY_EXHAUSTED if a wait gave up */
 SG_API sg_status sg_deque_size(sg_deque* dq, void* stream, int64_t* out_size);
 /* Copy the stored elements front to back to out (device) and return their count (synchronises). */

@@ -263,8 +263,8 @@ struct deque_counters
     unsigned int error;
     unsigned int pad;
     long long avail;
-    unsigned long long op_t0; // push_front / pop_back launches: the end before the launch
-    long long op_k;           // and how many elements it moves
+    unsigned long long op_t0; // not used
+    long long op_k;           // not used
 };
 
 

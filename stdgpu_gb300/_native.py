@@ -170,6 +170,8 @@ SIGNATURES = {
     "sg_deque_create_with_allocator": (c_int32, [c_int32, c_int64, POINTER(sg_allocator), POINTER(c_void_p)]),
     "sg_deque_destroy": (c_int32, [c_void_p]),
     "sg_deque_ops": (c_int32, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p]),
+    "sg_deque_ops_zero": (c_int32, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p]),
+    "sg_deque_pop_front": (c_int32, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p]),
     "sg_deque_size": (c_int32, [c_void_p, c_void_p, POINTER(c_int64)]),
     "sg_deque_copy_out": (c_int32, [c_void_p, c_void_p, c_void_p, POINTER(c_int64)]),
     "sg_deque_clear": (c_int32, [c_void_p, c_void_p]),

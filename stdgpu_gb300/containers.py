@@ -613,10 +613,10 @@ class deque:
         """One launch: element i push_back(values[i]) if is_push[i] else pop_front().  Returns (popped, ok)."""
         values = _as_bits(values, self.elem_bytes, "values")
         n = values.numel()
-        popped = torch.zeros(n, dtype=_INT_DTYPE[self.elem_bytes], device=values.device)
-        ok = torch.zeros(n, dtype=torch.uint8, device=values.device)
-        N.check(N.load().sg_deque_ops(self._h, _ptr(is_push), _ptr(values), n, _ptr(popped), _ptr(ok),
-                                      _stream(stream)), "deque::ops")
+        popped = torch.empty(n, dtype=_INT_DTYPE[self.elem_bytes], device=values.device)
+        ok = torch.empty(n, dtype=torch.uint8, device=values.device)
+        N.check(N.load().sg_deque_ops_zero(self._h, _ptr(is_push), _ptr(values), n, _ptr(popped), _ptr(ok),
+                                           _stream(stream)), "deque::ops")
         return popped, ok
 
     def size(self, stream=None) -> int:
@@ -635,11 +635,18 @@ class deque:
 
     def push_back(self, values: torch.Tensor, stream=None) -> torch.Tensor:
         values = _as_bits(values, self.elem_bytes, "values")
-        return self.ops(None, values, stream=stream)[1]
+        ok = torch.empty(values.numel(), dtype=torch.uint8, device=values.device)
+        N.check(N.load().sg_deque_ops(self._h, None, _ptr(values), values.numel(), None, _ptr(ok), _stream(stream)),
+                "deque::push_back")
+        return ok
 
     def pop_front(self, n: int, stream=None) -> tuple[torch.Tensor, torch.Tensor]:
-        return self.ops(torch.zeros(n, dtype=torch.uint8, device="cuda"),
-                        torch.zeros(n, dtype=_INT_DTYPE[self.elem_bytes], device="cuda"), stream=stream)
+        """pop_front() n times; returns (values, ok): element i is the i-th from the front, 0 where there is none."""
+        vals = torch.empty(n, dtype=_INT_DTYPE[self.elem_bytes], device="cuda")
+        ok = torch.empty(n, dtype=torch.uint8, device="cuda")
+        N.check(N.load().sg_deque_pop_front(self._h, int(n), _ptr(vals), _ptr(ok), _stream(stream)),
+                "deque::pop_front")
+        return vals, ok
 
     def push_front(self, values: torch.Tensor, stream=None) -> torch.Tensor:
         """push_front() of each value in order (the last one ends at the front); returns ok flags."""

@@ -2,17 +2,17 @@
 //
 // vector / deque replace the reference's per-element global atomic plus slot
 // spin lock (src/stdgpu/impl/vector_detail.cuh:181-238,
-// src/stdgpu/impl/deque_detail.cuh:202-258, 388-446) with one reservation per
-// tile of 2048 elements: the warps ballot, one warp scans the counts, one
-// thread adds the tile's total to the shared counter and every element takes
-// its rank.  A counter that every warp hits once saturates near 0.5 G updates
-// a second on one address; once per tile it is no longer the bound.
+// src/stdgpu/impl/deque_detail.cuh:202-258, 388-446).  A vector reserves once
+// per tile of up to 8192 elements (a counter that every warp hits once saturates
+// near 0.5 G updates a second on one address); a deque's mixed call counts its
+// pushes first, which settles every element's ticket without a reservation.
 //
 // The deque is a ring of tickets: push k and pop k use slot k mod capacity; a
 // per-slot turn counter (the k-th push stores k+1 after writing the element,
 // the k-th pop stores k+capacity after reading it) orders a pop after the push
-// of the same ticket and a push after the pop one lap earlier.  Those waits are
-// bounded: a wait that runs out sets an error bit and the operation reports
+// of the same ticket and a push after the pop one lap earlier.  Only small rings
+// and mixed calls of more elements than slots order their launches by the turn
+// words.  Those waits are bounded: a wait that runs out sets an error bit and the operation reports
 // failure instead of spinning on.
 //
 // bitset::count (src/stdgpu/impl/bitset_detail.cuh:388-404, count_block_bits
@@ -106,118 +106,199 @@ scan_counts(unsigned* cnt, int lane)
     return __shfl_sync(0xffffffffu, s, 31);
 }
 
-// ---------------------------------------------------------------- vector
-
-// Bulk push_back tiles: kVecItems elements per thread, one reservation on the shared size counter per tile.
-// Measured for 2^28 threads (30 % push): 4 items (1024-element tiles) 0.69 ms, 8 items 0.80 ms, 12 items
-// 1.31 ms, 16 items 1.33 ms -- larger tiles cost registers and resident warps more than their fewer
-// reservations save; 8 items with the values loaded after the reservation took 1.18 ms.
-#ifndef SG_VEC_ITEMS
-#define SG_VEC_ITEMS 4
-#endif
-constexpr int kVecItems = SG_VEC_ITEMS;
-constexpr int kVecCounts = kVecItems * kWarps;
-constexpr int64_t kVecTileElems = int64_t{ kVecItems } * kCThreads;
-static_assert(kVecCounts % 32 == 0 && kVecCounts <= 32 * 8, "whole counts per lane of the scanning warp");
-
-// Exclusive scan of cnt[0, kVecCounts) in place by one warp (kVecCounts / 32 consecutive counts per lane);
-// returns the total to every lane.
-SG_D unsigned
-scan_vec_counts(unsigned* cnt, int lane)
+// True in every thread of the last block to arrive here (`arrived` 0 before the launch, and again after it): that
+// block's threads see what all blocks wrote before they arrived.
+SG_D bool
+last_block(unsigned int* arrived)
 {
-    constexpr int per = kVecCounts / 32;
-    unsigned v[per];
-    unsigned sum = 0u;
-#pragma unroll
-    for (int k = 0; k < per; ++k)
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0)
     {
-        v[k] = cnt[per * lane + k];
-        sum += v[k];
-    }
-    unsigned incl = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1)
-    {
-        const unsigned t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d)
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+        if (last)
         {
-            incl += t;
+            *arrived = 0u;
+            __threadfence();
         }
     }
-    unsigned run = incl - sum;
-#pragma unroll
-    for (int k = 0; k < per; ++k)
-    {
-        cnt[per * lane + k] = run;
-        run += v[k];
-    }
-    return __shfl_sync(0xffffffffu, incl, 31);
+    __syncthreads();
+    return last;
 }
 
-// Bulk push_back: element i pushes values[i] where pred[i] != 0 (every element without pred).  Per tile the
-// selected values are loaded before the tile's reservation, so their loads are in flight while warp 0 scans
-// the counts and adds the tile's total to the size; a reservation past capacity fails the tile's elements
-// there, as the reference's push_back fails past capacity() (its size is clamped when read,
-// vector_detail.cuh:484-511).  Two count buffers alternate between tiles, so a tile needs two barriers.
-template <typename T>
+// Bit j set when byte j of x is not zero.
+SG_D unsigned
+nonzero_bytes(unsigned x)
+{
+    return ((__vsetne4(x, 0u) * 0x10204080u) >> 28) & 0xFu;
+}
+
+// ---------------------------------------------------------------- vector
+
+// Control word of a vector's launches, behind the sync words of its device calls.
+struct vector_control
+{
+    unsigned int arrived; // last_block
+};
+constexpr size_t kControlOffset = 64;
+constexpr size_t kSyncBytes = 256;
+
+// Size and device-call state at the end of a bulk call: the size clamped into [0, capacity] after `minus`
+// elements are taken from its back, the device calls' epoch advanced and the size it starts from recorded.
+SG_D void
+vector_call_ends(long long* size, int64_t cap, int64_t minus, sg_vector_sync* sync, uint32_t epoch)
+{
+    long long s = __ldcg(size);
+    s = s < 0 ? 0 : (s > cap ? cap : s);
+    s = s > minus ? s - minus : 0;
+    *size = s;
+    sync->base_size = s;
+    sync->epoch = epoch;
+}
+
+// Bulk push_back: element i pushes values[i] where pred[i] != 0 (every element without pred).  A warp takes ROWS
+// rows of 32 elements: its lanes read the predicate bytes of consecutive elements, so a lane soon holds a whole
+// row's mask; the block makes one reservation on the size for all its rows, and only then are the selected values
+// read, eight rows of loads in flight.  A reservation past capacity fails the elements there, as the reference's
+// push_back fails past capacity() (its size is clamped when read, vector_detail.cuh:484-511).
+//
+// What bounds it: at 32 rows (8192 elements per reservation) the memory; below that the reservations, updates of one
+// address that complete at about 0.5 G a second.  2^26 threads, 8-byte elements, 30 % pushed, with flags:
+// 130 us, 179 us with one reservation per 1024 elements and the values read before it (4-byte elements 99 / 179).
+// Launches below kVecLargeTile take 4 rows (1024 elements per block), which spreads them over more SMs.
+template <typename T, int ROWS>
 __global__ void __launch_bounds__(kCThreads)
 k_vector_push_back(T* data, long long* size, int64_t cap, const T* values, const uint8_t* pred, int64_t n,
-                   uint8_t* out_pushed)
+                   uint8_t* out_pushed, sg_vector_sync* sync, uint32_t epoch, vector_control* ctl)
 {
-    __shared__ unsigned cnt[2][kVecCounts];
+    static_assert(ROWS == 4 || ROWS == 32, "a lane reads 4 or 32 predicate bytes");
+    constexpr int64_t kWarpElems = ROWS * 32;
+    constexpr int64_t kTile = kWarpElems * kWarps;
+    __shared__ unsigned warp_total[2][kWarps];
     __shared__ long long s_base[2];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
+    const bool words = (reinterpret_cast<uintptr_t>(pred) % ROWS == 0 || reinterpret_cast<uintptr_t>(pred) % 16 == 0) &&
+                       pred != nullptr;
     int buf = 0;
-    for (int64_t tile = static_cast<int64_t>(blockIdx.x) * kVecTileElems; tile < n;
-         tile += static_cast<int64_t>(gridDim.x) * kVecTileElems, buf ^= 1)
+    for (int64_t tile = static_cast<int64_t>(blockIdx.x) * kTile; tile < n;
+         tile += static_cast<int64_t>(gridDim.x) * kTile, buf ^= 1)
     {
-        unsigned masks[kVecItems];
-        T vals[kVecItems];
-#pragma unroll
-        for (int j = 0; j < kVecItems; ++j)
+        const int64_t first = tile + warp * kWarpElems; // the warp's first element
+        const int64_t mine = first + lane * ROWS;       // the lane's first predicate byte
+        unsigned bits = 0u;                             // of the elements mine .. mine + ROWS
+        if (pred != nullptr && words && mine + ROWS <= n)
         {
-            const int64_t i = tile + j * kCThreads + threadIdx.x;
-            const bool want = i < n && (pred == nullptr || pred[i] != 0);
-            masks[j] = __ballot_sync(0xffffffffu, want);
-            if (lane == 0)
+            if constexpr (ROWS == 32)
             {
-                cnt[buf][j * kWarps + warp] = __popc(masks[j]);
+                const uint4 a = __ldg(reinterpret_cast<const uint4*>(pred + mine));
+                const uint4 b = __ldg(reinterpret_cast<const uint4*>(pred + mine) + 1);
+                bits = nonzero_bytes(a.x) | nonzero_bytes(a.y) << 4 | nonzero_bytes(a.z) << 8 |
+                       nonzero_bytes(a.w) << 12 | nonzero_bytes(b.x) << 16 | nonzero_bytes(b.y) << 20 |
+                       nonzero_bytes(b.z) << 24 | nonzero_bytes(b.w) << 28;
             }
-            vals[j] = want ? ld_stream(values + i) : T{};
+            else
+            {
+                bits = nonzero_bytes(__ldg(reinterpret_cast<const unsigned*>(pred + mine)));
+            }
+        }
+        else
+        {
+            for (int j = 0; j < ROWS; ++j)
+            {
+                bits |= static_cast<unsigned>(mine + j < n && (pred == nullptr || pred[mine + j] != 0)) << j;
+            }
+        }
+        // lane r (r < ROWS): the mask of row r
+        unsigned row;
+        if constexpr (ROWS == 32)
+        {
+            row = bits;
+        }
+        else
+        {
+            row = 0u;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+            {
+                row |= __shfl_sync(0xffffffffu, bits, ((lane * 8) & 31) + k) << (4 * k);
+            }
+            row = lane < ROWS ? row : 0u;
+        }
+        const unsigned c = static_cast<unsigned>(__popc(row));
+        unsigned incl = c;
+#pragma unroll
+        for (int d = 1; d < ROWS; d <<= 1)
+        {
+            const unsigned t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d)
+            {
+                incl += t;
+            }
+        }
+        if (lane == ROWS - 1)
+        {
+            warp_total[buf][warp] = incl;
         }
         __syncthreads();
-        if (warp == 0)
+        unsigned before = 0u;
+        unsigned total = 0u;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w)
         {
-            const unsigned total = scan_vec_counts(cnt[buf], lane);
-            if (lane == 0)
-            {
-                // one reservation for the tile (vector_detail.cuh:186-195)
-                s_base[buf] = total > 0 ? static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(size),
-                                                                           static_cast<unsigned long long>(total)))
-                                        : -1;
-            }
+            const unsigned x = warp_total[buf][w];
+            before += w < warp ? x : 0u;
+            total += x;
+        }
+        if (threadIdx.x == 0)
+        {
+            // one reservation for the tile (vector_detail.cuh:186-195)
+            s_base[buf] = total > 0 ? static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(size),
+                                                                       static_cast<unsigned long long>(total)))
+                                    : 0;
         }
         __syncthreads();
-        const long long base = s_base[buf];
-#pragma unroll
-        for (int j = 0; j < kVecItems; ++j)
+        const long long base = s_base[buf] + before;
+        const unsigned row_before = incl - c;
+        constexpr int kFlight = ROWS < 8 ? ROWS : 8;
+#pragma unroll 1
+        for (int r0 = 0; r0 < ROWS; r0 += kFlight)
         {
-            const int64_t i = tile + j * kCThreads + threadIdx.x;
-            const bool want = (masks[j] >> lane) & 1u;
-            const long long pos = base + cnt[buf][j * kWarps + warp] + __popc(masks[j] & lanemask_lt());
-            const bool ok = want && base >= 0 && pos < cap;
-            if (ok)
+            T vals[kFlight];
+            unsigned masks[kFlight];
+#pragma unroll
+            for (int k = 0; k < kFlight; ++k)
             {
-                data[pos] = vals[j];
+                masks[k] = __shfl_sync(0xffffffffu, row, r0 + k);
+                if ((masks[k] >> lane) & 1u)
+                {
+                    vals[k] = ld_stream(values + first + (r0 + k) * 32 + lane);
+                }
             }
-            if (i < n && out_pushed != nullptr)
+#pragma unroll
+            for (int k = 0; k < kFlight; ++k)
             {
-                out_pushed[i] = static_cast<uint8_t>(ok);
+                const long long pos = base + __shfl_sync(0xffffffffu, row_before, r0 + k) +
+                                      __popc(masks[k] & lanemask_lt());
+                const bool ok = ((masks[k] >> lane) & 1u) && pos < cap;
+                if (ok)
+                {
+                    data[pos] = vals[k];
+                }
+                const int64_t i = first + (r0 + k) * 32 + lane;
+                if (out_pushed != nullptr && i < n)
+                {
+                    out_pushed[i] = static_cast<uint8_t>(ok);
+                }
             }
         }
-        // no barrier: the next tile fills the other count buffer, and the one after passes two barriers
-        // that every warp reaches only after reading this tile's counts
+        // no barrier: the next tile fills the other buffer, and the one after passes two barriers that every
+        // warp reaches only after reading this tile's totals
+    }
+    if (last_block(&ctl->arrived) && threadIdx.x == 0)
+    {
+        vector_call_ends(size, cap, 0, sync, epoch);
     }
 }
 
@@ -250,7 +331,7 @@ reserve(long long* counter, long long bound, long long want, bool grow)
     return take;
 }
 
-// Mixed launch: element i pushes values[i] when is_push[i] != 0 (or is_push == NULL), else pops.  Each
+// Mixed launch: element i pushes values[i] when is_push[i] != 0, else pops.  Each
 // tile reserves its pushes and its pops once; the tile's pushes take consecutive tickets in element
 // order, and so do its pops.
 // resident blocks per SM the mixed deque launch is compiled for (its fast path keeps 8 tickets per thread in
@@ -264,10 +345,313 @@ reserve(long long* counter, long long bound, long long want, bool grow)
 #define SG_DEQUE_FAST 1
 #endif
 
+// What a mixed call does, settled on the device by k_deque_plan; behind the sync words of the device calls.
+struct deque_control
+{
+    unsigned long long pushes;  // of the call
+    unsigned long long push_t0; // first ticket of its pushes
+    unsigned long long pop_t0;  // and of its pops
+    long long push_ok;          // pushes that succeed, the first in element order
+    long long pop_ok;           // pops that succeed
+    long long held;             // of these, pops of elements stored before the call
+    unsigned int arrived;       // last_block
+    unsigned int apart;         // 1: no push and pop of the call meet at a slot
+};
+
+// Device-call state at the end of a bulk call: the tickets it leaves, the epoch advanced; dirty: the turn words are
+// not kept (k_deque_rebuild_turns makes them before a launch that waits on them).
+SG_D void
+deque_call_ends(const deque_counters* c, sg_deque_sync* sync, uint32_t epoch, uint32_t dirty)
+{
+    sync->base_begin = c->begin;
+    sync->base_end = c->end;
+    sync->epoch = epoch;
+    sync->dirty = dirty;
+}
+
+constexpr int kPlanTile = 2048; // elements per warp of the plan, per block of the move
+static_assert(kPlanTile == kTileElems, "one count per tile of the move");
+
+// First launch of a mixed call of at most `capacity` elements: pushes per tile of 2048 elements, turned by the last
+// block into the pushes before each tile; that block then settles the call.  The order it stands for runs pushes
+// while there is room and pops while there are elements, in turn, so a push fails only where the deque ends full and
+// a pop only where it ends empty; pushes take the tickets from `end` on and pops those from `begin` on, in element
+// order, and the counters are moved here.  The launches that follow need neither turn words nor reservations.
+// counts: room for a word per tile (the turn words' array, which is marked dirty).
+__global__ void __launch_bounds__(kCThreads)
+k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters* c, int64_t cap, sg_deque_sync* sync,
+             uint32_t epoch, deque_control* ctl)
+{
+    __shared__ unsigned long long s_block;
+    __shared__ unsigned s_warp[kWarps];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int64_t tiles = (n + kPlanTile - 1) / kPlanTile;
+    const bool vec = reinterpret_cast<uintptr_t>(is_push) % 16 == 0;
+    if (threadIdx.x == 0)
+    {
+        s_block = 0;
+    }
+    __syncthreads();
+    unsigned long long mine = 0;
+    for (int64_t tile = static_cast<int64_t>(blockIdx.x) * kWarps + warp; tile < tiles;
+         tile += static_cast<int64_t>(gridDim.x) * kWarps)
+    {
+        const int64_t first = tile * kPlanTile;
+        unsigned count = 0;
+        if (vec && first + kPlanTile <= n)
+        {
+            const uint4* p = reinterpret_cast<const uint4*>(is_push + first);
+#pragma unroll
+            for (int k = 0; k < kPlanTile / 512; ++k)
+            {
+                const uint4 x = __ldg(p + k * 32 + lane);
+                count += __popc(__vsetne4(x.x, 0u)) + __popc(__vsetne4(x.y, 0u)) + __popc(__vsetne4(x.z, 0u)) +
+                         __popc(__vsetne4(x.w, 0u));
+            }
+        }
+        else
+        {
+            for (int64_t i = first + lane; i < n && i < first + kPlanTile; i += 32)
+            {
+                count += is_push[i] != 0;
+            }
+        }
+        count = __reduce_add_sync(0xffffffffu, count);
+        if (lane == 0)
+        {
+            counts[tile] = count;
+            mine += count;
+        }
+    }
+    if (lane == 0 && mine != 0)
+    {
+        atomicAdd(&s_block, mine);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_block != 0)
+    {
+        atomicAdd(&ctl->pushes, s_block);
+    }
+    if (!last_block(&ctl->arrived))
+    {
+        return;
+    }
+    // exclusive scan of the counts, 4 consecutive ones per thread at a time
+    unsigned carry = 0;
+    for (int64_t base = 0; base < tiles; base += 4 * kCThreads)
+    {
+        const int64_t k = base + 4 * static_cast<int64_t>(threadIdx.x);
+        unsigned v[4];
+        unsigned sum = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            v[j] = k + j < tiles ? __ldcg(counts + k + j) : 0u;
+            sum += v[j];
+        }
+        unsigned incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+            const unsigned t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d)
+            {
+                incl += t;
+            }
+        }
+        if (lane == 31)
+        {
+            s_warp[warp] = incl;
+        }
+        __syncthreads();
+        unsigned run = carry + incl - sum;
+        for (int w = 0; w < kWarps; ++w)
+        {
+            const unsigned x = s_warp[w];
+            run += w < warp ? x : 0u;
+            carry += x;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            if (k + j < tiles)
+            {
+                counts[k + j] = run;
+            }
+            run += v[j];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0)
+    {
+        const long long pushes = static_cast<long long>(__ldcg(&ctl->pushes));
+        const long long pops = n - pushes;
+        const long long held = c->avail;
+        const long long room = cap - held;
+        ctl->pushes = 0;
+        const long long net = held + pushes - pops; // elements left if all succeed
+        const long long push_ok = net > cap ? pushes - (net - cap) : pushes;
+        const long long pop_ok = net < 0 ? pops + net : pops;
+        ctl->push_ok = push_ok;
+        ctl->pop_ok = pop_ok;
+        ctl->held = pop_ok < held ? pop_ok : held;
+        ctl->push_t0 = c->end;
+        ctl->pop_t0 = c->begin;
+        ctl->apart = push_ok <= room && pop_ok <= held ? 1u : 0u;
+        c->end += static_cast<unsigned long long>(push_ok);
+        c->begin += static_cast<unsigned long long>(pop_ok);
+        c->size += push_ok - pop_ok;
+        c->avail += push_ok - pop_ok;
+        deque_call_ends(c, sync, epoch, 1u);
+    }
+}
+
+// Before a launch that waits on turn words, when the last call did not keep them: every slot's word from the tickets
+// -- a slot holding ticket t (t in [begin, end)) gets t + 1, a free slot the ticket of the next push_back that maps
+// to it.
+__global__ void
+k_deque_rebuild_turns(unsigned* seq, const deque_counters* c, const sg_deque_sync* sync, int64_t cap)
+{
+    if (*reinterpret_cast<const volatile uint32_t*>(&sync->dirty) == 0u)
+    {
+        return;
+    }
+    const unsigned long long b = c->begin;
+    const unsigned long long e = c->end;
+    const unsigned long long ucap = static_cast<unsigned long long>(cap);
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < cap; i += stride)
+    {
+        const unsigned long long ui = static_cast<unsigned long long>(i);
+        const unsigned long long from_b = (ui + ucap - b % ucap) % ucap; // tickets t = b + from_b map to slot i
+        unsigned v;
+        if (from_b < e - b)
+        {
+            v = static_cast<unsigned>(b + from_b + 1ull);
+        }
+        else
+        {
+            v = static_cast<unsigned>(e + (ui + ucap - e % ucap) % ucap);
+        }
+        seq[i] = v;
+    }
+}
+
+// The launches after the plan: element i moves its element.  Its rank among the pushes (or pops) before it is its
+// tile's count, its warp's and its row's, so tickets follow the element order and a row's pushes and pops go to
+// consecutive slots.  Bound by the bytes: flag, value or popped value, slot and outcome, about 27 bytes an operation.
+// kMoveFirst: pops of elements stored before the call, every outcome, and the pushes too when they meet no pop
+// at a slot (the other two launches then return at once); else kMovePush and kMoveLate follow, pushes
+// and then the pops of elements that the call pushed.
+// 2^24 mixed operations on 8-byte elements in steady state: 153 us in all, 303 us when every slot's turn word
+// was read, waited on and written (and the outputs filled before); from an empty deque, where each pop depends on a
+// push of the call, 375 us against 779 us.
+enum move_phase : int
+{
+    kMoveFirst = 0,
+    kMovePush = 1,
+    kMoveLate = 2
+};
+
+// Compiled for 6 resident blocks per SM: 153 us, with 5 of them 155 us, with the 4 that 64 registers allow 163 us.
+template <typename T, int PHASE>
+__global__ void __launch_bounds__(kCThreads, 6)
+k_deque_move(T* data, const unsigned* before, int64_t cap, const uint8_t* is_push, const T* values, int64_t n,
+             T* out_popped, uint8_t* out_ok, bool zero_rest, const deque_control* ctl)
+{
+    const bool apart = ctl->apart != 0u;
+    if (PHASE != kMoveFirst && apart)
+    {
+        return;
+    }
+    __shared__ unsigned s_warp[2][kWarps];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const unsigned ucap = static_cast<unsigned>(cap);
+    const unsigned push_pos = static_cast<unsigned>(ctl->push_t0 % static_cast<unsigned long long>(cap));
+    const unsigned pop_pos = static_cast<unsigned>(ctl->pop_t0 % static_cast<unsigned long long>(cap));
+    const long long push_ok = ctl->push_ok;
+    const long long pop_ok = ctl->pop_ok;
+    const long long held = ctl->held;
+    int buf = 0;
+    for (int64_t tile = blockIdx.x; tile * kPlanTile < n; tile += gridDim.x, buf ^= 1)
+    {
+        const int64_t first = tile * kPlanTile + warp * (kItems * 32) + lane;
+        unsigned masks[kItems]; // pushes of row j
+        unsigned total = 0;
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+        {
+            const int64_t i = first + j * 32;
+            masks[j] = __ballot_sync(0xffffffffu, i < n && is_push[i] != 0);
+            total += __popc(masks[j]);
+        }
+        if (lane == 0)
+        {
+            s_warp[buf][warp] = total;
+        }
+        __syncthreads();
+        long long rank = __ldg(before + tile); // pushes before the tile, then before the row
+        for (int w = 0; w < warp; ++w)
+        {
+            rank += s_warp[buf][w];
+        }
+        T v[kItems];
+        unsigned pos[kItems];
+        unsigned done = 0u; // bit j: item j succeeds
+        unsigned move = 0u; // bit j: and moves its element in this launch
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+        {
+            const int64_t i = first + j * 32;
+            const bool push = (masks[j] >> lane) & 1u;
+            const long long pushes = rank + __popc(masks[j] & lanemask_lt()); // before element i
+            const long long r = push ? pushes : i - pushes;
+            const bool ok = i < n && r < (push ? push_ok : pop_ok);
+            const bool now = PHASE == kMoveFirst ? (push ? apart : r < held)
+                                                 : (PHASE == kMovePush ? push : !push && r >= held);
+            const unsigned p = (push ? push_pos : pop_pos) + static_cast<unsigned>(r);
+            pos[j] = p >= ucap ? p - ucap : p;
+            v[j] = T{};
+            done |= static_cast<unsigned>(ok) << j;
+            if (ok && now)
+            {
+                move |= 1u << j;
+                v[j] = push ? ld_stream(values + i) : __ldcg(data + pos[j]);
+            }
+            rank += __popc(masks[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+        {
+            const int64_t i = first + j * 32;
+            const bool push = (masks[j] >> lane) & 1u;
+            const bool moves = (move >> j) & 1u;
+            if (push && moves)
+            {
+                data[pos[j]] = v[j];
+            }
+            // a pop of an element that the call pushed is written by the last launch
+            if (out_popped != nullptr && i < n &&
+                (PHASE == kMoveFirst ? zero_rest || (!push && moves) : !push && moves))
+            {
+                out_popped[i] = push ? T{} : v[j];
+            }
+            if (PHASE == kMoveFirst && out_ok != nullptr && i < n)
+            {
+                out_ok[i] = static_cast<uint8_t>((done >> j) & 1u);
+            }
+        }
+        // no barrier: the next tile fills the other count buffer
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kCThreads, SG_DEQUE_MIN_BLOCKS)
 k_deque_ops(T* data, unsigned* seq, deque_counters* c, int64_t cap, const uint8_t* is_push, const T* values,
-            int64_t n, T* out_popped, uint8_t* out_ok)
+            int64_t n, T* out_popped, uint8_t* out_ok, bool zero_rest, deque_control* ctl, sg_deque_sync* sync,
+            uint32_t epoch)
 {
     __shared__ unsigned cpush[kCounts];
     __shared__ unsigned cpop[kCounts];
@@ -285,7 +669,11 @@ k_deque_ops(T* data, unsigned* seq, deque_counters* c, int64_t cap, const uint8_
         {
             const int64_t i = tile + j * kCThreads + threadIdx.x;
             const bool in = i < n;
-            const bool push = in && (is_push == nullptr || is_push[i] != 0);
+            const bool push = in && is_push[i] != 0;
+            if (in && zero_rest && out_popped != nullptr)
+            {
+                out_popped[i] = T{}; // a pop that succeeds writes over it below, in this thread
+            }
             const unsigned pm = __ballot_sync(0xffffffffu, push);
             const unsigned qm = __ballot_sync(0xffffffffu, in && !push);
             if (lane == 0)
@@ -494,97 +882,145 @@ k_deque_ops(T* data, unsigned* seq, deque_counters* c, int64_t cap, const uint8_
         }
         __syncthreads(); // the counts and reservations are rewritten by the next tile
     }
-}
-
-// push_front / pop_back: a launch holds one of them only (the reference runs them concurrently with the
-// other end under per-slot locks, src/stdgpu/impl/deque_detail.cuh:260-386).  Element i of the launch acts
-// as the i-th of a sequence of calls: push_front of values[0..n) leaves values[n-1] at the front, pop_back
-// pops the back element first.  One thread first reserves min(n, room) elements and moves the end
-// (k_deque_reserve_end); then element i < k takes ticket t0 - 1 - i.  Nothing else runs on the deque
-// during the launch, so there are no slot waits; the slot's turn word is left as the FIFO launches that
-// follow expect (a front push leaves the word a push_back of its ticket would leave; a back pop leaves the
-// word that lets push_back reuse its ticket).
-template <bool FRONT_PUSH>
-__global__ void
-k_deque_reserve_end(deque_counters* c, int64_t cap, int64_t n)
-{
-    // push_front needs free capacity (size), pop_back needs elements (avail); both move their end down
-    const long long room = FRONT_PUSH ? cap - c->size : c->avail;
-    const long long k = room <= 0 ? 0 : (room < n ? room : n);
-    unsigned long long* end = FRONT_PUSH ? &c->begin : &c->end;
-    c->op_t0 = *end;
-    c->op_k = k;
-    *end -= static_cast<unsigned long long>(k);
-    c->size += FRONT_PUSH ? k : -k;
-    c->avail += FRONT_PUSH ? k : -k;
-}
-
-template <typename T, bool FRONT_PUSH>
-__global__ void
-k_deque_end_ops(T* data, unsigned* seq, const deque_counters* c, int64_t cap, const T* values, int64_t n,
-                T* out_popped, uint8_t* out_ok)
-{
-    const unsigned long long t0 = c->op_t0;
-    const long long k = c->op_k;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
+    if (last_block(&ctl->arrived) && threadIdx.x == 0)
     {
-        const bool ok = i < k;
-        if (ok)
+        deque_call_ends(c, sync, epoch, 0u);
+    }
+}
+
+// A launch of one kind of operation: element i acts as the i-th of a sequence of calls (push_front of values[0..n)
+// leaves values[n-1] at the front, pop_back pops the back element first; the reference runs them concurrently with
+// the other end under per-slot locks, src/stdgpu/impl/deque_detail.cuh:202-446).  The first min(n, room) elements
+// succeed.  Nothing else runs on the deque during the launch; every block reads the counters as the call found
+// them, and the last one to finish moves them.
+// keep: the ring keeps its turn words between calls (kTurnsKeptMax): a push_back or pop_front waits, bounded, for its
+// slot's turn, and every operation leaves the word that the launches that follow expect (a front push the word of a
+// push_back of its ticket, a back pop the one that lets push_back reuse its ticket).  Larger rings leave them out.
+enum deque_end : int
+{
+    kPushFront = 0,
+    kPopBack = 1,
+    kPushBack = 2,
+    kPopFront = 3
+};
+
+template <typename T, int OP>
+__global__ void __launch_bounds__(kCThreads)
+k_deque_end_ops(T* data, deque_counters* c, int64_t cap, const T* values, int64_t n, T* out_popped, uint8_t* out_ok,
+                bool zero_rest, unsigned* seq, bool keep, sg_deque_sync* sync, uint32_t epoch, deque_control* ctl)
+{
+    constexpr bool push = OP == kPushFront || OP == kPushBack;
+    constexpr bool up = OP == kPushBack || OP == kPopFront; // tickets go up from t0, else down from t0 - 1
+    const unsigned long long ucap = static_cast<unsigned long long>(cap);
+    const unsigned long long begin = __ldcg(&c->begin), end = __ldcg(&c->end);
+    const long long room = push ? cap - __ldcg(&c->size) : __ldcg(&c->avail);
+    const long long k = room <= 0 ? 0 : (room < n ? room : n);
+    const unsigned long long t0 = OP == kPushFront || OP == kPopFront ? begin : end;
+    const int64_t base = static_cast<int64_t>((up ? t0 : t0 - 1ull) % ucap);
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    const uint32_t dirty = *reinterpret_cast<const volatile uint32_t*>(&sync->dirty);
+    if (keep)
+    {
+        for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
         {
-            const unsigned long long tk = t0 - 1ull - static_cast<unsigned long long>(i);
-            const int64_t pos = static_cast<int64_t>(tk % static_cast<unsigned long long>(cap));
-            if constexpr (FRONT_PUSH)
+            bool ok = i < k;
+            T v{};
+            if (ok)
             {
-                data[pos] = values[i];
-                store_turn(seq + pos, static_cast<unsigned>(tk + 1));
-            }
-            else
-            {
-                const T v = data[pos];
-                store_turn(seq + pos, static_cast<unsigned>(tk));
-                if (out_popped != nullptr)
+                int64_t p = up ? base + i : base - i;
+                p = p >= cap ? p - cap : (p < 0 ? p + cap : p);
+                const unsigned tk = static_cast<unsigned>(up ? t0 + static_cast<unsigned long long>(i)
+                                                             : t0 - 1ull - static_cast<unsigned long long>(i));
+                if (up && dirty == 0u)
                 {
-                    out_popped[i] = v;
+                    ok = wait_turn(seq + p, push ? tk : tk + 1u, &c->error);
+                }
+                if (ok)
+                {
+                    if constexpr (push)
+                    {
+                        data[p] = values[i];
+                    }
+                    else
+                    {
+                        v = __ldcg(data + p);
+                    }
+                    seq[p] = push ? tk + 1u : (OP == kPopFront ? tk + static_cast<unsigned>(cap) : tk);
                 }
             }
+            if (!push && out_popped != nullptr && (ok || zero_rest))
+            {
+                out_popped[i] = v;
+            }
+            if (out_ok != nullptr)
+            {
+                out_ok[i] = static_cast<uint8_t>(ok);
+            }
         }
-        if (out_ok != nullptr)
+    }
+    constexpr int kFlight = 4;
+    for (int64_t i0 = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; !keep && i0 < n;
+         i0 += kFlight * stride)
+    {
+        T v[kFlight];
+        int64_t pos[kFlight];
+#pragma unroll
+        for (int j = 0; j < kFlight; ++j)
         {
-            out_ok[i] = static_cast<uint8_t>(ok);
+            const int64_t i = i0 + j * stride;
+            v[j] = T{};
+            if (i < k) // k <= capacity: the slot index wraps at most once
+            {
+                int64_t p = up ? base + i : base - i;
+                p = p >= cap ? p - cap : (p < 0 ? p + cap : p);
+                pos[j] = p;
+                v[j] = push ? ld_stream(values + i) : __ldcg(data + p);
+            }
         }
+#pragma unroll
+        for (int j = 0; j < kFlight; ++j)
+        {
+            const int64_t i = i0 + j * stride;
+            if (i >= n)
+            {
+                break;
+            }
+            const bool ok = i < k;
+            if (push && ok)
+            {
+                data[pos[j]] = v[j];
+            }
+            if (!push && out_popped != nullptr && (ok || zero_rest))
+            {
+                out_popped[i] = v[j];
+            }
+            if (out_ok != nullptr)
+            {
+                out_ok[i] = static_cast<uint8_t>(ok);
+            }
+        }
+    }
+    if (last_block(&ctl->arrived) && threadIdx.x == 0)
+    {
+        const unsigned long long uk = static_cast<unsigned long long>(k);
+        c->begin = OP == kPushFront ? begin - uk : (OP == kPopFront ? begin + uk : begin);
+        c->end = OP == kPushBack ? end + uk : (OP == kPopBack ? end - uk : end);
+        c->size += push ? k : -k;
+        c->avail += push ? k : -k;
+        deque_call_ends(c, sync, epoch, keep ? dirty : 1u);
     }
 }
 
 // vector::pop_back for n elements (src/stdgpu/impl/vector_detail.cuh:240-299): element i takes the i-th
-// element from the back.  The size is clamped into [0, capacity] first (a push launch may leave it above),
-// read by every thread, and lowered by one thread afterwards.
-__global__ void
-k_vector_clamp(long long* size, int64_t cap, int64_t minus)
-{
-    long long s = *size;
-    s = s < 0 ? 0 : (s > cap ? cap : s);
-    s -= minus;
-    *size = s < 0 ? 0 : s;
-}
-
-// End of every bulk call: size clamped into [0, capacity], the device calls' epoch advanced and the size
-// it starts from recorded (sg_vector_sync).
-__global__ void
-k_vector_epoch(long long* size, int64_t cap, sg_vector_sync* sync, uint32_t epoch)
-{
-    long long s = *size;
-    s = s < 0 ? 0 : (s > cap ? cap : s);
-    *size = s;
-    sync->base_size = s;
-    sync->epoch = epoch;
-}
-
+// element from the back.  Every block reads the size as the call found it (clamped into [0, capacity]: a push
+// launch may leave it above); the last one to finish lowers it.
 template <typename T>
-__global__ void
-k_vector_pop_back(const T* data, const long long* size, int64_t n, T* out_values, uint8_t* out_ok)
+__global__ void __launch_bounds__(kCThreads)
+k_vector_pop_back(const T* data, long long* size, int64_t cap, int64_t n, T* out_values, uint8_t* out_ok,
+                  sg_vector_sync* sync, uint32_t epoch, vector_control* ctl)
 {
-    const long long sz = *size;
+    long long sz = __ldcg(size);
+    sz = sz < 0 ? 0 : (sz > cap ? cap : sz);
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
     {
@@ -599,69 +1035,48 @@ k_vector_pop_back(const T* data, const long long* size, int64_t n, T* out_values
             out_ok[i] = static_cast<uint8_t>(ok);
         }
     }
+    if (last_block(&ctl->arrived) && threadIdx.x == 0)
+    {
+        vector_call_ends(size, cap, n, sync, epoch);
+    }
 }
 
-// Before a bulk call: when device calls ran since the last bulk call (they keep per-slot occupied words,
-// not turn words), every slot's turn word is rebuilt from the tickets -- a slot holding ticket t (t in
-// [begin, end)) gets t + 1, a free slot the ticket of the next push_back that maps to it.
+// clear(), and the end of the calls that the host drives (insert, erase).
 __global__ void
-k_deque_rebuild_turns(unsigned* seq, const deque_counters* c, const sg_deque_sync* sync, int64_t cap)
+k_vector_call_ends(long long* size, int64_t cap, bool clear, sg_vector_sync* sync, uint32_t epoch)
 {
-    if (*reinterpret_cast<const volatile uint32_t*>(&sync->dirty) == 0u)
+    if (clear)
+    {
+        *size = 0;
+    }
+    vector_call_ends(size, cap, 0, sync, epoch);
+}
+
+// keep: the turn words too (slot i is free for ticket i, modulo 2^32)
+__global__ void
+k_deque_reset(unsigned* seq, deque_counters* c, int64_t cap, bool keep, sg_deque_sync* sync, uint32_t epoch)
+{
+    if (keep)
+    {
+        for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < cap;
+             i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+        {
+            seq[i] = static_cast<unsigned>(i);
+        }
+    }
+    if (blockIdx.x != 0 || threadIdx.x != 0)
     {
         return;
     }
-    const unsigned long long b = c->begin;
-    const unsigned long long e = c->end;
-    const unsigned long long ucap = static_cast<unsigned long long>(cap);
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < cap; i += stride)
-    {
-        const unsigned long long ui = static_cast<unsigned long long>(i);
-        const unsigned long long from_b = (ui + ucap - b % ucap) % ucap; // tickets t = b + from_b map to slot i
-        unsigned v;
-        if (from_b < e - b)
-        {
-            v = static_cast<unsigned>(b + from_b + 1ull);
-        }
-        else
-        {
-            v = static_cast<unsigned>(e + (ui + ucap - e % ucap) % ucap);
-        }
-        seq[i] = v;
-    }
-}
-
-// After the rebuild, and at the end of every bulk call: the device calls' epoch advanced and the tickets
-// it starts from recorded; dirty cleared.
-__global__ void
-k_deque_epoch(const deque_counters* c, sg_deque_sync* sync, uint32_t epoch)
-{
-    sync->base_begin = c->begin;
-    sync->base_end = c->end;
-    sync->epoch = epoch;
-    sync->dirty = 0u;
-}
-
-__global__ void
-k_deque_reset(unsigned* seq, deque_counters* c, int64_t cap)
-{
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < cap; i += stride)
-    {
-        seq[i] = static_cast<unsigned>(i);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-    {
-        // tickets start at capacity x 2^32: a multiple of the capacity (so ticket mod capacity is the slot)
-        // and of 2^32 (so the 32-bit turn words start at the slot index), far enough from zero for
-        // push_front to move begin down
-        c->size = 0;
-        c->begin = static_cast<unsigned long long>(cap) << 32;
-        c->end = static_cast<unsigned long long>(cap) << 32;
-        c->error = 0;
-        c->avail = 0;
-    }
+    // tickets start at capacity x 2^32: a multiple of the capacity (so ticket mod capacity is the slot)
+    // and of 2^32 (so the 32-bit turn words start at the slot index), far enough from zero for
+    // push_front to move begin down
+    c->size = 0;
+    c->begin = static_cast<unsigned long long>(cap) << 32;
+    c->end = static_cast<unsigned long long>(cap) << 32;
+    c->error = 0;
+    c->avail = 0;
+    deque_call_ends(c, sync, epoch, keep ? 0u : 1u);
 }
 
 template <typename T>
@@ -899,20 +1314,10 @@ count_scratch g_count_scratch[64];
 namespace
 {
 
-// Every bulk call on a deque runs between these two: the turn words rebuilt if device calls ran since the
-// last bulk call, and afterwards the device calls' epoch advanced (slot words cleared when it wraps).
+// The device calls' epoch at the end of a bulk call: 1 .. 32767 (slot words are cleared when it wraps).
+template <typename Object>
 sg_status
-deque_bulk_begin(sg_deque* d, cudaStream_t s)
-{
-    static const int mg = persistent_grid(k_deque_rebuild_turns, kCThreads);
-    k_deque_rebuild_turns<<<grid_for(d->capacity, kCThreads, mg), kCThreads, 0, s>>>(d->seq, d->counters, d->sync,
-                                                                                     d->capacity);
-    SG_LAUNCH_CHECK();
-    return SG_OK;
-}
-
-sg_status
-deque_bulk_end(sg_deque* d, cudaStream_t s)
+next_epoch(Object* d, cudaStream_t s)
 {
     uint32_t e = d->epoch + 1;
     if (e > 32767u)
@@ -921,16 +1326,47 @@ deque_bulk_end(sg_deque* d, cudaStream_t s)
         e = 1;
     }
     d->epoch = e;
-    k_deque_epoch<<<1, 1, 0, s>>>(d->counters, d->sync, e);
+    return SG_OK;
+}
+
+// Rings of at most this many slots keep their turn words from call to call and order every mixed launch by them: two
+// launches instead of four.  4096 mixed operations on a ring of 16384: 23 us in steady state and 19 us from empty
+// (30 and 28 us with the rebuild and the epoch as launches of their own).  Larger rings make the words for the
+// launches that wait on them, those of more elements than the ring has slots.
+constexpr int64_t kTurnsKeptMax = int64_t{ 1 } << 16;
+
+deque_control*
+control_of(const sg_deque* d)
+{
+    return reinterpret_cast<deque_control*>(reinterpret_cast<char*>(d->sync) + kControlOffset);
+}
+
+vector_control*
+control_of(const sg_vector* v)
+{
+    return reinterpret_cast<vector_control*>(reinterpret_cast<char*>(v->sync) + kControlOffset);
+}
+
+template <typename T, int OP>
+sg_status
+deque_end_launch(sg_deque* d, const void* values, int64_t n, void* out_popped, uint8_t* out_ok, bool zero_rest,
+                 cudaStream_t s)
+{
+    static const int mg = persistent_grid(k_deque_end_ops<T, OP>, kCThreads);
+    k_deque_end_ops<T, OP><<<grid_for(n, kCThreads, mg), kCThreads, 0, s>>>(
+            static_cast<T*>(d->data), d->counters, d->capacity, static_cast<const T*>(values), n,
+            static_cast<T*>(out_popped), out_ok, zero_rest, d->seq, d->capacity <= kTurnsKeptMax, d->sync, d->epoch,
+            control_of(d));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
 
-template <bool FRONT_PUSH>
+template <int OP>
 sg_status
-deque_end_ops(sg_deque* d, const void* values, int64_t n, void* out_popped, uint8_t* out_ok, void* stream)
+deque_end_ops(sg_deque* d, const void* values, int64_t n, void* out_popped, uint8_t* out_ok, bool zero_rest,
+              void* stream)
 {
-    if (d == nullptr || n < 0 || (FRONT_PUSH && n > 0 && values == nullptr))
+    if (d == nullptr || n < 0 || ((OP == kPushFront || OP == kPushBack) && n > 0 && values == nullptr))
     {
         return SG_ERR_BAD_ARG;
     }
@@ -939,47 +1375,118 @@ deque_end_ops(sg_deque* d, const void* values, int64_t n, void* out_popped, uint
         return SG_OK;
     }
     cudaStream_t s = as_stream(stream);
-    sg_status st = deque_bulk_begin(d, s);
+    const sg_status st = next_epoch(d, s);
     if (st != SG_OK)
     {
         return st;
     }
-    k_deque_reserve_end<FRONT_PUSH><<<1, 1, 0, s>>>(d->counters, d->capacity, n);
-    SG_LAUNCH_CHECK();
-    const int g = grid_for(n, kCThreads, 4096);
-    if (d->elem_bytes == 4)
-    {
-        k_deque_end_ops<uint32_t, FRONT_PUSH><<<g, kCThreads, 0, s>>>(
-                static_cast<uint32_t*>(d->data), d->seq, d->counters, d->capacity, static_cast<const uint32_t*>(values), n,
-                static_cast<uint32_t*>(out_popped), out_ok);
-    }
-    else
-    {
-        k_deque_end_ops<unsigned long long, FRONT_PUSH><<<g, kCThreads, 0, s>>>(
-                static_cast<unsigned long long*>(d->data), d->seq, d->counters, d->capacity,
-                static_cast<const unsigned long long*>(values), n, static_cast<unsigned long long*>(out_popped), out_ok);
-    }
-    SG_LAUNCH_CHECK();
-    return deque_bulk_end(d, s);
+    return d->elem_bytes == 4
+                   ? deque_end_launch<uint32_t, OP>(d, values, n, out_popped, out_ok, zero_rest, s)
+                   : deque_end_launch<unsigned long long, OP>(d, values, n, out_popped, out_ok, zero_rest, s);
 }
 
-} // namespace
-
-namespace
-{
-
-// Ends a bulk call on v: the next epoch (1 .. 32767; slot words are cleared when it wraps).
+// A mixed call: the plan and the moves; by turn words on a small ring, or with more elements than slots, whose pushes
+// and pops may pass through a slot several times.
+template <typename T>
 sg_status
-vector_next_epoch(sg_vector* v, cudaStream_t s)
+deque_mixed(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, void* out_popped, uint8_t* out_ok,
+            bool zero_rest, cudaStream_t s)
 {
-    uint32_t e = v->epoch + 1;
-    if (e > 32767u)
+    T* const data = static_cast<T*>(d->data);
+    const T* const in = static_cast<const T*>(values);
+    T* const out = static_cast<T*>(out_popped);
+    if (d->capacity <= kTurnsKeptMax || n > d->capacity)
     {
-        SG_CUDA_TRY(cudaMemsetAsync(v->slot_state, 0, static_cast<size_t>(v->capacity) * sizeof(uint16_t), s));
-        e = 1;
+        static const int mr = persistent_grid(k_deque_rebuild_turns, kCThreads);
+        k_deque_rebuild_turns<<<grid_for(d->capacity, kCThreads, mr), kCThreads, 0, s>>>(d->seq, d->counters, d->sync,
+                                                                                         d->capacity);
+        SG_LAUNCH_CHECK();
+        static const int mo = persistent_grid(k_deque_ops<T>, kCThreads);
+        k_deque_ops<T><<<grid_for(n, static_cast<int>(kTileElems), mo), kCThreads, 0, s>>>(
+                data, d->seq, d->counters, d->capacity, is_push, in, n, out, out_ok, zero_rest, control_of(d), d->sync,
+                d->epoch);
+        SG_LAUNCH_CHECK();
+        return SG_OK;
     }
-    v->epoch = e;
-    k_vector_epoch<<<1, 1, 0, s>>>(v->size, v->capacity, v->sync, e);
+    const int64_t tiles = (n + kPlanTile - 1) / kPlanTile;
+    static const int mp = persistent_grid(k_deque_plan, kCThreads);
+    k_deque_plan<<<grid_for(tiles, kWarps, mp), kCThreads, 0, s>>>(is_push, n, d->seq, d->counters, d->capacity,
+                                                                   d->sync, d->epoch, control_of(d));
+    SG_LAUNCH_CHECK();
+    static const int m0 = persistent_grid(k_deque_move<T, kMoveFirst>, kCThreads);
+    static const int m1 = persistent_grid(k_deque_move<T, kMovePush>, kCThreads);
+    static const int m2 = persistent_grid(k_deque_move<T, kMoveLate>, kCThreads);
+    k_deque_move<T, kMoveFirst><<<grid_for(tiles, 1, m0), kCThreads, 0, s>>>(data, d->seq, d->capacity, is_push, in, n,
+                                                                            out, out_ok, zero_rest, control_of(d));
+    SG_LAUNCH_CHECK();
+    k_deque_move<T, kMovePush><<<grid_for(tiles, 1, m1), kCThreads, 0, s>>>(data, d->seq, d->capacity, is_push, in, n,
+                                                                           out, out_ok, zero_rest, control_of(d));
+    SG_LAUNCH_CHECK();
+    k_deque_move<T, kMoveLate><<<grid_for(tiles, 1, m2), kCThreads, 0, s>>>(data, d->seq, d->capacity, is_push, in, n,
+                                                                           out, out_ok, zero_rest, control_of(d));
+    SG_LAUNCH_CHECK();
+    return SG_OK;
+}
+
+sg_status
+deque_ops(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, void* out_popped, uint8_t* out_ok,
+          bool zero_rest, void* stream)
+{
+    if (d == nullptr || n < 0)
+    {
+        return SG_ERR_BAD_ARG;
+    }
+    if (n == 0)
+    {
+        return SG_OK;
+    }
+    cudaStream_t s = as_stream(stream);
+    if (is_push == nullptr)
+    {
+        // all push_back; nothing is popped
+        if (zero_rest && out_popped != nullptr)
+        {
+            SG_CUDA_TRY(cudaMemsetAsync(out_popped, 0, static_cast<size_t>(n) * d->elem_bytes, s));
+        }
+        return deque_end_ops<kPushBack>(d, values, n, nullptr, out_ok, false, stream);
+    }
+    const sg_status st = next_epoch(d, s);
+    if (st != SG_OK)
+    {
+        return st;
+    }
+    return d->elem_bytes == 4
+                   ? deque_mixed<uint32_t>(d, is_push, values, n, out_popped, out_ok, zero_rest, s)
+                   : deque_mixed<unsigned long long>(d, is_push, values, n, out_popped, out_ok, zero_rest, s);
+}
+
+// Ends a bulk call on v that the host drives, or clears it.
+sg_status
+vector_call_ends(sg_vector* v, bool clear, cudaStream_t s)
+{
+    const sg_status st = next_epoch(v, s);
+    if (st != SG_OK)
+    {
+        return st;
+    }
+    k_vector_call_ends<<<1, 1, 0, s>>>(v->size, v->capacity, clear, v->sync, v->epoch);
+    SG_LAUNCH_CHECK();
+    return SG_OK;
+}
+
+// Launches of at least this many elements reserve once per 8192 of them (k_vector_push_back): from here on they
+// have a block of that size for every SM.  2^20 elements (4 rows) 10.9 us, 2^21 (32 rows) 10.9 us, back to back with
+// the call that ends each (11.9 and 12.9 before).
+constexpr int64_t kVecLargeTile = int64_t{ 1 } << 21;
+
+template <typename T, int ROWS>
+sg_status
+push_back_launch(sg_vector* v, const void* values, const uint8_t* pred, int64_t n, uint8_t* out_pushed, cudaStream_t s)
+{
+    static const int mg = persistent_grid(k_vector_push_back<T, ROWS>, kCThreads);
+    k_vector_push_back<T, ROWS><<<grid_for(n, ROWS * kCThreads, mg), kCThreads, 0, s>>>(
+            static_cast<T*>(v->data), v->size, v->capacity, static_cast<const T*>(values), pred, n, out_pushed, v->sync,
+            v->epoch, control_of(v));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -1027,7 +1534,11 @@ create_vector(int32_t elem_bytes, int64_t capacity, const object_allocator& oa, 
     }
     if (e == cudaSuccess)
     {
-        e = sg::detail::obj_malloc(v->oa, &v->sync, sizeof(sg_vector_sync));
+        e = sg::detail::obj_malloc(v->oa, &v->sync, kSyncBytes);
+    }
+    if (e == cudaSuccess)
+    {
+        e = cudaMemset(v->sync, 0, kSyncBytes);
     }
     if (e == cudaSuccess)
     {
@@ -1104,22 +1615,18 @@ sg_vector_push_back(sg_vector* v, const void* values, const uint8_t* pred, int64
         return SG_OK;
     }
     cudaStream_t s = as_stream(stream);
-    if (v->elem_bytes == 4)
+    const sg_status st = next_epoch(v, s);
+    if (st != SG_OK)
     {
-        static const int mg = persistent_grid(k_vector_push_back<uint32_t>, kCThreads);
-        k_vector_push_back<uint32_t><<<grid_for(n, static_cast<int>(kVecTileElems), mg), kCThreads, 0, s>>>(
-                static_cast<uint32_t*>(v->data), v->size, v->capacity, static_cast<const uint32_t*>(values), pred, n,
-                out_pushed);
+        return st;
     }
-    else
+    if (n >= kVecLargeTile)
     {
-        static const int mg = persistent_grid(k_vector_push_back<unsigned long long>, kCThreads);
-        k_vector_push_back<unsigned long long><<<grid_for(n, static_cast<int>(kVecTileElems), mg), kCThreads, 0, s>>>(
-                static_cast<unsigned long long*>(v->data), v->size, v->capacity,
-                static_cast<const unsigned long long*>(values), pred, n, out_pushed);
+        return v->elem_bytes == 4 ? push_back_launch<uint32_t, 32>(v, values, pred, n, out_pushed, s)
+                                  : push_back_launch<unsigned long long, 32>(v, values, pred, n, out_pushed, s);
     }
-    SG_LAUNCH_CHECK();
-    return vector_next_epoch(v, s);
+    return v->elem_bytes == 4 ? push_back_launch<uint32_t, 4>(v, values, pred, n, out_pushed, s)
+                              : push_back_launch<unsigned long long, 4>(v, values, pred, n, out_pushed, s);
 }
 
 sg_status
@@ -1144,8 +1651,7 @@ sg_vector_clear(sg_vector* v, void* stream)
     {
         return SG_ERR_BAD_ARG;
     }
-    SG_CUDA_TRY(cudaMemsetAsync(v->size, 0, sizeof(long long), as_stream(stream)));
-    return vector_next_epoch(v, as_stream(stream));
+    return vector_call_ends(v, true, as_stream(stream));
 }
 
 sg_status
@@ -1160,24 +1666,26 @@ sg_vector_pop_back(sg_vector* v, int64_t n, void* out_values, uint8_t* out_ok, v
         return SG_OK;
     }
     cudaStream_t s = as_stream(stream);
-    k_vector_clamp<<<1, 1, 0, s>>>(v->size, v->capacity, 0);
-    SG_LAUNCH_CHECK();
+    const sg_status st = next_epoch(v, s);
+    if (st != SG_OK)
+    {
+        return st;
+    }
     const int g = grid_for(n, kCThreads, 4096);
     if (v->elem_bytes == 4)
     {
-        k_vector_pop_back<uint32_t><<<g, kCThreads, 0, s>>>(static_cast<const uint32_t*>(v->data), v->size, n,
-                                                            static_cast<uint32_t*>(out_values), out_ok);
+        k_vector_pop_back<uint32_t><<<g, kCThreads, 0, s>>>(static_cast<const uint32_t*>(v->data), v->size,
+                                                            v->capacity, n, static_cast<uint32_t*>(out_values), out_ok,
+                                                            v->sync, v->epoch, control_of(v));
     }
     else
     {
         k_vector_pop_back<unsigned long long><<<g, kCThreads, 0, s>>>(
-                static_cast<const unsigned long long*>(v->data), v->size, n, static_cast<unsigned long long*>(out_values),
-                out_ok);
+                static_cast<const unsigned long long*>(v->data), v->size, v->capacity, n,
+                static_cast<unsigned long long*>(out_values), out_ok, v->sync, v->epoch, control_of(v));
     }
     SG_LAUNCH_CHECK();
-    k_vector_clamp<<<1, 1, 0, s>>>(v->size, v->capacity, n);
-    SG_LAUNCH_CHECK();
-    return vector_next_epoch(v, s);
+    return SG_OK;
 }
 
 sg_status
@@ -1202,7 +1710,7 @@ sg_vector_insert(sg_vector* v, const void* values, int64_t n, void* stream)
                                 static_cast<size_t>(n) * v->elem_bytes, cudaMemcpyDeviceToDevice, s));
     *v->host = size + n;
     SG_CUDA_TRY(cudaMemcpyAsync(v->size, v->host, sizeof(long long), cudaMemcpyHostToDevice, s));
-    const sg_status e = vector_next_epoch(v, s);
+    const sg_status e = vector_call_ends(v, false, s);
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     return e;
 }
@@ -1227,7 +1735,7 @@ sg_vector_erase(sg_vector* v, int64_t n, void* stream)
     cudaStream_t s = as_stream(stream);
     *v->host = size - n;
     SG_CUDA_TRY(cudaMemcpyAsync(v->size, v->host, sizeof(long long), cudaMemcpyHostToDevice, s));
-    const sg_status e = vector_next_epoch(v, s);
+    const sg_status e = vector_call_ends(v, false, s);
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     return e;
 }
@@ -1288,11 +1796,11 @@ create_deque(int32_t elem_bytes, int64_t capacity, const object_allocator& oa, s
     }
     if (e == cudaSuccess)
     {
-        e = sg::detail::obj_malloc(d->oa, &d->sync, sizeof(sg_deque_sync));
+        e = sg::detail::obj_malloc(d->oa, &d->sync, kSyncBytes);
     }
     if (e == cudaSuccess)
     {
-        e = cudaMemset(d->sync, 0, sizeof(sg_deque_sync));
+        e = cudaMemset(d->sync, 0, kSyncBytes);
     }
     if (e != cudaSuccess)
     {
@@ -1365,59 +1873,49 @@ sg_deque_clear(sg_deque* d, void* stream)
         return SG_ERR_BAD_ARG;
     }
     cudaStream_t s = as_stream(stream);
-    static const int mg = persistent_grid(k_deque_reset, kCThreads);
-    k_deque_reset<<<grid_for(d->capacity, kCThreads, mg), kCThreads, 0, s>>>(d->seq, d->counters, d->capacity);
+    const sg_status st = next_epoch(d, s);
+    if (st != SG_OK)
+    {
+        return st;
+    }
+    const bool keep = d->capacity <= kTurnsKeptMax;
+    k_deque_reset<<<keep ? grid_for(d->capacity, kCThreads, 256) : 1, kCThreads, 0, s>>>(d->seq, d->counters,
+                                                                                          d->capacity, keep, d->sync,
+                                                                                          d->epoch);
     SG_LAUNCH_CHECK();
-    return deque_bulk_end(d, s);
+    return SG_OK;
 }
 
 sg_status
 sg_deque_push_front(sg_deque* d, const void* values, int64_t n, uint8_t* out_ok, void* stream)
 {
-    return deque_end_ops<true>(d, values, n, nullptr, out_ok, stream);
+    return deque_end_ops<kPushFront>(d, values, n, nullptr, out_ok, false, stream);
 }
 
 sg_status
 sg_deque_pop_back(sg_deque* d, int64_t n, void* out_popped, uint8_t* out_ok, void* stream)
 {
-    return deque_end_ops<false>(d, nullptr, n, out_popped, out_ok, stream);
+    return deque_end_ops<kPopBack>(d, nullptr, n, out_popped, out_ok, false, stream);
 }
 
 sg_status
 sg_deque_ops(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, void* out_popped, uint8_t* out_ok,
              void* stream)
 {
-    if (d == nullptr || n < 0)
-    {
-        return SG_ERR_BAD_ARG;
-    }
-    if (n == 0)
-    {
-        return SG_OK;
-    }
-    cudaStream_t s = as_stream(stream);
-    sg_status st = deque_bulk_begin(d, s);
-    if (st != SG_OK)
-    {
-        return st;
-    }
-    if (d->elem_bytes == 4)
-    {
-        static const int mg = persistent_grid(k_deque_ops<uint32_t>, kCThreads);
-        k_deque_ops<uint32_t><<<grid_for(n, static_cast<int>(kTileElems), mg), kCThreads, 0, s>>>(
-                static_cast<uint32_t*>(d->data), d->seq, d->counters, d->capacity, is_push,
-                static_cast<const uint32_t*>(values), n, static_cast<uint32_t*>(out_popped), out_ok);
-    }
-    else
-    {
-        static const int mg = persistent_grid(k_deque_ops<unsigned long long>, kCThreads);
-        k_deque_ops<unsigned long long><<<grid_for(n, static_cast<int>(kTileElems), mg), kCThreads, 0, s>>>(
-                static_cast<unsigned long long*>(d->data), d->seq, d->counters, d->capacity, is_push,
-                static_cast<const unsigned long long*>(values), n, static_cast<unsigned long long*>(out_popped),
-                out_ok);
-    }
-    SG_LAUNCH_CHECK();
-    return deque_bulk_end(d, s);
+    return deque_ops(d, is_push, values, n, out_popped, out_ok, false, stream);
+}
+
+sg_status
+sg_deque_ops_zero(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, void* out_popped,
+                  uint8_t* out_ok, void* stream)
+{
+    return deque_ops(d, is_push, values, n, out_popped, out_ok, true, stream);
+}
+
+sg_status
+sg_deque_pop_front(sg_deque* d, int64_t n, void* out_popped, uint8_t* out_ok, void* stream)
+{
+    return deque_end_ops<kPopFront>(d, nullptr, n, out_popped, out_ok, true, stream);
 }
 
 sg_status
