@@ -27,7 +27,7 @@ constexpr int kThreads = 256;
 #ifndef SG_ORDERED_MIN_BLOCKS
 #define SG_ORDERED_MIN_BLOCKS SG_BULK_MIN_BLOCKS
 #endif
-constexpr int kRangeChunk = 2048; // slots per block in the compaction kernels (256 threads x 8 slots)
+constexpr int kRangeChunk = 2048; // slots per word of a table's compaction scratch
 
 // Kernel view of a table.  Group and slot indices fit 32 bits (max_size() < 2^31), so the hot paths
 // index in 32-bit arithmetic and widen only to form addresses.

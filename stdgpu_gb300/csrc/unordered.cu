@@ -1455,205 +1455,215 @@ k_popc_words(const uint32_t* w, int64_t n, unsigned long long* out)
     block_add<1>(vv, dst);
 }
 
-// Compaction, pass 1: live slots per chunk of kRangeChunk slots.
+// Compaction of the live slots in slot order (device_range(), range_copy()) in one launch.  Each block takes the next
+// run of tiles (a tile: 1 or 2 KB of slots, read by a warp), shares it out to its warps, counts the live slots,
+// publishes the count, adds up the counts of the runs before its own, and goes through the run again to write.  Runs
+// are taken in order from a counter, so every count waited for is being made by a resident block; the wait is bounded
+// all the same.  The second time the tiles are read last to first: the ones read last are still in L2.  The last run
+// appends the out-of-band keys and leaves the total in hdr->count.
+// Bound by reading the slots, up to the size of L2 once, beyond it up to twice.  Calls with their read-back of the
+// count: 13.7 M slots of 16 bytes (219 MB), 3.1 M live, 96 us; 27 M slots of 8 bytes, 8.4 M live, 117 us; 219 M slots
+// of 16 bytes (3.5 GB) 1219 us -- 144, 185 and 1580 us as a counting pass, a one-block scan, a second pass and a
+// launch for the out-of-band keys.  A single pass whose tiles look back at one another's counts took 156-207 us for
+// the first: its blocks run in lockstep and wait for one another every 32 KB.  Twice the slots per lane cost the
+// 8-byte case 30 %, 6 or 8 blocks per SM nothing or 5 %; keeping the masks of the first time gave nothing.
+constexpr unsigned int kErrRange = 16u; // a wait for an earlier run gave up (table header error bit)
+constexpr int kRangePolls = 1 << 20;
+
 template <int KIND>
-__global__ void __launch_bounds__(kThreads)
-k_range_count(dview t, unsigned int* chunk_counts)
+struct range_tile
 {
-    using C = kind_consts<KIND>;
-    using K = typename C::K;
-    const int64_t c = blockIdx.x;
-    const int64_t first = c * kRangeChunk;
-    const int64_t limit = t.total;
-    unsigned int live = 0;
-#pragma unroll
-    for (int r = 0; r < kRangeChunk / kThreads; ++r)
-    {
-        const int64_t s = first + r * kThreads + threadIdx.x;
-        if (s < limit)
-        {
-            const K k = __ldcg(reinterpret_cast<const K*>(t.slots + s * C::slot_bytes));
-            live += (k != C::empty_key && k != C::tomb_key);
-        }
-    }
-    __shared__ unsigned int red[kThreads / 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        live += __shfl_xor_sync(0xffffffffu, live, o);
-    }
-    if ((threadIdx.x & 31) == 0)
-    {
-        red[threadIdx.x >> 5] = live;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        unsigned int s = 0;
-        for (int w = 0; w < kThreads / 32; ++w)
-        {
-            s += red[w];
-        }
-        chunk_counts[c] = s;
-    }
-}
+    static constexpr int items = kind_consts<KIND>::slot_bytes == 16 ? 4 : 8; // slots per lane
+    static constexpr int64_t slots = int64_t{ items } * 32;
+};
 
-// Compaction, pass 2: exclusive scan of the chunk counts (one block), then the out-of-band keys are
-// appended after the probed ones; the total lands in hdr->count.
-__global__ void __launch_bounds__(1024)
-k_range_scan(unsigned int* chunk_counts, int64_t nchunks, table_header* hdr, int32_t* out_slots,
-             int64_t special_base, int want_slots)
-{
-    __shared__ unsigned long long part[1024];
-    const int64_t per = (nchunks + blockDim.x - 1) / blockDim.x;
-    const int64_t lo = threadIdx.x * per;
-    const int64_t hi = lo + per < nchunks ? lo + per : nchunks;
-    unsigned long long s = 0;
-    for (int64_t c = lo; c < hi; ++c)
-    {
-        s += chunk_counts[c];
-    }
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        unsigned long long run = 0;
-        for (int w = 0; w < static_cast<int>(blockDim.x); ++w)
-        {
-            const unsigned long long x = part[w];
-            part[w] = run;
-            run += x;
-        }
-        unsigned long long total = run;
-        for (int sp = 0; sp < 2; ++sp)
-        {
-            if (hdr->special_state[sp] == 1u)
-            {
-                if (want_slots && out_slots != nullptr)
-                {
-                    out_slots[total] = static_cast<int32_t>(special_base + sp);
-                }
-                ++total;
-            }
-        }
-        hdr->count = total;
-    }
-    __syncthreads();
-    unsigned long long run = part[threadIdx.x];
-    for (int64_t c = lo; c < hi; ++c)
-    {
-        const unsigned int x = chunk_counts[c];
-        chunk_counts[c] = static_cast<unsigned int>(run);
-        run += x;
-    }
-}
-
-// Compaction, pass 3: write slot indices (or keys / mapped values) of live slots in slot order.
+// words[r]: 0 not known, or 1 + the live slots of run r; the run counter behind them; all zero before the launch.
+// Writes slot indices (SLOTS) or keys and mapped values (each nullable).
 template <int KIND, bool SLOTS>
-__global__ void __launch_bounds__(kThreads)
-k_range_write(dview t, const unsigned int* chunk_offsets, int32_t* out_slots, void* out_keys, void* out_vals)
+__global__ void __launch_bounds__(kThreads, 4)
+k_range(dview t, unsigned int* words, int runs, int64_t tiles, int32_t* out_slots, void* out_keys, void* out_vals)
 {
     using C = kind_consts<KIND>;
     using K = typename C::K;
     using V = typename C::V;
-    const int64_t c = blockIdx.x;
-    const int64_t first = c * kRangeChunk;
+    using I = typename slot_image<KIND>::type;
+    constexpr int ITEMS = range_tile<KIND>::items;
+    constexpr int kWarpCount = kThreads / 32;
+    __shared__ unsigned int s_run;
+    __shared__ unsigned int s_warp[kWarpCount];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    __shared__ unsigned int warp_base[kThreads / 32];
-    __shared__ unsigned int round_base;
     if (threadIdx.x == 0)
     {
-        round_base = chunk_offsets[c];
+        s_run = atomicAdd(words + runs, 1u);
     }
     __syncthreads();
-    for (int r = 0; r < kRangeChunk / kThreads; ++r)
-    {
-        const int64_t s = first + r * kThreads + threadIdx.x;
-        bool live = false;
-        K k = C::empty_key;
-        if (s < t.total)
-        {
-            k = __ldcg(reinterpret_cast<const K*>(t.slots + s * C::slot_bytes));
-            live = (k != C::empty_key && k != C::tomb_key);
-        }
-        const unsigned b = __ballot_sync(0xffffffffu, live);
+    const int run = static_cast<int>(s_run);
+    const int64_t tile_lo = tiles * (static_cast<int64_t>(run) * kWarpCount + warp) / (static_cast<int64_t>(runs) * kWarpCount);
+    const int64_t tile_hi =
+            tiles * (static_cast<int64_t>(run) * kWarpCount + warp + 1) / (static_cast<int64_t>(runs) * kWarpCount);
+    // slot of row 0 of the lane in a tile: its ITEMS rows of 32 slots lie one after another
+    const auto first_slot = [&](int64_t tile) { return static_cast<uint32_t>(tile * range_tile<KIND>::slots) + lane; };
+    // sum over the block, and over the warps before the caller's
+    const auto block_sum = [&](unsigned int x, unsigned int& before) {
+        __syncthreads();
+        x = __reduce_add_sync(0xffffffffu, x);
         if (lane == 0)
         {
-            warp_base[warp] = __popc(b);
+            s_warp[warp] = x;
         }
         __syncthreads();
-        unsigned int before = round_base;
-        for (int w = 0; w < warp; ++w)
+        unsigned int sum = 0u;
+        before = 0u;
+#pragma unroll
+        for (int w = 0; w < kWarpCount; ++w)
         {
-            before += warp_base[w];
+            before += w < warp ? s_warp[w] : 0u;
+            sum += s_warp[w];
         }
-        if (live)
+        return sum;
+    };
+    unsigned int live = 0u; // of the warp
+    for (int64_t tile = tile_lo; tile < tile_hi; ++tile)
+    {
+        const uint32_t first = first_slot(tile);
+        K key[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
         {
-            const unsigned int pos = before + __popc(b & ((1u << lane) - 1u));
+            const uint32_t slot = first + r * 32;
+            key[r] = slot < t.total
+                             ? *reinterpret_cast<const K*>(t.slots + static_cast<uint64_t>(slot) * C::slot_bytes)
+                             : C::empty_key;
+        }
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+        {
+            live += __popc(__ballot_sync(0xffffffffu, key[r] < C::tomb_key));
+        }
+    }
+    unsigned int warps_before, unused;
+    const unsigned int total = block_sum(lane == 0 ? live : 0u, warps_before);
+    if (threadIdx.x == 0)
+    {
+        asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(words + run), "r"(total + 1u) : "memory");
+    }
+    unsigned int earlier = 0u;
+    for (int r = static_cast<int>(threadIdx.x); r < run; r += kThreads)
+    {
+        unsigned int v = 0u;
+        for (int polls = 0; polls < kRangePolls; ++polls)
+        {
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(words + r) : "memory");
+            if (v != 0u)
+            {
+                break;
+            }
+            __nanosleep(100);
+        }
+        if (v == 0u)
+        {
+            atomicOr(&t.hdr->error, kErrRange);
+        }
+        else
+        {
+            earlier += v - 1u;
+        }
+    }
+    const unsigned int base = block_sum(earlier, unused);
+    // position behind the tiles not yet written
+    unsigned int end = base + warps_before + live;
+    for (int64_t tile = tile_hi - 1; tile >= tile_lo; --tile)
+    {
+        const uint32_t first = first_slot(tile);
+        I image[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+        {
+            const uint32_t slot = first + r * 32;
+            if (slot < t.total)
+            {
+                image[r] = __ldcs(reinterpret_cast<const I*>(t.slots) + slot);
+            }
+        }
+        unsigned int rows[ITEMS];
+        unsigned int count = 0u;
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+        {
+            K key;
+            V val;
+            unpack_element<KIND>(image[r], key, val);
+            rows[r] = __ballot_sync(0xffffffffu, first + r * 32 < t.total && key < C::tomb_key);
+            count += __popc(rows[r]);
+        }
+        end -= count;
+        unsigned int row = end;
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+        {
+            K key;
+            V val;
+            unpack_element<KIND>(image[r], key, val);
+            const unsigned b = rows[r];
+            if ((b >> lane) & 1u)
+            {
+                const unsigned int pos = row + __popc(b & ((1u << lane) - 1u));
+                if constexpr (SLOTS)
+                {
+                    out_slots[pos] = static_cast<int32_t>(first + r * 32);
+                }
+                else
+                {
+                    if (out_keys != nullptr)
+                    {
+                        reinterpret_cast<K*>(out_keys)[pos] = key;
+                    }
+                    if constexpr (kind_traits<KIND>::is_map)
+                    {
+                        if (out_vals != nullptr)
+                        {
+                            reinterpret_cast<V*>(out_vals)[pos] = val;
+                        }
+                    }
+                }
+            }
+            row += __popc(b);
+        }
+    }
+    if (run == runs - 1 && threadIdx.x == 0)
+    {
+        // the out-of-band keys after the probed ones
+        unsigned int pos = base + total;
+        for (int sp = 0; sp < 2; ++sp)
+        {
+            if (t.hdr->special_state[sp] != 1u)
+            {
+                continue;
+            }
+            const uint32_t slot = t.num_groups * C::slots_per_group + sp;
             if constexpr (SLOTS)
             {
-                out_slots[pos] = static_cast<int32_t>(s);
+                out_slots[pos] = static_cast<int32_t>(slot);
             }
             else
             {
                 if (out_keys != nullptr)
                 {
-                    reinterpret_cast<K*>(out_keys)[pos] = k;
+                    reinterpret_cast<K*>(out_keys)[pos] = sp == 0 ? C::empty_key : C::tomb_key;
                 }
                 if constexpr (kind_traits<KIND>::is_map)
                 {
                     if (out_vals != nullptr)
                     {
                         reinterpret_cast<V*>(out_vals)[pos] = *reinterpret_cast<const V*>(
-                                t.slots + s * C::slot_bytes + kind_traits<KIND>::val_offset);
+                                t.slots + static_cast<uint64_t>(slot) * C::slot_bytes + kind_traits<KIND>::val_offset);
                     }
-                }
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            unsigned int add = 0;
-            for (int w = 0; w < kThreads / 32; ++w)
-            {
-                add += warp_base[w];
-            }
-            round_base += add;
-        }
-        __syncthreads();
-    }
-}
-
-// Appends the out-of-band keys (keys / mapped values) after the probed ones.
-template <int KIND>
-__global__ void
-k_range_specials(dview t, const unsigned int* chunk_offsets, int64_t nchunks, const unsigned int* last_count,
-                 void* out_keys, void* out_vals)
-{
-    using C = kind_consts<KIND>;
-    using K = typename C::K;
-    using V = typename C::V;
-    unsigned long long pos = static_cast<unsigned long long>(chunk_offsets[nchunks - 1]) + *last_count;
-    for (int sp = 0; sp < 2; ++sp)
-    {
-        if (t.hdr->special_state[sp] == 1u)
-        {
-            const int64_t slot = static_cast<int64_t>(t.num_groups) * C::slots_per_group + sp;
-            if (out_keys != nullptr)
-            {
-                reinterpret_cast<K*>(out_keys)[pos] = sp == 0 ? C::empty_key : C::tomb_key;
-            }
-            if constexpr (kind_traits<KIND>::is_map)
-            {
-                if (out_vals != nullptr)
-                {
-                    reinterpret_cast<V*>(out_vals)[pos] =
-                            *reinterpret_cast<const V*>(t.slots + slot * C::slot_bytes + kind_traits<KIND>::val_offset);
                 }
             }
             ++pos;
         }
+        t.hdr->count = pos;
     }
 }
 
@@ -2292,30 +2302,31 @@ struct do_range
     static sg_status
     run(sg_unordered* t, int32_t* out_slots, void* out_keys, void* out_vals, cudaStream_t s)
     {
-        const int64_t nch = t->nchunks;
-        k_range_count<KIND><<<static_cast<unsigned>(nch), kThreads, 0, s>>>(view_of(t), t->chunk_counts);
-        SG_LAUNCH_CHECK();
-        // keep the last chunk's count for the tail append before the scan overwrites it
-        SG_CUDA_TRY(cudaMemcpyAsync(t->chunk_counts + nch, t->chunk_counts + nch - 1, sizeof(unsigned int),
-                                    cudaMemcpyDeviceToDevice, s));
-        const int64_t special_base = t->num_groups * (kGroupBytes / t->slot_bytes);
-        k_range_scan<<<1, 1024, 0, s>>>(t->chunk_counts, nch, t->hdr, out_slots, special_base, out_slots != nullptr);
-        SG_LAUNCH_CHECK();
+        const int64_t tiles = (t->total + range_tile<KIND>::slots - 1) / range_tile<KIND>::slots;
+        // a run per resident block; the words, and one, fit the counts' array
+        const auto launch = [&](auto kernel, int max_grid) {
+            const int runs = grid_for(tiles, 2 * kThreads / 32, max_grid);
+            SG_CUDA_TRY(cudaMemsetAsync(t->chunk_counts, 0, static_cast<size_t>(runs + 1) * sizeof(unsigned int), s));
+            kernel<<<runs, kThreads, 0, s>>>(view_of(t), t->chunk_counts, runs, tiles, out_slots, out_keys, out_vals);
+            return SG_OK;
+        };
+        static_assert(range_tile<KIND>::slots * 2 * (kThreads / 32) >= kRangeChunk, "at least as many words as runs");
+        sg_status st;
         if (out_slots != nullptr)
         {
-            k_range_write<KIND, true><<<static_cast<unsigned>(nch), kThreads, 0, s>>>(view_of(t), t->chunk_counts,
-                                                                                      out_slots, nullptr, nullptr);
-            SG_LAUNCH_CHECK();
+            static const int max_grid = persistent_grid(k_range<KIND, true>, kThreads);
+            st = launch(k_range<KIND, true>, max_grid);
         }
         else
         {
-            k_range_write<KIND, false><<<static_cast<unsigned>(nch), kThreads, 0, s>>>(view_of(t), t->chunk_counts,
-                                                                                       nullptr, out_keys, out_vals);
-            SG_LAUNCH_CHECK();
-            k_range_specials<KIND><<<1, 1, 0, s>>>(view_of(t), t->chunk_counts, nch, t->chunk_counts + nch, out_keys,
-                                                   out_vals);
-            SG_LAUNCH_CHECK();
+            static const int max_grid = persistent_grid(k_range<KIND, false>, kThreads);
+            st = launch(k_range<KIND, false>, max_grid);
         }
+        if (st != SG_OK)
+        {
+            return st;
+        }
+        SG_LAUNCH_CHECK();
         return SG_OK;
     }
 };
@@ -3072,7 +3083,7 @@ sg_unordered_device_range(sg_unordered* t, int32_t* out_slots, void* stream, int
         return st;
     }
     *out_n = static_cast<int64_t>(host_header(t).count);
-    return SG_OK;
+    return (host_header(t).error & kErrRange) != 0u ? SG_ERR_RETRY_EXHAUSTED : SG_OK;
 }
 
 sg_status
@@ -3095,7 +3106,7 @@ sg_unordered_range_copy(sg_unordered* t, void* out_keys, void* out_mapped, void*
         return st;
     }
     *out_n = static_cast<int64_t>(host_header(t).count);
-    return SG_OK;
+    return (host_header(t).error & kErrRange) != 0u ? SG_ERR_RETRY_EXHAUSTED : SG_OK;
 }
 
 sg_status
