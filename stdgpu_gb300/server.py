@@ -6,14 +6,19 @@ requests and keeps each request's device buffers alive until it completes.
 
 from __future__ import annotations
 
-from ctypes import byref, c_double, c_int32, c_int64, c_void_p
+from ctypes import POINTER, byref, c_double, c_int32, c_int64, c_void_p
 
+import numpy as np
 import torch
 
 from . import _native as N
 from .containers import KINDS, _as_bits, _INT_DTYPE, _KEY_BYTES, _MAPPED_BYTES, _ptr
 
 INSERT, FIND, ERASE = 0, 1, 2
+
+# sg_request as an array element
+REQUEST = np.dtype([("table", np.int32), ("op", np.int32), ("n", np.int64), ("keys", np.uint64), ("mapped", np.uint64),
+                    ("out_mapped", np.uint64), ("out_flags", np.uint64)])
 
 
 class server:
@@ -48,8 +53,7 @@ class server:
         keys = _as_bits(keys, self.key_bytes, "keys")
         if mapped is not None:
             mapped = _as_bits(mapped, self.mapped_bytes, "mapped")
-        r = N.sg_request(int(table), int(op), keys.numel(), _ptr(keys).value, _ptr(mapped).value,
-                         _ptr(out_mapped).value, _ptr(out_flags).value)
+        r = N.sg_request(int(table), int(op), keys.numel(), _ptr(keys), _ptr(mapped), _ptr(out_mapped), _ptr(out_flags))
         t = c_int64()
         N.check(N.load().sg_server_submit(self._h, byref(r), byref(t)), "server::submit")
         self._live[t.value] = (keys, mapped, out_mapped, out_flags)
@@ -57,17 +61,21 @@ class server:
 
     def submit_many(self, items) -> list[int]:
         """items: (table, op, keys, mapped, out_mapped, out_flags) tuples, submitted in order in one call."""
+        # the request records are filled as one array of plain numbers (REQUEST lies as sg_request does)
         n = len(items)
-        arr = (N.sg_request * n)()
-        for k, (table, op, keys, mapped, out_mapped, out_flags) in enumerate(items):
+        rows = []
+        held = []
+        for table, op, keys, mapped, out_mapped, out_flags in items:
             keys = _as_bits(keys, self.key_bytes, "keys")
-            arr[k] = N.sg_request(int(table), int(op), keys.numel(), _ptr(keys).value, _ptr(mapped).value,
-                                  _ptr(out_mapped).value, _ptr(out_flags).value)
-        tickets = (c_int64 * n)()
-        N.check(N.load().sg_server_submit_many(self._h, arr, n, tickets), "server::submit_many")
-        out = list(tickets)
-        for tk, it in zip(out, items):
-            self._live[tk] = it
+            rows.append((table, op, keys.numel(), _ptr(keys) or 0, _ptr(mapped) or 0, _ptr(out_mapped) or 0,
+                         _ptr(out_flags) or 0))
+            held.append((keys, mapped, out_mapped, out_flags))
+        arr = np.array(rows, dtype=REQUEST)
+        tickets = np.empty(n, dtype=np.int64)
+        N.check(N.load().sg_server_submit_many(self._h, arr.ctypes.data_as(POINTER(N.sg_request)), n,
+                                               tickets.ctypes.data_as(POINTER(c_int64))), "server::submit_many")
+        out = tickets.tolist()
+        self._live.update(zip(out, held))
         return out
 
     def set_policy(self, direct_keys: int = 1 << 16, chunk_keys: int = 1 << 22, max_direct: int = 8,
