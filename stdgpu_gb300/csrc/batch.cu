@@ -259,7 +259,6 @@ struct sg_table_batch
     init_chunk* chunks;      // device
     int64_t nchunks;
     int64_t* prefix;         // device, n + 1
-    long long* sizes_dev;    // device, n
     long long* sizes_host;   // pinned, n
     int64_t arena_bytes;
     unsigned int* locks;     // stripe locks of native device inserts, shared by the batch's tables
@@ -477,10 +476,6 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
     }
     if (e == cudaSuccess)
     {
-        e = sg::detail::dev_malloc(&b->sizes_dev, sizeof(long long) * n_tables);
-    }
-    if (e == cudaSuccess)
-    {
         e = cudaMallocHost(&b->sizes_host, sizeof(long long) * n_tables);
     }
     if (e == cudaSuccess)
@@ -541,7 +536,6 @@ sg_batch_destroy(sg_table_batch* b)
     sg::detail::dev_free(b->views);
     sg::detail::dev_free(b->chunks);
     sg::detail::dev_free(b->prefix);
-    sg::detail::dev_free(b->sizes_dev);
     sg::detail::dev_free(b->locks);
     if (b->sizes_host != nullptr)
     {
@@ -637,9 +631,8 @@ sg_batch_sizes(sg_table_batch* b, void* stream, int64_t* out_sizes)
         return SG_ERR_BAD_ARG;
     }
     cudaStream_t s = as_stream(stream);
-    k_batch_gather_sizes<<<(b->n + 255) / 256, 256, 0, s>>>(b->views, b->n, b->sizes_dev);
+    k_batch_gather_sizes<<<(b->n + 255) / 256, 256, 0, s>>>(b->views, b->n, b->sizes_host); // pinned
     SG_LAUNCH_CHECK();
-    SG_CUDA_TRY(cudaMemcpyAsync(b->sizes_host, b->sizes_dev, sizeof(long long) * b->n, cudaMemcpyDeviceToHost, s));
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     for (int32_t t = 0; t < b->n; ++t)
     {

