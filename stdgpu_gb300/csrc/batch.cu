@@ -11,11 +11,13 @@
 // can be captured in a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <new>
 #include <vector>
 
+#include "region_build.cuh"
 #include "sg_internal.cuh"
 #include "stdgpu_gb300.h"
 #include "table_core.cuh"
@@ -35,41 +37,67 @@ struct init_chunk
     int64_t unit_end;
 };
 
-// Prefix of tile counts: prefix[t] = sum over u < t of ceil(n_u / 32); prefix[n] = all tiles.
-__global__ void __launch_bounds__(1024)
-k_batch_tiles(const int64_t* offsets, int32_t n, int64_t* prefix, bool has_keys)
+// Exclusive scan over the tables t < n of count(t) into prefix[0, n], prefix[n] = the sum, by one block of 1024
+// threads.  The threads' sums go through warp shuffles (one thread walking all 1024 of them took most of the 12 us
+// that the tiles of 4096 tables took; now 6).
+template <typename Count>
+SG_D void
+scan_tables(int32_t n, int64_t* prefix, Count count)
 {
-    __shared__ long long part[1024];
+    __shared__ long long warp_sums[32];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
     const int64_t per = (static_cast<int64_t>(n) + blockDim.x - 1) / blockDim.x;
     const int64_t lo = threadIdx.x * per;
     const int64_t hi = lo + per < n ? lo + per : n;
     long long s = 0;
     for (int64_t t = lo; t < hi; ++t)
     {
-        const int64_t cnt = has_keys ? offsets[t + 1] - offsets[t] : 0;
-        s += cnt > 0 ? (cnt + 31) / 32 : 0;
+        s += count(t);
     }
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0)
+    long long incl = s;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1)
     {
-        long long run = 0;
-        for (int w = 0; w < static_cast<int>(blockDim.x); ++w)
-        {
-            const long long x = part[w];
-            part[w] = run;
-            run += x;
-        }
-        prefix[n] = run;
+        const long long x = __shfl_up_sync(0xffffffffu, incl, d);
+        incl += lane >= d ? x : 0;
+    }
+    if (lane == 31)
+    {
+        warp_sums[warp] = incl;
     }
     __syncthreads();
-    long long run = part[threadIdx.x];
+    long long run = incl - s;
+    for (int w = 0; w < warp; ++w)
+    {
+        run += warp_sums[w];
+    }
     for (int64_t t = lo; t < hi; ++t)
     {
         prefix[t] = run;
-        const int64_t cnt = has_keys ? offsets[t + 1] - offsets[t] : 0;
-        run += cnt > 0 ? (cnt + 31) / 32 : 0;
+        run += count(t);
     }
+    if (threadIdx.x == blockDim.x - 1)
+    {
+        prefix[n] = run;
+    }
+}
+
+SG_D long long
+tiles_of(const int64_t* offsets, int64_t t, int tile)
+{
+    const int64_t cnt = offsets[t + 1] - offsets[t];
+    return cnt > 0 ? (cnt + tile - 1) / tile : 0;
+}
+
+// Prefix of tile counts: prefix[t] = sum over u < t of ceil(n_u / 32); prefix[n] = all tiles.  Tables whose `todo`
+// (nullable) is 0 have no tiles.
+__global__ void __launch_bounds__(1024)
+k_batch_tiles(const int64_t* offsets, int32_t n, int64_t* prefix, bool has_keys, const uint8_t* todo)
+{
+    scan_tables(n, prefix, [&](int64_t t) -> long long {
+        return has_keys && (todo == nullptr || todo[t] != 0) ? tiles_of(offsets, t, 32) : 0;
+    });
 }
 
 // Table of tile x: the last t with prefix[t] <= x (binary search by lane 0, broadcast to the warp).
@@ -97,15 +125,234 @@ tile_table(const int64_t* prefix, int32_t n, int64_t x)
     return __shfl_sync(0xffffffffu, t, 0);
 }
 
-SG_D unsigned long long
-warp_sum(unsigned long long v)
+// ---------------------------------------------------------------- inserts into empty tables (region_build.cuh)
+
+// A region of one table.
+struct build_item
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    int32_t table;
+    uint32_t first; // groups
+    uint32_t count;
+    int32_t whole; // the table's only region: its keys are read from the input, not from a list
+};
+
+constexpr int kListPer = 4; // elements per thread and tile of the lists
+
+// A key that found no room in its region, for the probe kernel.  More of them than the buffer holds mark their
+// tables todo.
+struct spill_entry
+{
+    uint4 image; // the slot's bytes (16, 8 or 4 of them)
+    int32_t table;
+    int32_t pad[3];
+};
+constexpr unsigned int kSpillMax = 1u << 15;
+
+struct spill_list
+{
+    unsigned int* count; // offered (may exceed kSpillMax)
+    spill_entry* entry;
+};
+
+// First launch of an insert into a batch that may be empty (one block): build[t] = 1 for a table that holds nothing
+// and gets at least a key per two groups (a region is written whole, so fewer keys are cheaper to insert one by one);
+// todo[t] = 1 for the others that get keys.  Tables of several regions get lists (prefix: their
+// tiles of list_tile elements), which leave no room for an element's index: with per-key flags they go to the probe
+// kernel.
+__global__ void __launch_bounds__(1024)
+k_batch_choose(const dview* views, const int64_t* offsets, int32_t n, const int32_t* first_item, bool flags, int tile,
+               uint8_t* build, uint8_t* todo, int64_t* prefix)
+{
+    for (int32_t t = threadIdx.x; t < n; t += blockDim.x)
     {
-        v += __shfl_xor_sync(0xffffffffu, v, o);
+        const dview v = views[t];
+        const int64_t cnt = offsets[t + 1] - offsets[t];
+        const int32_t regions = first_item[t + 1] - first_item[t];
+        const bool ok = cnt > 0 && 2 * cnt >= v.num_groups && regions > 0 && (regions == 1 || !flags) &&
+                        v.hdr->size == 0 && v.hdr->tombstones == 0;
+        build[t] = ok ? 1 : 0;
+        todo[t] = cnt > 0 && !ok ? 1 : 0;
     }
-    return v;
+    __syncthreads();
+    scan_tables(n, prefix, [&](int64_t t) -> long long {
+        return build[t] != 0 && first_item[t + 1] - first_item[t] > 1 ? tiles_of(offsets, t, tile) : 0;
+    });
+}
+
+// Second launch: the keys of the tables that are built and have several regions, appended to the lists in their
+// regions' slots.
+template <int KIND, bool AOS>
+__global__ void __launch_bounds__(kListThreads, 3)
+k_batch_lists(const dview* views, const int64_t* offsets, const int64_t* prefix, int32_t n, const int32_t* first_item,
+              unsigned int* fill, uint8_t* todo, const void* in0, const void* in1)
+{
+    using C = kind_consts<KIND>;
+    using E = typename slot_image<KIND>::type;
+    constexpr int PER = kListPer;
+    constexpr int64_t kTile = int64_t{ PER } * kListThreads;
+    extern __shared__ __align__(128) unsigned char smem[];
+    auto& s = *reinterpret_cast<list_tile<E, PER>*>(smem);
+    __shared__ int32_t s_table;
+    // a block takes consecutive tiles: one search, then the tables in order
+    const int64_t tiles = __ldg(prefix + n);
+    const int64_t x_lo = tiles * blockIdx.x / gridDim.x, x_hi = tiles * (blockIdx.x + 1) / gridDim.x;
+    if (x_lo == x_hi)
+    {
+        return;
+    }
+    if (threadIdx.x < 32)
+    {
+        const int32_t t = tile_table(prefix, n, x_lo);
+        if (threadIdx.x == 0)
+        {
+            s_table = t;
+        }
+    }
+    __syncthreads();
+    int32_t tb = s_table;
+    for (int64_t x = x_lo; x < x_hi; ++x)
+    {
+        while (__ldg(prefix + tb + 1) <= x)
+        {
+            ++tb;
+        }
+        const dview t = views[tb];
+        const int32_t i0 = __ldg(first_item + tb);
+        const int regions = __ldg(first_item + tb + 1) - i0;
+        const int64_t lo = __ldg(offsets + tb) + (x - __ldg(prefix + tb)) * kTile;
+        const int64_t hi = __ldg(offsets + tb + 1);
+        E elem[PER];
+        int rid[PER];
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+        {
+            const int64_t i = lo + j * kListThreads + threadIdx.x;
+            rid[j] = -1;
+            if (i < hi)
+            {
+                typename C::K key;
+                typename C::V val;
+                load_input<KIND, AOS>(in0, in1, i, key, val);
+                if (key >= C::tomb_key)
+                {
+                    if (special_insert<KIND>(t, key, val) != 0)
+                    {
+                        atomicAdd(&t.hdr->size, 1ull);
+                    }
+                }
+                else
+                {
+                    elem[j] = pack_element<KIND>(key, val);
+                    rid[j] = static_cast<int>(home_of<KIND>(t, key) >> kRegionGroupsLog2);
+                }
+            }
+        }
+        const bool lost = append_to_lists<E, PER>(
+                s, regions, elem, rid, fill + i0,
+                [&](int r, unsigned int k) {
+                    return reinterpret_cast<E*>(t.slots + (static_cast<uint64_t>(r) << (kRegionGroupsLog2 + 7))) + k;
+                },
+                [&](int r) {
+                    return min(t.num_groups - (static_cast<uint32_t>(r) << kRegionGroupsLog2), kRegionGroups) *
+                           C::slots_per_group;
+                });
+        if (lost)
+        {
+            todo[tb] = 1;
+        }
+    }
+}
+
+// Third launch: one region per block.  Spilled keys go to the probe kernel one by one.  A table some of whose keys
+// found no room in a list is marked todo: the probe kernel then runs over all its keys, which changes nothing for
+// those stored here.
+template <int KIND, bool AOS>
+__global__ void __launch_bounds__(kRegionThreads, kRegionBlocks)
+k_batch_build(const dview* views, const int64_t* offsets, const build_item* items, const uint8_t* build,
+              const unsigned int* fill, uint8_t* todo, const void* in0, const void* in1, uint8_t* out_flags,
+              spill_list spills)
+{
+    using C = kind_consts<KIND>;
+    using K = typename C::K;
+    using V = typename C::V;
+    using E = typename slot_image<KIND>::type;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const build_item it = items[blockIdx.x];
+    const dview t = views[it.table];
+    const int64_t lo = __ldg(offsets + it.table), hi = __ldg(offsets + it.table + 1);
+    const unsigned int listed = fill[blockIdx.x];
+    if (__ldg(build + it.table) == 0)
+    {
+        return;
+    }
+    const region r{ reinterpret_cast<char*>(smem), it.first, it.count, it.whole != 0 };
+    region_start<KIND>(t, r);
+    __syncthreads();
+    const E* const list = reinterpret_cast<const E*>(t.slots + (static_cast<uint64_t>(it.first) << 7));
+    const int64_t count = it.whole != 0 ? hi - lo
+                                        : static_cast<int64_t>(min(listed, it.count * C::slots_per_group));
+    unsigned int done = 0, refused = 0;
+    constexpr int kAhead = 4; // keys loaded before any is inserted
+    for (int64_t base = threadIdx.x; base < count; base += kAhead * kRegionThreads)
+    {
+        K key[kAhead];
+        V val[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+        {
+            const int64_t i = base + j * kRegionThreads;
+            if (i < count)
+            {
+                if (it.whole != 0)
+                {
+                    load_input<KIND, AOS>(in0, in1, lo + i, key[j], val[j]);
+                }
+                else
+                {
+                    unpack_element<KIND>(__ldcg(list + i), key[j], val[j]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+        {
+            const int64_t i = base + j * kRegionThreads;
+            if (i >= count)
+            {
+                break;
+            }
+            const int res = key[j] >= C::tomb_key
+                                    ? special_insert<KIND>(t, key[j], val[j])
+                                    : region_insert<KIND>(r, home_of<KIND>(t, key[j]) - it.first,
+                                                          rot_of(static_cast<uint64_t>(key[j])), key[j], val[j]);
+            done += (res == kRegionInserted);
+            refused += (res == kRegionRefused);
+            if (res == kRegionSpill)
+            {
+                const unsigned int k = atomicAdd(spills.count, 1u);
+                if (k < kSpillMax)
+                {
+                    spill_entry x{};
+                    *reinterpret_cast<E*>(&x.image) = pack_element<KIND>(key[j], val[j]);
+                    x.table = it.table;
+                    spills.entry[k] = x;
+                }
+                else
+                {
+                    todo[it.table] = 1;
+                }
+            }
+            if (out_flags != nullptr)
+            {
+                out_flags[lo + i] = static_cast<uint8_t>(res == kRegionInserted);
+            }
+        }
+    }
+    __syncthreads(); // the list, which lies in the region's slots, is read
+    region_write(t, r);
+    unsigned int c[2] = { done, refused };
+    unsigned long long* const dst[2] = { &t.hdr->size, &t.hdr->refused };
+    region_add<2>(c, dst);
 }
 
 enum batch_op : int
@@ -117,42 +364,71 @@ enum batch_op : int
     kOpContains = 4
 };
 
-// Persistent walk over the tile list; each warp takes `tiles_per_step` consecutive tiles at a time.
+// Persistent walk over the tile list; each warp takes up to `tiles_per_step` consecutive tiles at a time (fewer when
+// there are not that many for every warp).  Bound by the probes' instructions and L2 reads; what a step pays beyond
+// its probes is the search for its first table, a dozen dependent loads.  25.8 M queries over 4096 tables: 449 us
+// with 8 tiles a step, 483 with 4, 719 with 1, 564 with a search and a view per tile at 4 a step.
 template <int KIND, int OP, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 k_batch(const dview* views, const int64_t* offsets, const int64_t* prefix, int32_t n, int tiles_per_step,
-        const void* in0, const void* in1, void* out_vals, uint8_t* out_flags)
+        const void* in0, const void* in1, void* out_vals, uint8_t* out_flags, const uint8_t* built,
+        spill_list spills)
 {
     const tile_lanes L;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     const int64_t tiles = __ldg(prefix + n);
     unsigned long long retry = 0;
+    const int64_t share = tiles / nwarps;
+    tiles_per_step = share < tiles_per_step ? (share < 1 ? 1 : static_cast<int>(share)) : tiles_per_step;
     for (int64_t x0 = warp * tiles_per_step; x0 < tiles; x0 += nwarps * tiles_per_step)
     {
         const int64_t x1 = x0 + tiles_per_step < tiles ? x0 + tiles_per_step : tiles;
-        for (int64_t x = x0; x < x1; ++x)
+        // one search per step, then the tables in order; a table's counts are added once per step
+        int32_t tb = tile_table(prefix, n, x0);
+        int64_t next = __ldg(prefix + tb + 1); // first tile of the table after
+        for (int64_t x = x0; x < x1;)
         {
-            const int32_t tb = tile_table(prefix, n, x);
+            while (next <= x)
+            {
+                ++tb;
+                next = __ldg(prefix + tb + 1);
+            }
             const dview t = views[tb];
             const int64_t end = __ldg(offsets + tb + 1);
-            const int64_t i = __ldg(offsets + tb) + (x - __ldg(prefix + tb)) * 32 + L.lane;
-            const bool valid = i < end;
+            int64_t i = __ldg(offsets + tb) + (x - __ldg(prefix + tb)) * 32 + L.lane;
             step_counts c;
+            for (const int64_t stop = next < x1 ? next : x1; x < stop; ++x, i += 32)
+            {
+                const bool valid = i < end;
+                if constexpr (OP == kOpInsertAos || OP == kOpInsertSoa)
+                {
+                    insert_step<KIND, OP == kOpInsertAos>(t, L, in0, in1, i, valid, out_flags, c);
+                }
+                else if constexpr (OP == kOpErase)
+                {
+                    erase_step<KIND>(t, L, in0, i, valid, out_flags, c);
+                }
+                else
+                {
+                    find_step<KIND, OP == kOpFind>(t, L, in0, i, valid, out_vals, out_flags);
+                }
+            }
             if constexpr (OP == kOpInsertAos || OP == kOpInsertSoa)
             {
-                insert_step<KIND, OP == kOpInsertAos>(t, L, in0, in1, i, valid, out_flags, c);
-                const unsigned long long d = warp_sum(c.done), r = warp_sum(c.refused), u = warp_sum(c.reused);
+                const unsigned int d = __reduce_add_sync(0xffffffffu, c.done);
+                const unsigned int r = __reduce_add_sync(0xffffffffu, c.refused);
+                const unsigned int u = __reduce_add_sync(0xffffffffu, c.reused);
                 retry += c.retry;
                 if (L.lane == 0)
                 {
                     if (d != 0)
                     {
-                        atomicAdd(&t.hdr->size, d);
+                        atomicAdd(&t.hdr->size, static_cast<unsigned long long>(d));
                     }
                     if (r != 0)
                     {
-                        atomicAdd(&t.hdr->refused, r);
+                        atomicAdd(&t.hdr->refused, static_cast<unsigned long long>(r));
                     }
                     if (u != 0)
                     {
@@ -162,17 +438,34 @@ k_batch(const dview* views, const int64_t* offsets, const int64_t* prefix, int32
             }
             else if constexpr (OP == kOpErase)
             {
-                erase_step<KIND>(t, L, in0, i, valid, out_flags, c);
-                const unsigned long long d = warp_sum(c.done), o = warp_sum(c.oob);
+                const unsigned int d = __reduce_add_sync(0xffffffffu, c.done);
+                const unsigned int o = __reduce_add_sync(0xffffffffu, c.oob);
                 if (L.lane == 0 && d != 0)
                 {
                     atomicAdd(&t.hdr->size, 0ull - d);
-                    atomicAdd(&t.hdr->tombstones, d - o);
+                    atomicAdd(&t.hdr->tombstones, static_cast<unsigned long long>(d - o));
                 }
             }
-            else
+        }
+    }
+    if constexpr (OP == kOpInsertAos || OP == kOpInsertSoa)
+    {
+        // keys that found no room in their region, one per warp step (their tables differ)
+        const int64_t spilled = built != nullptr ? min(*spills.count, kSpillMax) : 0u;
+        for (int64_t e = warp; e < spilled; e += nwarps)
+        {
+            const spill_entry x = spills.entry[e];
+            const dview t = views[x.table];
+            typename kind_consts<KIND>::K key;
+            typename kind_consts<KIND>::V val;
+            unpack_element<KIND>(*reinterpret_cast<const typename slot_image<KIND>::type*>(&x.image), key, val);
+            step_counts c;
+            insert_kv_step<KIND>(t, L, key, val, 0, L.lane == 0, nullptr, c);
+            retry += c.retry;
+            if (L.lane == 0)
             {
-                find_step<KIND, OP == kOpFind>(t, L, in0, i, valid, out_vals, out_flags);
+                atomicAdd(c.done != 0 ? &t.hdr->size : &t.hdr->refused,
+                          static_cast<unsigned long long>(c.done + c.refused));
             }
         }
     }
@@ -259,9 +552,20 @@ struct sg_table_batch
     init_chunk* chunks;      // device
     int64_t nchunks;
     int64_t* prefix;         // device, n + 1
+    long long* sizes_dev;    // device, n
     long long* sizes_host;   // pinned, n
     int64_t arena_bytes;
     unsigned int* locks;     // stripe locks of native device inserts, shared by the batch's tables
+    // Inserts into empty tables: the regions, table by table; per table its first region (n + 1), the two marks of a
+    // call and the prefix of its lists' tiles; per region the length of its list.
+    build_item* items;       // device
+    int64_t n_items;
+    int32_t* first_item;     // device, n + 1
+    uint8_t* marks;          // device, 2 n
+    unsigned int* fill;      // device, n_items
+    int64_t* list_prefix;    // device, n + 1
+    spill_list spills;       // device
+    bool maybe_empty;        // cleared or created since the last insert: tries the build (the device decides per table)
 };
 
 constexpr int64_t kBatchInsertLocks = int64_t{ 1 } << 16;
@@ -287,7 +591,7 @@ struct batch_launch
     template <int OP, int THREADS>
     static sg_status
     go(sg_table_batch* b, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
-       uint8_t* out_flags, cudaStream_t s)
+       uint8_t* out_flags, const uint8_t* built, cudaStream_t s)
     {
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<KIND, OP, THREADS>, THREADS, 0);
@@ -295,7 +599,7 @@ struct batch_launch
         const int want = b->blocks_per_sm > 0 ? (b->blocks_per_sm < per_sm ? b->blocks_per_sm : per_sm) : per_sm;
         k_batch<KIND, OP, THREADS><<<b->sms * want, THREADS, 0, s>>>(b->views, offsets, b->prefix, b->n,
                                                                       b->tiles_per_step, in0, in1, out_vals,
-                                                                      out_flags);
+                                                                      out_flags, built, b->spills);
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -303,36 +607,63 @@ struct batch_launch
     template <int OP>
     static sg_status
     run_op(sg_table_batch* b, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
-           uint8_t* out_flags, cudaStream_t s)
+           uint8_t* out_flags, const uint8_t* built, cudaStream_t s)
     {
         switch (b->threads)
         {
             case 128:
-                return go<OP, 128>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return go<OP, 128>(b, offsets, in0, in1, out_vals, out_flags, built, s);
             case 512:
-                return go<OP, 512>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return go<OP, 512>(b, offsets, in0, in1, out_vals, out_flags, built, s);
             default:
-                return go<OP, 256>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return go<OP, 256>(b, offsets, in0, in1, out_vals, out_flags, built, s);
         }
     }
 
     static sg_status
     run(sg_table_batch* b, int op, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
-        uint8_t* out_flags, cudaStream_t s)
+        uint8_t* out_flags, const uint8_t* built, cudaStream_t s)
     {
         switch (op)
         {
             case kOpInsertAos:
-                return run_op<kOpInsertAos>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return run_op<kOpInsertAos>(b, offsets, in0, in1, out_vals, out_flags, built, s);
             case kOpInsertSoa:
-                return run_op<kOpInsertSoa>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return run_op<kOpInsertSoa>(b, offsets, in0, in1, out_vals, out_flags, built, s);
             case kOpErase:
-                return run_op<kOpErase>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return run_op<kOpErase>(b, offsets, in0, in1, out_vals, out_flags, built, s);
             case kOpFind:
-                return run_op<kOpFind>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return run_op<kOpFind>(b, offsets, in0, in1, out_vals, out_flags, built, s);
             default:
-                return run_op<kOpContains>(b, offsets, in0, in1, out_vals, out_flags, s);
+                return run_op<kOpContains>(b, offsets, in0, in1, out_vals, out_flags, built, s);
         }
+    }
+
+    // The tables of an insert that are built; the others are marked todo for the probe kernel.
+    template <bool AOS>
+    static sg_status
+    build(sg_table_batch* b, const int64_t* offsets, const void* in0, const void* in1, uint8_t* out_flags,
+          cudaStream_t s)
+    {
+        using Lists = list_tile<typename slot_image<KIND>::type, kListPer>;
+        uint8_t* const todo = b->marks + b->n;
+        // the lists' lengths, and the spill count behind them
+        SG_CUDA_TRY(cudaMemsetAsync(b->fill, 0, sizeof(unsigned int) * static_cast<size_t>(b->n_items + 1), s));
+        k_batch_choose<<<1, 1024, 0, s>>>(b->views, offsets, b->n, b->first_item, out_flags != nullptr,
+                                          kListPer * kListThreads, b->marks, todo, b->list_prefix);
+        SG_LAUNCH_CHECK();
+        SG_CUDA_TRY(cudaFuncSetAttribute(k_batch_lists<KIND, AOS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(sizeof(Lists))));
+        static const int lists_grid = persistent_grid(k_batch_lists<KIND, AOS>, kListThreads, sizeof(Lists));
+        k_batch_lists<KIND, AOS><<<lists_grid, kListThreads, sizeof(Lists), s>>>(
+                b->views, offsets, b->list_prefix, b->n, b->first_item, b->fill, todo, in0, in1);
+        SG_LAUNCH_CHECK();
+        SG_CUDA_TRY(cudaFuncSetAttribute(k_batch_build<KIND, AOS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(kRegionBytes)));
+        k_batch_build<KIND, AOS><<<static_cast<unsigned>(b->n_items), kRegionThreads, kRegionBytes, s>>>(
+                b->views, offsets, b->items, b->marks, b->fill, todo, in0, in1, out_flags, b->spills);
+        SG_LAUNCH_CHECK();
+        return SG_OK;
     }
 
     static sg_status
@@ -345,27 +676,74 @@ struct batch_launch
     }
 };
 
+template <int KIND>
+sg_status
+build_kind(sg_table_batch* b, bool aos, const int64_t* offsets, const void* in0, const void* in1, uint8_t* out_flags,
+           cudaStream_t s)
+{
+    return aos ? batch_launch<KIND>::template build<true>(b, offsets, in0, in1, out_flags, s)
+               : batch_launch<KIND>::template build<false>(b, offsets, in0, in1, out_flags, s);
+}
+
+sg_status
+dispatch_build(sg_table_batch* b, bool aos, const int64_t* offsets, const void* in0, const void* in1,
+               uint8_t* out_flags, cudaStream_t s)
+{
+    switch (b->kind)
+    {
+        case 0:
+            return build_kind<0>(b, aos, offsets, in0, in1, out_flags, s);
+        case 1:
+            return build_kind<1>(b, aos, offsets, in0, in1, out_flags, s);
+        case 2:
+            return build_kind<2>(b, aos, offsets, in0, in1, out_flags, s);
+        case 3:
+            return build_kind<3>(b, aos, offsets, in0, in1, out_flags, s);
+        case 4:
+            return build_kind<4>(b, aos, offsets, in0, in1, out_flags, s);
+        case 5:
+            return build_kind<5>(b, aos, offsets, in0, in1, out_flags, s);
+        default:
+            return SG_ERR_BAD_ARG;
+    }
+}
+
 sg_status
 dispatch_op(sg_table_batch* b, int op, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
             uint8_t* out_flags, cudaStream_t s)
 {
+    const bool insert = op == kOpInsertAos || op == kOpInsertSoa;
+    const bool build = insert && b->maybe_empty && in0 != nullptr && b->n_items > 0;
+    if (insert && in0 != nullptr)
+    {
+        b->maybe_empty = false;
+    }
+    if (build)
+    {
+        const sg_status st = dispatch_build(b, op == kOpInsertAos, offsets, in0, in1, out_flags, s);
+        if (st != SG_OK)
+        {
+            return st;
+        }
+    }
+    const uint8_t* built = build ? b->marks : nullptr;
     // a NULL key array (all ranges empty, as an empty tensor gives) walks no tile
-    k_batch_tiles<<<1, 1024, 0, s>>>(offsets, b->n, b->prefix, in0 != nullptr);
+    k_batch_tiles<<<1, 1024, 0, s>>>(offsets, b->n, b->prefix, in0 != nullptr, build ? b->marks + b->n : nullptr);
     SG_LAUNCH_CHECK();
     switch (b->kind)
     {
         case 0:
-            return batch_launch<0>::run(b, op, offsets, in0, in1, out_vals, out_flags, s);
+            return batch_launch<0>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
         case 1:
-            return batch_launch<1>::run(b, op, offsets, in0, in1, out_vals, out_flags, s);
+            return batch_launch<1>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
         case 2:
-            return batch_launch<2>::run(b, op, offsets, in0, in1, out_vals, out_flags, s);
+            return batch_launch<2>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
         case 3:
-            return batch_launch<3>::run(b, op, offsets, in0, in1, out_vals, out_flags, s);
+            return batch_launch<3>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
         case 4:
-            return batch_launch<4>::run(b, op, offsets, in0, in1, out_vals, out_flags, s);
+            return batch_launch<4>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
         case 5:
-            return batch_launch<5>::run(b, op, offsets, in0, in1, out_vals, out_flags, s);
+            return batch_launch<5>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
         default:
             return SG_ERR_BAD_ARG;
     }
@@ -457,6 +835,22 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
         }
     }
     b->nchunks = static_cast<int64_t>(chunks.size());
+    std::vector<build_item> items;
+    std::vector<int32_t> first_item(n_tables + 1, 0);
+    for (int32_t t = 0; t < n_tables; ++t)
+    {
+        const int64_t regions = (groups[t] + kRegionGroups - 1) / kRegionGroups;
+        // (larger tables have no regions: their inserts fill the chip on their own)
+        for (int64_t k = 0; regions <= kListRegions && k < regions; ++k)
+        {
+            const int64_t g = k * kRegionGroups;
+            items.push_back(build_item{ t, static_cast<uint32_t>(g),
+                                        static_cast<uint32_t>(std::min<int64_t>(groups[t] - g, kRegionGroups)),
+                                        regions == 1 ? 1 : 0 });
+        }
+        first_item[t + 1] = static_cast<int32_t>(items.size());
+    }
+    b->n_items = static_cast<int64_t>(items.size());
     cudaError_t e = sg::detail::dev_malloc(&b->arena, static_cast<size_t>(b->arena_bytes));
     if (e == cudaSuccess)
     {
@@ -476,11 +870,40 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
     }
     if (e == cudaSuccess)
     {
+        e = sg::detail::dev_malloc(&b->sizes_dev, sizeof(long long) * n_tables);
+    }
+    if (e == cudaSuccess)
+    {
         e = cudaMallocHost(&b->sizes_host, sizeof(long long) * n_tables);
     }
     if (e == cudaSuccess)
     {
         e = sg::detail::dev_malloc(&b->locks, sizeof(unsigned int) * kBatchInsertLocks);
+    }
+    if (e == cudaSuccess && !items.empty())
+    {
+        e = sg::detail::dev_malloc(&b->items, sizeof(build_item) * items.size());
+    }
+    if (e == cudaSuccess && !items.empty())
+    {
+        e = sg::detail::dev_malloc(&b->fill, sizeof(unsigned int) * (items.size() + 1));
+        b->spills.count = b->fill + items.size();
+    }
+    if (e == cudaSuccess && !items.empty())
+    {
+        e = sg::detail::dev_malloc(&b->spills.entry, sizeof(spill_entry) * kSpillMax);
+    }
+    if (e == cudaSuccess)
+    {
+        e = sg::detail::dev_malloc(&b->first_item, sizeof(int32_t) * (n_tables + 1));
+    }
+    if (e == cudaSuccess)
+    {
+        e = sg::detail::dev_malloc(&b->list_prefix, sizeof(int64_t) * (n_tables + 1));
+    }
+    if (e == cudaSuccess)
+    {
+        e = sg::detail::dev_malloc(&b->marks, 2 * static_cast<size_t>(n_tables));
     }
     if (e == cudaSuccess)
     {
@@ -504,6 +927,15 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
     {
         e = cudaMemcpyAsync(b->chunks, chunks.data(), sizeof(init_chunk) * chunks.size(), cudaMemcpyHostToDevice, s);
     }
+    if (e == cudaSuccess && !items.empty())
+    {
+        e = cudaMemcpyAsync(b->items, items.data(), sizeof(build_item) * items.size(), cudaMemcpyHostToDevice, s);
+    }
+    if (e == cudaSuccess)
+    {
+        e = cudaMemcpyAsync(b->first_item, first_item.data(), sizeof(int32_t) * first_item.size(),
+                            cudaMemcpyHostToDevice, s);
+    }
     if (e == cudaSuccess)
     {
         e = cudaStreamSynchronize(s); // host vectors above are released on return
@@ -519,6 +951,7 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
         sg_batch_destroy(b);
         return st;
     }
+    b->maybe_empty = true;
     *out = b;
     return SG_OK;
 }
@@ -536,7 +969,14 @@ sg_batch_destroy(sg_table_batch* b)
     sg::detail::dev_free(b->views);
     sg::detail::dev_free(b->chunks);
     sg::detail::dev_free(b->prefix);
+    sg::detail::dev_free(b->sizes_dev);
     sg::detail::dev_free(b->locks);
+    sg::detail::dev_free(b->items);
+    sg::detail::dev_free(b->fill);
+    sg::detail::dev_free(b->spills.entry);
+    sg::detail::dev_free(b->first_item);
+    sg::detail::dev_free(b->list_prefix);
+    sg::detail::dev_free(b->marks);
     if (b->sizes_host != nullptr)
     {
         cudaFreeHost(b->sizes_host);
@@ -566,7 +1006,9 @@ sg_batch_clear(sg_table_batch* b, void* stream)
     {
         return SG_ERR_BAD_ARG;
     }
-    return dispatch_init(b, as_stream(stream));
+    const sg_status st = dispatch_init(b, as_stream(stream));
+    b->maybe_empty = b->maybe_empty || st == SG_OK;
+    return st;
 }
 
 sg_status
@@ -631,8 +1073,10 @@ sg_batch_sizes(sg_table_batch* b, void* stream, int64_t* out_sizes)
         return SG_ERR_BAD_ARG;
     }
     cudaStream_t s = as_stream(stream);
-    k_batch_gather_sizes<<<(b->n + 255) / 256, 256, 0, s>>>(b->views, b->n, b->sizes_host); // pinned
+    // by way of device memory: thousands of stores into host memory take the kernel longer than the copy
+    k_batch_gather_sizes<<<(b->n + 255) / 256, 256, 0, s>>>(b->views, b->n, b->sizes_dev);
     SG_LAUNCH_CHECK();
+    SG_CUDA_TRY(cudaMemcpyAsync(b->sizes_host, b->sizes_dev, sizeof(long long) * b->n, cudaMemcpyDeviceToHost, s));
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     for (int32_t t = 0; t < b->n; ++t)
     {

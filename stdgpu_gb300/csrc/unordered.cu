@@ -217,60 +217,6 @@ part_of(typename kind_consts<KIND>::K key, int bits, int shift)
     return static_cast<uint32_t>(fibonacci_bucket(static_cast<uint64_t>(key), bits)) >> shift;
 }
 
-template <int KIND>
-struct slot_image
-{
-    using type = typename std::conditional<kind_consts<KIND>::slot_bytes == 16, uint4,
-                                           typename std::conditional<kind_consts<KIND>::slot_bytes == 8, uint2,
-                                                                     unsigned int>::type>::type;
-};
-
-// A partitioned element of a table whose buckets come from caller-supplied hashes: the element's bytes and
-// its key's hash, so the ordered kernels need not read the hash array at random positions.
-template <typename E>
-struct with_hash
-{
-    E e;
-    uint64_t h;
-};
-
-// value_type bytes of (key, mapped); padding bytes are zero.
-template <int KIND>
-SG_D typename slot_image<KIND>::type
-pack_element(typename kind_consts<KIND>::K key, typename kind_consts<KIND>::V val)
-{
-    using K = typename kind_consts<KIND>::K;
-    using V = typename kind_consts<KIND>::V;
-    uint32_t w[4] = { 0u, 0u, 0u, 0u };
-    w[0] = static_cast<uint32_t>(key);
-    if constexpr (sizeof(K) == 8)
-    {
-        w[1] = static_cast<uint32_t>(static_cast<uint64_t>(key) >> 32);
-    }
-    if constexpr (kind_traits<KIND>::is_map)
-    {
-        constexpr int vo = kind_traits<KIND>::val_offset / 4;
-        w[vo] = static_cast<uint32_t>(val);
-        if constexpr (sizeof(V) == 8)
-        {
-            w[vo + 1] = static_cast<uint32_t>(static_cast<uint64_t>(val) >> 32);
-        }
-    }
-    constexpr int sb = kind_consts<KIND>::slot_bytes;
-    if constexpr (sb == 16)
-    {
-        return make_uint4(w[0], w[1], w[2], w[3]);
-    }
-    else if constexpr (sb == 8)
-    {
-        return make_uint2(w[0], w[1]);
-    }
-    else
-    {
-        return w[0];
-    }
-}
-
 // Scratch layout of a partitioned call: partition p owns elements [p * cap, (p + 1) * cap); elements past
 // a partition's capacity go to the overflow region [parts * cap, parts * cap + ocap); an element that finds
 // no room there either is not stored and sets *lost, and the direct kernel then runs over the whole input
@@ -655,31 +601,6 @@ struct staged_elem
 // The set kind holding the key type of KIND (erase partitions bare keys).
 template <int KIND>
 constexpr int keys_kind = sizeof(typename kind_consts<KIND>::K) == 8 ? SG_SET_U64 : SG_SET_U32;
-
-// key / mapped value of a value_type image (padding ignored)
-template <int KIND>
-SG_D void
-unpack_element(const typename slot_image<KIND>::type& e, typename kind_consts<KIND>::K& key,
-               typename kind_consts<KIND>::V& val)
-{
-    constexpr int sb = kind_consts<KIND>::slot_bytes;
-    if constexpr (sb == 16)
-    {
-        key = key_in_lane<KIND>(e, 0);
-        val = value_in_lane<KIND>(e, 0);
-    }
-    else if constexpr (sb == 8)
-    {
-        const uint4 q = make_uint4(e.x, e.y, 0u, 0u);
-        key = key_in_lane<KIND>(q, 0);
-        val = value_in_lane<KIND>(q, 0);
-    }
-    else
-    {
-        key = static_cast<typename kind_consts<KIND>::K>(e);
-        val = typename kind_consts<KIND>::V{};
-    }
-}
 
 // resident blocks per SM the ordered erase is compiled for (its step holds fewer values than the insert's):
 // 5 (48 registers) against 4 (64): 1.206 / 1.219 ms for the 2^25-key erase phase; 6 spills
