@@ -481,6 +481,31 @@ first_from(unsigned m, uint32_t o)
     return static_cast<int>((static_cast<uint32_t>(__ffs(r) - 1) + o) & (G - 1));
 }
 
+// A group's slots as the bytes of a word, sector j's S slots in the low bits of byte j: slot order is bit order, so
+// the first slot at or after slot o (cyclically) is the first set bit at or after o's bit.
+template <uint32_t S>
+SG_D uint32_t
+slot_bit(uint32_t slot)
+{
+    return S == 8 ? slot : (slot / S) * 8 + slot % S;
+}
+
+template <uint32_t S>
+SG_D uint32_t
+bit_slot(uint32_t bit)
+{
+    return S == 8 ? bit : (bit >> 3) * S + (bit & 7u);
+}
+
+// Bit of the first set bit of the word m (not 0) at or after slot o of the group's 4 S slots, cyclically.
+template <uint32_t S>
+SG_D uint32_t
+first_bit_from(uint32_t m, uint32_t o)
+{
+    const uint32_t b = slot_bit<S>(o & (4 * S - 1));
+    return (static_cast<uint32_t>(__ffs(__funnelshift_r(m, m, b)) - 1) + b) & 31u;
+}
+
 // G-bit mask of a group from the tile's four S-bit sector masks (lane q holds sector q).
 template <uint32_t S>
 SG_D unsigned
@@ -722,20 +747,43 @@ tile_nibble(unsigned ballot, int tbase)
     return (ballot >> tbase) & 0xFu;
 }
 
-// Loads the home groups of the tile's 4 keys; a lane with nothing to probe reports home 0 (a valid
-// group, read and ignored).
+// Transposes the 4 x 4 bytes of the tile's words: byte j of lane q's result is byte q of lane j's word.  Lane q then
+// holds what the four lanes found in the four sectors of its own key's group, in two shuffles for all four keys.
+SG_D uint32_t
+tile_transpose(uint32_t x, const tile_lanes& L)
+{
+    uint32_t y = __shfl_xor_sync(0xffffffffu, x, 1);
+    x = __byte_perm(x, y, (L.q & 1) != 0 ? 0x3715u : 0x6240u);
+    y = __shfl_xor_sync(0xffffffffu, x, 2);
+    return __byte_perm(x, y, (L.q & 2) != 0 ? 0x3276u : 0x5410u);
+}
+
+// For lane q the v[q] of the lane of its tile that has it not zero (the others' v[q] are 0).
+template <typename V>
+SG_D V
+tile_pick(const V (&v)[kTile], const tile_lanes& L)
+{
+    const bool odd = (L.q & 1) != 0, high = (L.q & 2) != 0;
+    V a = odd ? v[1] : v[0];
+    V b = odd ? v[3] : v[2];
+    a |= __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[1], 1);
+    b |= __shfl_xor_sync(0xffffffffu, odd ? v[2] : v[3], 1);
+    return (high ? b : a) | __shfl_xor_sync(0xffffffffu, high ? a : b, 2);
+}
+
+// Loads the home groups of the tile's 4 keys and returns the lane's own home group; a lane with nothing to probe has
+// home 0 (a valid group, read and ignored).
 template <int KIND>
-SG_D void
-load_homes(const dview& t, const tile_lanes& L, uint64_t hash, bool probe, uint32_t (&hr)[kTile],
-           uint32_t (&pre)[kTile][8])
+SG_D uint32_t
+load_homes(const dview& t, const tile_lanes& L, uint64_t hash, bool probe, uint32_t (&pre)[kTile][8])
 {
     const uint32_t home = probe ? home_of<KIND>(t, hash) : 0u;
 #pragma unroll
     for (int r = 0; r < kTile; ++r)
     {
-        hr[r] = __shfl_sync(0xffffffffu, home, L.tbase + r);
-        load_sector(t, hr[r], L.q, pre[r]);
+        load_sector(t, __shfl_sync(0xffffffffu, home, L.tbase + r), L.q, pre[r]);
     }
+    return home;
 }
 
 // Insert step.  Per key, from its home group: present (nothing to do), or a claim of the first erased
@@ -769,39 +817,32 @@ insert_kv_place(const dview& t, const tile_lanes& L, typename kind_consts<KIND>:
         slot = t.num_groups * G + (key == C::empty_key ? 0u : 1u);
     }
     const bool probe = valid && !special;
-    uint32_t hr[kTile];
     uint32_t pre[kTile][8];
     const uint64_t hash = GIVEN ? given_hash
                                 : (hashes != nullptr && probe ? __ldcs(hashes + i) : static_cast<uint64_t>(key));
-    load_homes<KIND>(t, L, hash, probe, hr, pre);
-    int my_state = 0; // 0 present, 1 claim my_target, 2 decided beyond the home group
-    uint32_t my_target = 0;
-    bool my_tomb = false;
-    unsigned my_free = 0u; // never-used slots of the home group as read (bit = slot within the group)
+    const uint32_t home = load_homes<KIND>(t, L, hash, probe, pre);
     const uint32_t my_rot = rot_of(hash);
+    uint32_t match = 0u, never = 0u, erased = 0u; // what the lane's sector of key r's group holds, in byte r
 #pragma unroll
     for (int r = 0; r < kTile; ++r)
     {
         const K kr = __shfl_sync(0xffffffffu, key, L.tbase + r);
-        const uint32_t rot = __shfl_sync(0xffffffffu, my_rot, L.tbase + r);
+        const uint32_t hr = __shfl_sync(0xffffffffu, home, L.tbase + r);
         unsigned mm, me, mt;
-        sector_masks<KIND, true>(pre[r], kr, hr[r] * G + L.q * S, t.total, mm, me, mt);
-        const unsigned tm = tile_nibble(__ballot_sync(0xffffffffu, mm != 0u), L.tbase);
-        // the group's never-used and erased slots, gathered from the tile's 4 sectors
-        const unsigned gfree = group_mask<S>(me, L.q, 0xffffffffu);
-        const unsigned gtomb = group_mask<S>(mt, L.q, 0xffffffffu);
-        const bool tomb = gtomb != 0u;
-        const int s_claim = first_from<G>(tomb ? gtomb : gfree, rot);
-        const uint32_t target = hr[r] * G + static_cast<uint32_t>(s_claim < 0 ? 0 : s_claim);
-        const int state = tm != 0u ? 0 : (gfree != 0u ? 1 : 2);
-        if (L.q == r)
-        {
-            my_state = state;
-            my_target = target;
-            my_tomb = tomb;
-            my_free = gfree;
-        }
+        sector_masks<KIND, true>(pre[r], kr, hr * G + L.q * S, t.total, mm, me, mt);
+        match |= mm << (8 * r);
+        never |= me << (8 * r);
+        erased |= mt << (8 * r);
     }
+    // what the four sectors of the lane's own group hold
+    match = tile_transpose(match, L);
+    never = tile_transpose(never, L);
+    erased = tile_transpose(erased, L);
+    // 0 present, 1 claim my_target, 2 decided beyond the home group
+    const int my_state = match != 0u ? 0 : (never != 0u ? 1 : 2);
+    const bool my_tomb = erased != 0u;
+    const uint32_t my_bit = my_state == 1 ? first_bit_from<S>(my_tomb ? erased : never, my_rot) : 0u;
+    const uint32_t my_target = home * G + bit_slot<S>(my_bit);
     bool again = false;
     if (probe && my_state == 1)
     {
@@ -821,13 +862,12 @@ insert_kv_place(const dview& t, const tile_lanes& L, typename kind_consts<KIND>:
             again = true;
             if (!my_tomb)
             {
-                const uint32_t gbase = my_target - my_target % G;
-                unsigned rest = my_free & ~(1u << (my_target - gbase));
+                uint32_t rest = never & ~(1u << my_bit);
                 while (rest != 0u)
                 {
-                    const uint32_t s = static_cast<uint32_t>(first_from<G>(rest, my_rot));
-                    const uint32_t next = gbase + s;
-                    rest &= ~(1u << s);
+                    const uint32_t b = first_bit_from<S>(rest, my_rot);
+                    const uint32_t next = home * G + bit_slot<S>(b);
+                    rest &= ~(1u << b);
                     if (claim_slot<KIND>(t, next, false, key, val, old))
                     {
                         res = 1;
@@ -856,12 +896,12 @@ insert_kv_place(const dview& t, const tile_lanes& L, typename kind_consts<KIND>:
             {
                 const K kr = __shfl_sync(L.tmask, key, L.tbase + r);
                 const V vr = __shfl_sync(L.tmask, val, L.tbase + r);
+                const uint32_t hr = __shfl_sync(L.tmask, home, L.tbase + r);
                 uint32_t w[8];
-                load_sector(t, hr[r], L.q, w);
+                load_sector(t, hr, L.q, w);
                 const uint32_t rot = __shfl_sync(L.tmask, my_rot, L.tbase + r);
                 uint32_t where = 0;
-                const int x =
-                        tile_insert<KIND, true>(t, kr, vr, hr[r], w, L.tmask, L.tbase, L.q, c.reused, rot, where);
+                const int x = tile_insert<KIND, true>(t, kr, vr, hr, w, L.tmask, L.tbase, L.q, c.reused, rot, where);
                 if (L.q == r)
                 {
                     res = x;
@@ -920,36 +960,33 @@ locate_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K k
     using V = typename C::V;
     constexpr uint32_t G = C::slots_per_group;
     constexpr uint32_t S = sector_consts<KIND>::slots;
-    uint32_t hr[kTile];
     uint32_t pre[kTile][8];
-    load_homes<KIND>(t, L, hash, probe, hr, pre);
-    int32_t my_slot = -1;
-    bool my_more = false;
+    const uint32_t home = load_homes<KIND>(t, L, hash, probe, pre);
+    uint32_t match = 0u, never = 0u; // what the lane's sector of key r's group holds, in byte r
+    V vals[kTile];
 #pragma unroll
     for (int r = 0; r < kTile; ++r)
     {
         const K kr = __shfl_sync(0xffffffffu, key, L.tbase + r);
         unsigned mm, me, mt;
         sector_masks<KIND, false>(pre[r], kr, 0, 0, mm, me, mt);
-        const unsigned tm = tile_nibble(__ballot_sync(0xffffffffu, mm != 0u), L.tbase);
-        const unsigned te = tile_nibble(__ballot_sync(0xffffffffu, me != 0u), L.tbase);
-        const int owner = (__ffs(tm) - 1) & (kTile - 1);
-        const unsigned om = __shfl_sync(0xffffffffu, mm, L.tbase + owner);
-        V vr{};
+        match |= mm << (8 * r);
+        never |= me << (8 * r);
         if constexpr (WANT_VALUE && kind_traits<KIND>::is_map)
         {
-            vr = __shfl_sync(0xffffffffu, select_sector_value<KIND>(pre[r], mm), L.tbase + owner);
-        }
-        const int32_t slot = tm != 0u ? static_cast<int32_t>(hr[r] * G + static_cast<uint32_t>(owner) * S +
-                                                             static_cast<uint32_t>(__ffs(om) - 1))
-                                      : -1;
-        if (L.q == r)
-        {
-            my_slot = slot;
-            my_more = tm == 0u && te == 0u;
-            val = vr;
+            vals[r] = select_sector_value<KIND>(pre[r], mm);
         }
     }
+    // what the four sectors of the lane's own group hold
+    match = tile_transpose(match, L);
+    never = tile_transpose(never, L);
+    if constexpr (WANT_VALUE && kind_traits<KIND>::is_map)
+    {
+        val = tile_pick<V>(vals, L);
+    }
+    int32_t my_slot = match != 0u ? static_cast<int32_t>(home * G + bit_slot<S>(static_cast<uint32_t>(__ffs(match) - 1)))
+                                  : -1;
+    const bool my_more = match == 0u && never == 0u;
     const unsigned mball = __ballot_sync(0xffffffffu, probe && my_more);
     if (mball != 0u)
     {
@@ -960,7 +997,7 @@ locate_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K k
             if (mmask & (1u << r))
             {
                 const K kr = __shfl_sync(L.tmask, key, L.tbase + r);
-                const uint32_t g = next_group32(hr[r], t.num_groups);
+                const uint32_t g = next_group32(__shfl_sync(L.tmask, home, L.tbase + r), t.num_groups);
                 uint32_t w[8];
                 load_sector(t, g, L.q, w);
                 V vr{};
