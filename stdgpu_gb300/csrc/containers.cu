@@ -437,15 +437,16 @@ k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters
     {
         return;
     }
-    // exclusive scan of the counts, 4 consecutive ones per thread at a time
+    // exclusive scan of the counts, kScan consecutive ones per thread at a time
+    constexpr int kScan = 4;
     unsigned carry = 0;
-    for (int64_t base = 0; base < tiles; base += 4 * kCThreads)
+    for (int64_t base = 0; base < tiles; base += kScan * kCThreads)
     {
-        const int64_t k = base + 4 * static_cast<int64_t>(threadIdx.x);
-        unsigned v[4];
+        const int64_t k = base + kScan * static_cast<int64_t>(threadIdx.x);
+        unsigned v[kScan];
         unsigned sum = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < kScan; ++j)
         {
             v[j] = k + j < tiles ? __ldcg(counts + k + j) : 0u;
             sum += v[j];
@@ -473,7 +474,7 @@ k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters
             carry += x;
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < kScan; ++j)
         {
             if (k + j < tiles)
             {
@@ -544,7 +545,7 @@ k_deque_rebuild_turns(unsigned* seq, const deque_counters* c, const sg_deque_syn
 // kMoveFirst: pops of elements stored before the call, every outcome, and the pushes too when they meet no pop
 // at a slot (the other two launches then return at once); else kMovePush and kMoveLate follow, pushes
 // and then the pops of elements that the call pushed.
-// 2^24 mixed operations on 8-byte elements in steady state: 153 us in all, 303 us when every slot's turn word
+// 2^24 mixed operations on 8-byte elements in steady state: 124 us in all, 303 us when every slot's turn word
 // was read, waited on and written (and the outputs filled before); from an empty deque, where each pop depends on a
 // push of the call, 375 us against 779 us.
 enum move_phase : int
@@ -554,10 +555,12 @@ enum move_phase : int
     kMoveLate = 2
 };
 
-// Compiled for 6 resident blocks per SM: 153 us, with 5 of them 155 us, with the 4 that 64 registers allow 163 us.
+// Compiled for 8 resident blocks per SM, two rows in flight at a time: 124 us; 7 blocks and 4 rows 126, 7 and 8 rows
+// 139, 6 and 8 rows 144 us (ranks in 64 bits 153), the 4 blocks that 64 registers allow 162 us: the loads wait for the
+// flags and the counts, and other warps fill that wait better than more loads per warp.
 template <typename T, int PHASE>
-__global__ void __launch_bounds__(kCThreads, 6)
-k_deque_move(T* data, const unsigned* before, int64_t cap, const uint8_t* is_push, const T* values, int64_t n,
+__global__ void __launch_bounds__(kCThreads, 8)
+k_deque_move(T* data, const unsigned* before, unsigned ucap, const uint8_t* is_push, const T* values, unsigned n,
              T* out_popped, uint8_t* out_ok, bool zero_rest, const deque_control* ctl)
 {
     const bool apart = ctl->apart != 0u;
@@ -568,22 +571,21 @@ k_deque_move(T* data, const unsigned* before, int64_t cap, const uint8_t* is_pus
     __shared__ unsigned s_warp[2][kWarps];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const unsigned ucap = static_cast<unsigned>(cap);
-    const unsigned push_pos = static_cast<unsigned>(ctl->push_t0 % static_cast<unsigned long long>(cap));
-    const unsigned pop_pos = static_cast<unsigned>(ctl->pop_t0 % static_cast<unsigned long long>(cap));
-    const long long push_ok = ctl->push_ok;
-    const long long pop_ok = ctl->pop_ok;
-    const long long held = ctl->held;
+    const unsigned push_pos = static_cast<unsigned>(ctl->push_t0 % ucap);
+    const unsigned pop_pos = static_cast<unsigned>(ctl->pop_t0 % ucap);
+    const unsigned push_ok = static_cast<unsigned>(ctl->push_ok);
+    const unsigned pop_ok = static_cast<unsigned>(ctl->pop_ok);
+    const unsigned held = static_cast<unsigned>(ctl->held);
     int buf = 0;
-    for (int64_t tile = blockIdx.x; tile * kPlanTile < n; tile += gridDim.x, buf ^= 1)
+    for (unsigned tile = blockIdx.x; tile * kPlanTile < n; tile += gridDim.x, buf ^= 1)
     {
-        const int64_t first = tile * kPlanTile + warp * (kItems * 32) + lane;
+        const unsigned first = tile * kPlanTile + warp * (kItems * 32) + lane;
         unsigned masks[kItems]; // pushes of row j
         unsigned total = 0;
 #pragma unroll
         for (int j = 0; j < kItems; ++j)
         {
-            const int64_t i = first + j * 32;
+            const unsigned i = first + j * 32;
             masks[j] = __ballot_sync(0xffffffffu, i < n && is_push[i] != 0);
             total += __popc(masks[j]);
         }
@@ -592,55 +594,62 @@ k_deque_move(T* data, const unsigned* before, int64_t cap, const uint8_t* is_pus
             s_warp[buf][warp] = total;
         }
         __syncthreads();
-        long long rank = __ldg(before + tile); // pushes before the tile, then before the row
+        unsigned rank = __ldg(before + tile); // pushes before the tile, then before the row
         for (int w = 0; w < warp; ++w)
         {
             rank += s_warp[buf][w];
         }
-        T v[kItems];
-        unsigned pos[kItems];
-        unsigned done = 0u; // bit j: item j succeeds
-        unsigned move = 0u; // bit j: and moves its element in this launch
+        // rows in flight together; more of them cost the registers that a second resident warp would use
+        constexpr int kRows = 2;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j0 = 0; j0 < kItems; j0 += kRows)
         {
-            const int64_t i = first + j * 32;
-            const bool push = (masks[j] >> lane) & 1u;
-            const long long pushes = rank + __popc(masks[j] & lanemask_lt()); // before element i
-            const long long r = push ? pushes : i - pushes;
-            const bool ok = i < n && r < (push ? push_ok : pop_ok);
-            const bool now = PHASE == kMoveFirst ? (push ? apart : r < held)
-                                                 : (PHASE == kMovePush ? push : !push && r >= held);
-            const unsigned p = (push ? push_pos : pop_pos) + static_cast<unsigned>(r);
-            pos[j] = p >= ucap ? p - ucap : p;
-            v[j] = T{};
-            done |= static_cast<unsigned>(ok) << j;
-            if (ok && now)
-            {
-                move |= 1u << j;
-                v[j] = push ? ld_stream(values + i) : __ldcg(data + pos[j]);
-            }
-            rank += __popc(masks[j]);
-        }
+            T v[kRows];
+            unsigned pos[kRows];
+            unsigned done = 0u; // bit j: row j0 + j's item succeeds
+            unsigned move = 0u; // bit j: and moves its element in this launch
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
-        {
-            const int64_t i = first + j * 32;
-            const bool push = (masks[j] >> lane) & 1u;
-            const bool moves = (move >> j) & 1u;
-            if (push && moves)
+            for (int j = 0; j < kRows; ++j)
             {
-                data[pos[j]] = v[j];
+                const unsigned i = first + (j0 + j) * 32;
+                const unsigned mask = masks[j0 + j];
+                const bool push = (mask >> lane) & 1u;
+                const unsigned pushes = rank + __popc(mask & lanemask_lt()); // before element i
+                const unsigned r = push ? pushes : i - pushes;
+                const bool ok = i < n && r < (push ? push_ok : pop_ok);
+                const bool now = PHASE == kMoveFirst ? (push ? apart : r < held)
+                                                     : (PHASE == kMovePush ? push : !push && r >= held);
+                const unsigned p = (push ? push_pos : pop_pos) + r;
+                pos[j] = p >= ucap ? p - ucap : p;
+                v[j] = T{};
+                done |= static_cast<unsigned>(ok) << j;
+                if (ok && now)
+                {
+                    move |= 1u << j;
+                    v[j] = push ? ld_stream(values + i) : __ldcg(data + pos[j]);
+                }
+                rank += __popc(mask);
             }
-            // a pop of an element that the call pushed is written by the last launch
-            if (out_popped != nullptr && i < n &&
-                (PHASE == kMoveFirst ? zero_rest || (!push && moves) : !push && moves))
+#pragma unroll
+            for (int j = 0; j < kRows; ++j)
             {
-                out_popped[i] = push ? T{} : v[j];
-            }
-            if (PHASE == kMoveFirst && out_ok != nullptr && i < n)
-            {
-                out_ok[i] = static_cast<uint8_t>((done >> j) & 1u);
+                const unsigned i = first + (j0 + j) * 32;
+                const bool push = (masks[j0 + j] >> lane) & 1u;
+                const bool moves = (move >> j) & 1u;
+                if (push && moves)
+                {
+                    data[pos[j]] = v[j];
+                }
+                // a pop of an element that the call pushed is written by the last launch
+                if (out_popped != nullptr && i < n &&
+                    (PHASE == kMoveFirst ? zero_rest || (!push && moves) : !push && moves))
+                {
+                    out_popped[i] = push ? T{} : v[j];
+                }
+                if (PHASE == kMoveFirst && out_ok != nullptr && i < n)
+                {
+                    out_ok[i] = static_cast<uint8_t>((done >> j) & 1u);
+                }
             }
         }
         // no barrier: the next tile fills the other count buffer
@@ -1424,16 +1433,19 @@ deque_mixed(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, 
     k_deque_plan<<<grid_for(tiles, kWarps, mp), kCThreads, 0, s>>>(is_push, n, d->seq, d->counters, d->capacity,
                                                                    d->sync, d->epoch, control_of(d));
     SG_LAUNCH_CHECK();
+    // at most `capacity` elements, below 2^31: 32-bit ranks
+    const unsigned ucap = static_cast<unsigned>(d->capacity);
+    const unsigned un = static_cast<unsigned>(n);
     static const int m0 = persistent_grid(k_deque_move<T, kMoveFirst>, kCThreads);
     static const int m1 = persistent_grid(k_deque_move<T, kMovePush>, kCThreads);
     static const int m2 = persistent_grid(k_deque_move<T, kMoveLate>, kCThreads);
-    k_deque_move<T, kMoveFirst><<<grid_for(tiles, 1, m0), kCThreads, 0, s>>>(data, d->seq, d->capacity, is_push, in, n,
+    k_deque_move<T, kMoveFirst><<<grid_for(tiles, 1, m0), kCThreads, 0, s>>>(data, d->seq, ucap, is_push, in, un,
                                                                             out, out_ok, zero_rest, control_of(d));
     SG_LAUNCH_CHECK();
-    k_deque_move<T, kMovePush><<<grid_for(tiles, 1, m1), kCThreads, 0, s>>>(data, d->seq, d->capacity, is_push, in, n,
+    k_deque_move<T, kMovePush><<<grid_for(tiles, 1, m1), kCThreads, 0, s>>>(data, d->seq, ucap, is_push, in, un,
                                                                            out, out_ok, zero_rest, control_of(d));
     SG_LAUNCH_CHECK();
-    k_deque_move<T, kMoveLate><<<grid_for(tiles, 1, m2), kCThreads, 0, s>>>(data, d->seq, d->capacity, is_push, in, n,
+    k_deque_move<T, kMoveLate><<<grid_for(tiles, 1, m2), kCThreads, 0, s>>>(data, d->seq, ucap, is_push, in, un,
                                                                            out, out_ok, zero_rest, control_of(d));
     SG_LAUNCH_CHECK();
     return SG_OK;
