@@ -73,6 +73,7 @@ static_assert(sizeof(table_header) <= kCountedControlOffset &&
 __global__ void
 k_read_header(const table_header* hdr, unsigned long long* host)
 {
+    wait_for_stream();
     if (threadIdx.x < sizeof(table_header) / 8)
     {
         host[threadIdx.x] = __ldcg(reinterpret_cast<const unsigned long long*>(hdr) + threadIdx.x);
@@ -87,6 +88,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kThreads)
 k_init(dview t, accounting_init acc)
 {
+    wait_for_stream();
     using C = kind_consts<KIND>;
     using K = typename C::K;
     constexpr int G = C::slots_per_group;
@@ -149,6 +151,7 @@ __global__ void __launch_bounds__(kThreads, SG_BULK_MIN_BLOCKS)
 k_insert(dview t, const void* in0, const void* in1, int64_t n, uint8_t* out_flags, const uint64_t* hashes,
          const unsigned int* gate)
 {
+    wait_for_stream();
     // a gated launch (the fallback of a partitioned insert) runs only when its gate word is set
     if (gate != nullptr && *gate == 0u)
     {
@@ -788,6 +791,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kThreads, SG_BULK_MIN_BLOCKS)
 k_erase(dview t, const void* keys, int64_t n, uint8_t* out_flags, const uint64_t* hashes, const unsigned int* gate)
 {
+    wait_for_stream();
     if (gate != nullptr && *gate == 0u)
     {
         return;
@@ -1056,6 +1060,7 @@ __global__ void __launch_bounds__(kThreads, SG_BULK_MIN_BLOCKS)
 k_counted_candidates(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n, const uint64_t* hashes,
                      uint32_t* cand)
 {
+    wait_for_stream();
     counted_candidates<KIND, AOS>(t, v, in0, in1, n, hashes, cand);
     // block_add's additions come from threads 0 and 1; the block that is last to add decides for the call
     __syncthreads();
@@ -1076,6 +1081,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 k_insert_counted(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n, uint8_t* out_flags,
                  const uint64_t* hashes, const uint32_t* cand)
 {
+    wait_for_stream();
     const unsigned int mode = __ldcg(&counted_words(t.hdr)->mode);
     const counted_changes ch = counted_insert<KIND, AOS>(t, v, in0, in1, n, out_flags, hashes, cand, mode);
     if (mode == kCountedQuiet)
@@ -1089,6 +1095,7 @@ __global__ void __launch_bounds__(kThreads)
 k_counted_reset(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n, const uint64_t* hashes,
                 uint32_t* cand)
 {
+    wait_for_stream();
     counted_reset<KIND, AOS>(v, t.hdr, in0, in1, n, hashes, cand);
 }
 
@@ -1098,6 +1105,7 @@ __global__ void __launch_bounds__(kThreads)
 k_insert_counted_cluster(dview t, sg_unordered_view v, const void* in0, const void* in1, int64_t n,
                          uint8_t* out_flags, const uint64_t* hashes, uint32_t* cand)
 {
+    wait_for_stream();
     __shared__ unsigned int s_mode;
     counted_candidates<KIND, AOS>(t, v, in0, in1, n, hashes, cand);
     __syncthreads();
@@ -1126,6 +1134,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kThreads, SG_BULK_MIN_BLOCKS)
 k_erase_counted(dview t, sg_unordered_view v, const void* keys, int64_t n, uint8_t* out_flags, const uint64_t* hashes)
 {
+    wait_for_stream();
     using C = kind_consts<KIND>;
     using K = typename C::K;
     const tile_lanes L;
@@ -1193,6 +1202,7 @@ __global__ void __launch_bounds__(kThreads, SG_FIND_MIN_BLOCKS)
 k_find(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found, const uint64_t* hashes,
        bool zero_absent)
 {
+    wait_for_stream();
     const tile_lanes L;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
@@ -1832,7 +1842,7 @@ struct do_init
             acc.ones = reinterpret_cast<uint4*>(t->bucket_cand);
             acc.one_units = static_cast<int64_t>(bucket_cand_bytes(t->bucket_count)) / 16;
         }
-        k_init<KIND><<<grid_for(units, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), acc);
+        SG_CUDA_TRY(launch_early(k_init<KIND>, grid_for(units, kThreads, max_grid), kThreads, s, view_of(t), acc));
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -1979,17 +1989,19 @@ insert_counted(sg_unordered* t, const void* in0, const void* in1, int64_t n, uin
         {
             blocks <<= 1;
         }
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = static_cast<unsigned>(blocks);
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
+        cudaLaunchAttribute attr[2] = {};
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(blocks);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; // launch_early
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(static_cast<unsigned>(blocks));
         cfg.blockDim = dim3(kThreads);
         cfg.stream = s;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
         SG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_insert_counted_cluster<KIND, AOS>, d, v, in0, in1, n, flags, hashes,
                                        t->bucket_cand));
         SG_LAUNCH_CHECK();
@@ -1998,14 +2010,14 @@ insert_counted(sg_unordered* t, const void* in0, const void* in1, int64_t n, uin
     static const int g_cand = persistent_grid(k_counted_candidates<KIND, AOS>, kThreads);
     static const int g_ins = persistent_grid(k_insert_counted<KIND, AOS>, kThreads);
     static const int g_reset = persistent_grid(k_counted_reset<KIND, AOS>, kThreads);
-    k_counted_candidates<KIND, AOS><<<grid_for(n, kThreads, g_cand), kThreads, 0, s>>>(d, v, in0, in1, n, hashes,
-                                                                                      t->bucket_cand);
+    SG_CUDA_TRY(launch_early(k_counted_candidates<KIND, AOS>, grid_for(n, kThreads, g_cand), kThreads, s, d, v, in0,
+                             in1, n, hashes, t->bucket_cand));
     SG_LAUNCH_CHECK();
-    k_insert_counted<KIND, AOS><<<grid_for(n, kThreads, g_ins), kThreads, 0, s>>>(d, v, in0, in1, n, flags, hashes,
-                                                                                 t->bucket_cand);
+    SG_CUDA_TRY(launch_early(k_insert_counted<KIND, AOS>, grid_for(n, kThreads, g_ins), kThreads, s, d, v, in0, in1, n,
+                             flags, hashes, t->bucket_cand));
     SG_LAUNCH_CHECK();
-    k_counted_reset<KIND, AOS><<<grid_for(n, kThreads, g_reset), kThreads, 0, s>>>(d, v, in0, in1, n, hashes,
-                                                                                  t->bucket_cand);
+    SG_CUDA_TRY(launch_early(k_counted_reset<KIND, AOS>, grid_for(n, kThreads, g_reset), kThreads, s, d, v, in0, in1, n,
+                             hashes, t->bucket_cand));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -2080,14 +2092,14 @@ struct do_insert
         if (aos)
         {
             static const int max_grid = persistent_grid(k_insert<KIND, true>, kThreads);
-            k_insert<KIND, true><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), in0, in1, n, flags,
-                                                                                     hashes, gate);
+            SG_CUDA_TRY(launch_early(k_insert<KIND, true>, grid_for(n, kThreads, max_grid), kThreads, s, view_of(t),
+                                     in0, in1, n, flags, hashes, gate));
         }
         else
         {
             static const int max_grid = persistent_grid(k_insert<KIND, false>, kThreads);
-            k_insert<KIND, false><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), in0, in1, n,
-                                                                                      flags, hashes, gate);
+            SG_CUDA_TRY(launch_early(k_insert<KIND, false>, grid_for(n, kThreads, max_grid), kThreads, s, view_of(t),
+                                     in0, in1, n, flags, hashes, gate));
         }
         SG_LAUNCH_CHECK();
         return SG_OK;
@@ -2103,8 +2115,8 @@ struct do_erase
         if (t->bucket_heads != nullptr)
         {
             static const int max_grid = persistent_grid(k_erase_counted<KIND>, kThreads);
-            k_erase_counted<KIND><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), public_view(t), keys,
-                                                                                      n, flags, hashes);
+            SG_CUDA_TRY(launch_early(k_erase_counted<KIND>, grid_for(n, kThreads, max_grid), kThreads, s, view_of(t),
+                                     public_view(t), keys, n, flags, hashes));
             SG_LAUNCH_CHECK();
             return SG_OK;
         }
@@ -2153,7 +2165,8 @@ struct do_erase
             gate = pl.lost;
         }
         static const int max_grid = persistent_grid(k_erase<KIND>, kThreads);
-        k_erase<KIND><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), keys, n, flags, hashes, gate);
+        SG_CUDA_TRY(launch_early(k_erase<KIND>, grid_for(n, kThreads, max_grid), kThreads, s, view_of(t), keys, n,
+                                 flags, hashes, gate));
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -2186,14 +2199,14 @@ struct do_find
         if (vals != nullptr)
         {
             static const int max_grid = persistent_grid(k_find<KIND, true>, kThreads);
-            k_find<KIND, true><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), keys, n, vals, found,
-                                                                                   hashes, zero_absent);
+            SG_CUDA_TRY(launch_early(k_find<KIND, true>, grid_for(n, kThreads, max_grid), kThreads, s, view_of(t), keys,
+                                     n, vals, found, hashes, zero_absent));
         }
         else
         {
             static const int max_grid = persistent_grid(k_find<KIND, false>, kThreads);
-            k_find<KIND, false><<<grid_for(n, kThreads, max_grid), kThreads, 0, s>>>(view_of(t), keys, n, vals,
-                                                                                    found, hashes, false);
+            SG_CUDA_TRY(launch_early(k_find<KIND, false>, grid_for(n, kThreads, max_grid), kThreads, s, view_of(t),
+                                     keys, n, vals, found, hashes, false));
         }
         SG_LAUNCH_CHECK();
         return SG_OK;
@@ -2269,7 +2282,7 @@ sg_status
 read_header(sg_unordered* t, cudaStream_t s)
 {
     static_assert(sizeof(table_header) % 8 == 0 && sizeof(table_header) <= 32 * 8, "one warp copies the header");
-    k_read_header<<<1, 32, 0, s>>>(t->hdr, t->host_hdr);
+    SG_CUDA_TRY(launch_early(k_read_header, 1, 32, s, t->hdr, t->host_hdr));
     SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     return SG_OK;
