@@ -85,6 +85,7 @@ tiles_of(const int64_t* offsets, int64_t t, int tile)
 __global__ void __launch_bounds__(1024)
 k_batch_tiles(const int64_t* offsets, int32_t n, int64_t* prefix, bool has_keys, const uint8_t* todo)
 {
+    wait_for_stream();
     scan_tables(n, prefix, [&](int64_t t) -> long long {
         return has_keys && (todo == nullptr || todo[t] != 0) ? tiles_of(offsets, t, 32) : 0;
     });
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(1024)
 k_batch_choose(const dview* views, const int64_t* offsets, int32_t n, const int32_t* first_item, bool flags, int tile,
                uint8_t* build, uint8_t* todo, int64_t* prefix)
 {
+    wait_for_stream();
     for (int32_t t = threadIdx.x; t < n; t += blockDim.x)
     {
         const dview v = views[t];
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(kListThreads, 3)
 k_batch_lists(const dview* views, const int64_t* offsets, const int64_t* prefix, int32_t n, const int32_t* first_item,
               unsigned int* fill, uint8_t* todo, const void* in0, const void* in1)
 {
+    wait_for_stream();
     using C = kind_consts<KIND>;
     using E = typename slot_image<KIND>::type;
     constexpr int PER = kListPer;
@@ -262,6 +265,7 @@ k_batch_build(const dview* views, const int64_t* offsets, const build_item* item
               const unsigned int* fill, uint8_t* todo, const void* in0, const void* in1, uint8_t* out_flags,
               spill_list spills)
 {
+    wait_for_stream();
     using C = kind_consts<KIND>;
     using K = typename C::K;
     using V = typename C::V;
@@ -364,6 +368,7 @@ k_batch(const dview* views, const int64_t* offsets, const int64_t* prefix, int32
         const void* in0, const void* in1, void* out_vals, uint8_t* out_flags, const uint8_t* built,
         spill_list spills)
 {
+    wait_for_stream();
     const tile_lanes L;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
@@ -566,9 +571,8 @@ struct batch_launch
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<KIND, OP, THREADS>, THREADS, 0);
         per_sm = per_sm < 1 ? 1 : per_sm;
         const int want = b->blocks_per_sm > 0 ? (b->blocks_per_sm < per_sm ? b->blocks_per_sm : per_sm) : per_sm;
-        k_batch<KIND, OP, THREADS><<<b->sms * want, THREADS, 0, s>>>(b->views, offsets, b->prefix, b->n,
-                                                                      b->tiles_per_step, in0, in1, out_vals,
-                                                                      out_flags, built, b->spills);
+        SG_CUDA_TRY(launch_early(k_batch<KIND, OP, THREADS>, b->sms * want, THREADS, s, b->views, offsets, b->prefix,
+                                 b->n, b->tiles_per_step, in0, in1, out_vals, out_flags, built, b->spills));
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -618,19 +622,20 @@ struct batch_launch
         uint8_t* const todo = b->marks + b->n;
         // the lists' lengths, and the spill count behind them
         SG_CUDA_TRY(cudaMemsetAsync(b->fill, 0, sizeof(unsigned int) * static_cast<size_t>(b->n_items + 1), s));
-        k_batch_choose<<<1, 1024, 0, s>>>(b->views, offsets, b->n, b->first_item, out_flags != nullptr,
-                                          kListPer * kListThreads, b->marks, todo, b->list_prefix);
+        SG_CUDA_TRY(launch_early(k_batch_choose, 1, 1024, s, b->views, offsets, b->n, b->first_item,
+                                 out_flags != nullptr, kListPer * kListThreads, b->marks, todo, b->list_prefix));
         SG_LAUNCH_CHECK();
         SG_CUDA_TRY(cudaFuncSetAttribute(k_batch_lists<KIND, AOS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(sizeof(Lists))));
         static const int lists_grid = persistent_grid(k_batch_lists<KIND, AOS>, kListThreads, sizeof(Lists));
-        k_batch_lists<KIND, AOS><<<lists_grid, kListThreads, sizeof(Lists), s>>>(
-                b->views, offsets, b->list_prefix, b->n, b->first_item, b->fill, todo, in0, in1);
+        SG_CUDA_TRY(launch_early_shared(k_batch_lists<KIND, AOS>, lists_grid, kListThreads, sizeof(Lists), s, b->views,
+                                        offsets, b->list_prefix, b->n, b->first_item, b->fill, todo, in0, in1));
         SG_LAUNCH_CHECK();
         SG_CUDA_TRY(cudaFuncSetAttribute(k_batch_build<KIND, AOS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kRegionBytes)));
-        k_batch_build<KIND, AOS><<<static_cast<unsigned>(b->n_items), kRegionThreads, kRegionBytes, s>>>(
-                b->views, offsets, b->items, b->marks, b->fill, todo, in0, in1, out_flags, b->spills);
+        SG_CUDA_TRY(launch_early_shared(k_batch_build<KIND, AOS>, static_cast<unsigned>(b->n_items), kRegionThreads,
+                                        kRegionBytes, s, b->views, offsets, b->items, b->marks, b->fill, todo, in0, in1,
+                                        out_flags, b->spills));
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -697,7 +702,8 @@ dispatch_op(sg_table_batch* b, int op, const int64_t* offsets, const void* in0, 
     }
     const uint8_t* built = build ? b->marks : nullptr;
     // a NULL key array (all ranges empty, as an empty tensor gives) walks no tile
-    k_batch_tiles<<<1, 1024, 0, s>>>(offsets, b->n, b->prefix, in0 != nullptr, build ? b->marks + b->n : nullptr);
+    SG_CUDA_TRY(launch_early(k_batch_tiles, 1, 1024, s, offsets, b->n, b->prefix, in0 != nullptr,
+                             build ? b->marks + b->n : nullptr));
     SG_LAUNCH_CHECK();
     switch (b->kind)
     {

@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(kCThreads)
 k_vector_push_back(T* data, long long* size, int64_t cap, const T* values, const uint8_t* pred, int64_t n,
                    uint8_t* out_pushed, sg_vector_sync* sync, uint32_t epoch, vector_control* ctl)
 {
+    wait_for_stream();
     static_assert(ROWS == 4 || ROWS == 32, "a lane reads 4 or 32 predicate bytes");
     constexpr int64_t kWarpElems = ROWS * 32;
     constexpr int64_t kTile = kWarpElems * kWarps;
@@ -382,6 +383,7 @@ __global__ void __launch_bounds__(kCThreads)
 k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters* c, int64_t cap, sg_deque_sync* sync,
              uint32_t epoch, deque_control* ctl)
 {
+    wait_for_stream();
     __shared__ unsigned long long s_block;
     __shared__ unsigned s_warp[kWarps];
     const int lane = threadIdx.x & 31;
@@ -514,6 +516,7 @@ k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters
 __global__ void
 k_deque_rebuild_turns(unsigned* seq, const deque_counters* c, const sg_deque_sync* sync, int64_t cap)
 {
+    wait_for_stream();
     if (*reinterpret_cast<const volatile uint32_t*>(&sync->dirty) == 0u)
     {
         return;
@@ -563,6 +566,7 @@ __global__ void __launch_bounds__(kCThreads, 8)
 k_deque_move(T* data, const unsigned* before, unsigned ucap, const uint8_t* is_push, const T* values, unsigned n,
              T* out_popped, uint8_t* out_ok, bool zero_rest, const deque_control* ctl)
 {
+    wait_for_stream();
     const bool apart = ctl->apart != 0u;
     if (PHASE != kMoveFirst && apart)
     {
@@ -662,6 +666,7 @@ k_deque_ops(T* data, unsigned* seq, deque_counters* c, int64_t cap, const uint8_
             int64_t n, T* out_popped, uint8_t* out_ok, bool zero_rest, deque_control* ctl, sg_deque_sync* sync,
             uint32_t epoch)
 {
+    wait_for_stream();
     __shared__ unsigned cpush[kCounts];
     __shared__ unsigned cpop[kCounts];
     __shared__ unsigned mpush[kCounts]; // the ballots, so the wait loop below indexes no local array
@@ -918,6 +923,7 @@ __global__ void __launch_bounds__(kCThreads)
 k_deque_end_ops(T* data, deque_counters* c, int64_t cap, const T* values, int64_t n, T* out_popped, uint8_t* out_ok,
                 bool zero_rest, unsigned* seq, bool keep, sg_deque_sync* sync, uint32_t epoch, deque_control* ctl)
 {
+    wait_for_stream();
     constexpr bool push = OP == kPushFront || OP == kPushBack;
     constexpr bool up = OP == kPushBack || OP == kPopFront; // tickets go up from t0, else down from t0 - 1
     const unsigned long long ucap = static_cast<unsigned long long>(cap);
@@ -1028,6 +1034,7 @@ __global__ void __launch_bounds__(kCThreads)
 k_vector_pop_back(const T* data, long long* size, int64_t cap, int64_t n, T* out_values, uint8_t* out_ok,
                   sg_vector_sync* sync, uint32_t epoch, vector_control* ctl)
 {
+    wait_for_stream();
     long long sz = __ldcg(size);
     sz = sz < 0 ? 0 : (sz > cap ? cap : sz);
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -1054,6 +1061,7 @@ k_vector_pop_back(const T* data, long long* size, int64_t cap, int64_t n, T* out
 __global__ void
 k_vector_call_ends(long long* size, int64_t cap, bool clear, sg_vector_sync* sync, uint32_t epoch)
 {
+    wait_for_stream();
     if (clear)
     {
         *size = 0;
@@ -1065,6 +1073,7 @@ k_vector_call_ends(long long* size, int64_t cap, bool clear, sg_vector_sync* syn
 __global__ void
 k_deque_reset(unsigned* seq, deque_counters* c, int64_t cap, bool keep, sg_deque_sync* sync, uint32_t epoch)
 {
+    wait_for_stream();
     if (keep)
     {
         for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < cap;
@@ -1106,6 +1115,7 @@ k_deque_copy_out(const T* data, const deque_counters* c, int64_t cap, T* out)
 __global__ void
 k_read_words(const unsigned long long* src, unsigned long long* host, int words)
 {
+    wait_for_stream();
     if (static_cast<int>(threadIdx.x) < words)
     {
         host[threadIdx.x] = __ldcg(src + threadIdx.x);
@@ -1119,6 +1129,7 @@ constexpr int kCountThreads = 512;
 __global__ void __launch_bounds__(kCountThreads)
 k_bitset_count(const uint32_t* blocks, int64_t nbits, unsigned long long* partials)
 {
+    wait_for_stream();
     const int64_t nwords = (nbits + 31) / 32;
     const int64_t full_words = nbits / 32; // words with all 32 bits counted
     const bool aligned = (reinterpret_cast<uintptr_t>(blocks) & 15u) == 0;
@@ -1181,6 +1192,7 @@ k_bitset_count(const uint32_t* blocks, int64_t nbits, unsigned long long* partia
 __global__ void __launch_bounds__(1024)
 k_sum_partials(const unsigned long long* partials, int n, unsigned long long* out)
 {
+    wait_for_stream();
     unsigned long long s = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
     {
@@ -1373,10 +1385,10 @@ deque_end_launch(sg_deque* d, const void* values, int64_t n, void* out_popped, u
                  cudaStream_t s)
 {
     static const int mg = persistent_grid(k_deque_end_ops<T, OP>, kCThreads);
-    k_deque_end_ops<T, OP><<<grid_for(n, kCThreads, mg), kCThreads, 0, s>>>(
-            static_cast<T*>(d->data), d->counters, d->capacity, static_cast<const T*>(values), n,
-            static_cast<T*>(out_popped), out_ok, zero_rest, d->seq, d->capacity <= kTurnsKeptMax, d->sync, d->epoch,
-            control_of(d));
+    SG_CUDA_TRY(launch_early(k_deque_end_ops<T, OP>, grid_for(n, kCThreads, mg), kCThreads, s, static_cast<T*>(d->data),
+                             d->counters, d->capacity, static_cast<const T*>(values), n, static_cast<T*>(out_popped),
+                             out_ok, zero_rest, d->seq, d->capacity <= kTurnsKeptMax, d->sync, d->epoch,
+                             control_of(d)));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -1418,20 +1430,20 @@ deque_mixed(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, 
     if (d->capacity <= kTurnsKeptMax || n > d->capacity)
     {
         static const int mr = persistent_grid(k_deque_rebuild_turns, kCThreads);
-        k_deque_rebuild_turns<<<grid_for(d->capacity, kCThreads, mr), kCThreads, 0, s>>>(d->seq, d->counters, d->sync,
-                                                                                         d->capacity);
+        SG_CUDA_TRY(launch_early(k_deque_rebuild_turns, grid_for(d->capacity, kCThreads, mr), kCThreads, s, d->seq,
+                                 d->counters, d->sync, d->capacity));
         SG_LAUNCH_CHECK();
         static const int mo = persistent_grid(k_deque_ops<T>, kCThreads);
-        k_deque_ops<T><<<grid_for(n, static_cast<int>(kTileElems), mo), kCThreads, 0, s>>>(
-                data, d->seq, d->counters, d->capacity, is_push, in, n, out, out_ok, zero_rest, control_of(d), d->sync,
-                d->epoch);
+        SG_CUDA_TRY(launch_early(k_deque_ops<T>, grid_for(n, static_cast<int>(kTileElems), mo), kCThreads, s, data,
+                                 d->seq, d->counters, d->capacity, is_push, in, n, out, out_ok, zero_rest,
+                                 control_of(d), d->sync, d->epoch));
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
     const int64_t tiles = (n + kPlanTile - 1) / kPlanTile;
     static const int mp = persistent_grid(k_deque_plan, kCThreads);
-    k_deque_plan<<<grid_for(tiles, kWarps, mp), kCThreads, 0, s>>>(is_push, n, d->seq, d->counters, d->capacity,
-                                                                   d->sync, d->epoch, control_of(d));
+    SG_CUDA_TRY(launch_early(k_deque_plan, grid_for(tiles, kWarps, mp), kCThreads, s, is_push, n, d->seq, d->counters,
+                             d->capacity, d->sync, d->epoch, control_of(d)));
     SG_LAUNCH_CHECK();
     // at most `capacity` elements, below 2^31: 32-bit ranks
     const unsigned ucap = static_cast<unsigned>(d->capacity);
@@ -1439,14 +1451,14 @@ deque_mixed(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, 
     static const int m0 = persistent_grid(k_deque_move<T, kMoveFirst>, kCThreads);
     static const int m1 = persistent_grid(k_deque_move<T, kMovePush>, kCThreads);
     static const int m2 = persistent_grid(k_deque_move<T, kMoveLate>, kCThreads);
-    k_deque_move<T, kMoveFirst><<<grid_for(tiles, 1, m0), kCThreads, 0, s>>>(data, d->seq, ucap, is_push, in, un,
-                                                                            out, out_ok, zero_rest, control_of(d));
+    SG_CUDA_TRY(launch_early(k_deque_move<T, kMoveFirst>, grid_for(tiles, 1, m0), kCThreads, s, data, d->seq, ucap,
+                             is_push, in, un, out, out_ok, zero_rest, control_of(d)));
     SG_LAUNCH_CHECK();
-    k_deque_move<T, kMovePush><<<grid_for(tiles, 1, m1), kCThreads, 0, s>>>(data, d->seq, ucap, is_push, in, un,
-                                                                           out, out_ok, zero_rest, control_of(d));
+    SG_CUDA_TRY(launch_early(k_deque_move<T, kMovePush>, grid_for(tiles, 1, m1), kCThreads, s, data, d->seq, ucap,
+                             is_push, in, un, out, out_ok, zero_rest, control_of(d)));
     SG_LAUNCH_CHECK();
-    k_deque_move<T, kMoveLate><<<grid_for(tiles, 1, m2), kCThreads, 0, s>>>(data, d->seq, ucap, is_push, in, un,
-                                                                           out, out_ok, zero_rest, control_of(d));
+    SG_CUDA_TRY(launch_early(k_deque_move<T, kMoveLate>, grid_for(tiles, 1, m2), kCThreads, s, data, d->seq, ucap,
+                             is_push, in, un, out, out_ok, zero_rest, control_of(d)));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -1492,7 +1504,7 @@ vector_call_ends(sg_vector* v, bool clear, cudaStream_t s)
     {
         return st;
     }
-    k_vector_call_ends<<<1, 1, 0, s>>>(v->size, v->capacity, clear, v->sync, v->epoch);
+    SG_CUDA_TRY(launch_early(k_vector_call_ends, 1, 1, s, v->size, v->capacity, clear, v->sync, v->epoch));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -1507,9 +1519,9 @@ sg_status
 push_back_launch(sg_vector* v, const void* values, const uint8_t* pred, int64_t n, uint8_t* out_pushed, cudaStream_t s)
 {
     static const int mg = persistent_grid(k_vector_push_back<T, ROWS>, kCThreads);
-    k_vector_push_back<T, ROWS><<<grid_for(n, ROWS * kCThreads, mg), kCThreads, 0, s>>>(
-            static_cast<T*>(v->data), v->size, v->capacity, static_cast<const T*>(values), pred, n, out_pushed, v->sync,
-            v->epoch, control_of(v));
+    SG_CUDA_TRY(launch_early(k_vector_push_back<T, ROWS>, grid_for(n, ROWS * kCThreads, mg), kCThreads, s,
+                             static_cast<T*>(v->data), v->size, v->capacity, static_cast<const T*>(values), pred, n,
+                             out_pushed, v->sync, v->epoch, control_of(v)));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -1660,8 +1672,8 @@ sg_vector_size(sg_vector* v, void* stream, int64_t* out_size)
         return SG_ERR_BAD_ARG;
     }
     cudaStream_t s = as_stream(stream);
-    k_read_words<<<1, 32, 0, s>>>(reinterpret_cast<const unsigned long long*>(v->size),
-                                  reinterpret_cast<unsigned long long*>(v->host), 1);
+    SG_CUDA_TRY(launch_early(k_read_words, 1, 32, s, reinterpret_cast<const unsigned long long*>(v->size),
+                             reinterpret_cast<unsigned long long*>(v->host), 1));
     SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     long long x = *v->host;
@@ -1699,15 +1711,16 @@ sg_vector_pop_back(sg_vector* v, int64_t n, void* out_values, uint8_t* out_ok, v
     const int g = grid_for(n, kCThreads, 4096);
     if (v->elem_bytes == 4)
     {
-        k_vector_pop_back<uint32_t><<<g, kCThreads, 0, s>>>(static_cast<const uint32_t*>(v->data), v->size,
-                                                            v->capacity, n, static_cast<uint32_t*>(out_values), out_ok,
-                                                            v->sync, v->epoch, control_of(v));
+        SG_CUDA_TRY(launch_early(k_vector_pop_back<uint32_t>, g, kCThreads, s, static_cast<const uint32_t*>(v->data),
+                                 v->size, v->capacity, n, static_cast<uint32_t*>(out_values), out_ok, v->sync, v->epoch,
+                                 control_of(v)));
     }
     else
     {
-        k_vector_pop_back<unsigned long long><<<g, kCThreads, 0, s>>>(
-                static_cast<const unsigned long long*>(v->data), v->size, v->capacity, n,
-                static_cast<unsigned long long*>(out_values), out_ok, v->sync, v->epoch, control_of(v));
+        SG_CUDA_TRY(launch_early(k_vector_pop_back<unsigned long long>, g, kCThreads, s,
+                                 static_cast<const unsigned long long*>(v->data), v->size, v->capacity, n,
+                                 static_cast<unsigned long long*>(out_values), out_ok, v->sync, v->epoch,
+                                 control_of(v)));
     }
     SG_LAUNCH_CHECK();
     return SG_OK;
@@ -1904,9 +1917,8 @@ sg_deque_clear(sg_deque* d, void* stream)
         return st;
     }
     const bool keep = d->capacity <= kTurnsKeptMax;
-    k_deque_reset<<<keep ? grid_for(d->capacity, kCThreads, 256) : 1, kCThreads, 0, s>>>(d->seq, d->counters,
-                                                                                          d->capacity, keep, d->sync,
-                                                                                          d->epoch);
+    SG_CUDA_TRY(launch_early(k_deque_reset, keep ? grid_for(d->capacity, kCThreads, 256) : 1, kCThreads, s, d->seq,
+                             d->counters, d->capacity, keep, d->sync, d->epoch));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -1952,9 +1964,9 @@ sg_deque_size(sg_deque* d, void* stream, int64_t* out_size)
     }
     cudaStream_t s = as_stream(stream);
     static_assert(sizeof(deque_counters) % 8 == 0 && sizeof(deque_counters) <= 32 * 8, "one warp copies the counters");
-    k_read_words<<<1, 32, 0, s>>>(reinterpret_cast<const unsigned long long*>(d->counters),
-                                  reinterpret_cast<unsigned long long*>(d->host),
-                                  static_cast<int>(sizeof(deque_counters) / 8));
+    SG_CUDA_TRY(launch_early(k_read_words, 1, 32, s, reinterpret_cast<const unsigned long long*>(d->counters),
+                             reinterpret_cast<unsigned long long*>(d->host),
+                             static_cast<int>(sizeof(deque_counters) / 8)));
     SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     const long long x = d->host->size;
@@ -2045,9 +2057,9 @@ sg_bitset_count(const uint32_t* blocks, int64_t nbits, void* stream, int64_t* ou
     }
     const int64_t nvec = (nbits + 127) / 128;
     const int grid = grid_for(nvec, kCountThreads * 4, sc.blocks);
-    k_bitset_count<<<grid, kCountThreads, 0, s>>>(blocks, nbits, sc.partials);
+    SG_CUDA_TRY(launch_early(k_bitset_count, grid, kCountThreads, s, blocks, nbits, sc.partials));
     SG_LAUNCH_CHECK();
-    k_sum_partials<<<1, 1024, 0, s>>>(sc.partials, grid, sc.host); // straight into the pinned result
+    SG_CUDA_TRY(launch_early(k_sum_partials, 1, 1024, s, sc.partials, grid, sc.host)); // straight into the pinned result
     SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     *out_count = static_cast<int64_t>(*sc.host);
@@ -2118,7 +2130,8 @@ sg_bitset_count_noalloc(const uint32_t* blocks, int64_t nbits, int64_t* out_coun
         k_bitset_count_chunked<<<chunks, kCountThreads, 0, s>>>(blocks, nbits, scratch);
         SG_LAUNCH_CHECK();
     }
-    k_sum_partials<<<1, 1024, 0, s>>>(scratch, chunks, reinterpret_cast<unsigned long long*>(out_count));
+    SG_CUDA_TRY(launch_early(k_sum_partials, 1, 1024, s, scratch, chunks,
+                             reinterpret_cast<unsigned long long*>(out_count)));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }

@@ -160,15 +160,23 @@ persistent_grid(Kernel kernel, int threads, std::size_t smem = 0)
     return sms * per_sm;
 }
 
+// First statement of a kernel started by launch_early.
+__device__ __forceinline__ void
+wait_for_stream()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Launches a kernel that may be set up while the kernel before it on the stream ends (programmatic dependent launch).
 // Every thread of such a kernel calls wait_for_stream() before it touches memory, so it sees what the stream did before
 // just as after a plain launch, and what follows it on the stream sees the same.  What is overlapped is only the time
 // that starting a grid takes, and that is what bounds calls of a few thousand to a few hundred thousand keys: six set
-// calls on 700 keys 36.1 -> 32.7 us, four map calls on 45 K keys 50.9 -> 41.2 us, on 2^20 keys 84.1 -> 76.2 us, and
-// nothing is lost at 2^24 keys and more.
+// calls on 700 keys 36.1 -> 32.7 us, four map calls on 45 K keys 50.9 -> 41.2 us, on 2^20 keys 84.1 -> 76.2 us; a
+// deque's mixed call of 2^24 elements and its pop 297.9 -> 285.4 us, a vector's push_back of 5 M elements with the
+// bitset work around it 132.8 -> 120.8 us, calls on 697 small tables 97.1 -> 82.8 us.  Nothing is lost at 2^27 keys.
 template <typename... Params, typename... Args>
 inline cudaError_t
-launch_early(void (*kernel)(Params...), int grid, int block, cudaStream_t s, Args... args)
+launch_early_shared(void (*kernel)(Params...), int grid, int block, size_t shared, cudaStream_t s, Args... args)
 {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -176,10 +184,18 @@ launch_early(void (*kernel)(Params...), int grid, int block, cudaStream_t s, Arg
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>(grid));
     cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = shared;
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t
+launch_early(void (*kernel)(Params...), int grid, int block, cudaStream_t s, Args... args)
+{
+    return launch_early_shared(kernel, grid, block, 0, s, args...);
 }
 
 inline int

@@ -167,13 +167,6 @@ claim_slot(const dview& t, uint32_t slot, bool erased, typename kind_consts<KIND
     return claim_slot_image<KIND>(p, exp, key, val, old_key);
 }
 
-// First statement of a kernel started by launch_early.
-SG_D void
-wait_for_stream()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // Input element i: value_type array (AoS) or separate key / mapped arrays.
 template <int KIND, bool AOS>
 SG_D void

@@ -56,3 +56,58 @@ def test_calls_see_the_stream_before_them(n):
         assert torch.equal(out, want) and t.size() == n - n // 2
     assert t.valid()
     sg.unordered_set.destroyDeviceObject(t)
+
+
+@pytest.mark.parametrize("n", [1, 513, 70000, (1 << 21) + 5])
+def test_container_calls_see_the_stream_before_them(n):
+    v = sg.vector.createDeviceObject(2 * n, elem_bytes=8)
+    d = sg.deque.createDeviceObject(2 * n, elem_bytes=8)
+    src = torch.arange(1, n + 1, dtype=torch.int64, device="cuda")
+    mixed = torch.arange(n, device="cuda").remainder(2).to(torch.uint8)
+    buf = torch.zeros_like(src)
+    pred = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    pushes = int(mixed.sum())
+    for _ in range(3):
+        v.clear()
+        d.clear()
+        buf.copy_(src)
+        pred.copy_(mixed)
+        v.push_back(buf, pred)
+        pred.zero_()
+        d.push_back(buf)
+        buf.zero_()
+        vals, ok = v.pop_back(pushes)
+        assert v.size() == 0 and bool(ok.all()) and torch.equal(vals.sort().values, src[mixed.bool()])
+        buf.copy_(src)
+        pred.copy_(mixed)
+        popped, done = d.ops(pred, buf)  # the pops take the first elements, the pushes go behind them
+        buf.zero_()
+        pred.zero_()
+        assert bool(done.all()) and torch.equal(popped[~mixed.bool()].sort().values, src[: n - pushes])
+        vals, ok = d.pop_front(n + 1)
+        left = n - (n - pushes) + pushes
+        assert int(ok.sum()) == min(left, n + 1) and d.size() == left - int(ok.sum())
+        assert torch.equal(vals[: n - (n - pushes)], src[n - pushes :])
+    sg.vector.destroyDeviceObject(v)
+    sg.deque.destroyDeviceObject(d)
+
+
+def test_batched_calls_see_the_stream_before_them():
+    per, tables = 300, 200
+    b = sg.table_batch.createDeviceObjects([per] * tables, key="u64")
+    src = torch.arange(1, per * tables + 1, dtype=torch.int64, device="cuda")
+    offsets = torch.arange(tables + 1, dtype=torch.int64, device="cuda") * per
+    buf, off = torch.zeros_like(src), torch.zeros_like(offsets)
+    for _ in range(3):
+        b.clear()
+        buf.copy_(src)
+        off.copy_(offsets)
+        b.insert(buf, off)
+        buf.copy_(src + per)  # the next table's keys
+        none = b.contains(buf, off)
+        buf.copy_(src)
+        every = b.contains(buf, off)
+        off.zero_()
+        buf.zero_()
+        assert int(none.sum()) == 0 and int(every.sum()) == per * tables
+    sg.table_batch.destroyDeviceObjects(b)
