@@ -210,8 +210,8 @@ SG_API sg_status sg_unordered_set_insert_mode(sg_unordered* table, int32_t mode)
  * once that list is empty or the table is full (src/stdgpu/impl/unordered_base_detail.cuh:708-809, 958-994),
  * which can happen below max_size().  With the accounting on (on = 1), a table tracks the same state --
  * which buckets' own slots are taken and how many keys hold excess slots -- and refuses exactly then; bulk
- * inserts and erases then run one thread per key under the stripe locks, and a call of at most 4096 keys
- * that could reach the refusal takes its keys in input order, as the reference does on one thread.  Off
+ * inserts take the stripe locks only when the call could reach the refusal, and such a call of at most 4096
+ * keys takes its keys in input order, as the reference does on one thread.  Off
  * (on = 0), a table takes keys until no slot is free, through the tile and partitioned kernels.  On by
  * default for tables whose max_size() is at most 2^20; switched only on an empty table (size 0, else
  * SG_ERR_BAD_ARG), starting from the reference's empty state.  Synchronises.  Kept by rehash and clear;

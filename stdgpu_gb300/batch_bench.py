@@ -115,6 +115,11 @@ def run(steps: int = 5, warmup: int = 3, tuning: dict | None = None) -> dict:
     batched_ms = time_batched(batch, d_keys, d_q, d_off, out, steps, warmup)
     hits = int(out.sum())
     sizes = batch.sizes()
+    launches = C.kernel_launch_count()
+    batch.clear()
+    batch.insert(d_keys, d_off)
+    batch.contains(d_q, d_off, out=out)
+    launches = C.kernel_launch_count() - launches
     graph_ms = time_graph(batch, d_keys, d_q, d_off, out, steps, warmup)
     hits_graph = int(out.sum())
     storage = batch.storage_bytes()
@@ -131,5 +136,5 @@ def run(steps: int = 5, warmup: int = 3, tuning: dict | None = None) -> dict:
         "batched_mops": ops / (batched_ms * 1e-3) / 1e6, "graph_mops": ops / (graph_ms * 1e-3) / 1e6,
         "plain_mops": ops / (plain_ms * 1e-3) / 1e6,
         "results_agree": bool(hits == hits_graph == hits_plain and np.array_equal(sizes, expect)),
-        "launches_per_step": {"plain": 3 * len(counts), "batched": 5},
+        "launches_per_step": {"plain": 3 * len(counts), "batched": launches},
     }

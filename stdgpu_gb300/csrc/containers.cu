@@ -548,9 +548,9 @@ k_deque_rebuild_turns(unsigned* seq, const deque_counters* c, const sg_deque_syn
 // kMoveFirst: pops of elements stored before the call, every outcome, and the pushes too when they meet no pop
 // at a slot (the other two launches then return at once); else kMovePush and kMoveLate follow, pushes
 // and then the pops of elements that the call pushed.
-// 2^24 mixed operations on 8-byte elements in steady state: 124 us in all, 303 us when every slot's turn word
-// was read, waited on and written (and the outputs filled before); from an empty deque, where each pop depends on a
-// push of the call, 375 us against 779 us.
+// 2^24 mixed operations on 8-byte elements in steady state: 116 us in all (124 before launch_early), 303 us when
+// every slot's turn word was read, waited on and written (and the outputs filled before); from an empty deque, where
+// each pop depends on a push of the call, 262 us against 779 us.
 enum move_phase : int
 {
     kMoveFirst = 0,
@@ -558,9 +558,10 @@ enum move_phase : int
     kMoveLate = 2
 };
 
-// Compiled for 8 resident blocks per SM, two rows in flight at a time: 124 us; 7 blocks and 4 rows 126, 7 and 8 rows
-// 139, 6 and 8 rows 144 us (ranks in 64 bits 153), the 4 blocks that 64 registers allow 162 us: the loads wait for the
-// flags and the counts, and other warps fill that wait better than more loads per warp.
+// Compiled for 8 resident blocks per SM, two rows in flight at a time: 124 us (as plain launches, like the rest of
+// this line); 7 blocks and 4 rows 126, 7 and 8 rows 139, 6 and 8 rows 144 us (ranks in 64 bits 153), the 4 blocks that
+// 64 registers allow 162 us: the loads wait for the flags and the counts, and other warps fill that wait better than
+// more loads per warp.
 template <typename T, int PHASE>
 __global__ void __launch_bounds__(kCThreads, 8)
 k_deque_move(T* data, const unsigned* before, unsigned ucap, const uint8_t* is_push, const T* values, unsigned n,

@@ -68,7 +68,7 @@ static_assert(sizeof(table_header) <= kCountedControlOffset &&
 
 // The device header into its pinned host mirror.  Behind other work of the stream a kernel's stores are there sooner
 // than a copy of 64 bytes, which another engine starts when the kernels are done: a pass of clear, insert, contains,
-// erase and size() on a set of 2^20 keys takes 87.7 us, 90.7 with cudaMemcpyAsync (size() of an idle table: 11.5
+// erase and size() on a set of 2^20 keys took 87.7 us, 90.7 with cudaMemcpyAsync (size() of an idle table: 11.5
 // and 10.3 us).
 __global__ void
 k_read_header(const table_header* hdr, unsigned long long* host)
@@ -83,7 +83,8 @@ k_read_header(const table_header* hdr, unsigned long long* host)
 // Fills every slot with the never-used marker and the slots at or above total_count with the erased
 // marker; resets the header and the accounting's arrays.  clear(): unordered_base_detail.cuh:1220-1252, one
 // launch instead of four.  A small table's clear is bound by its launches: with the accounting's arrays reset by
-// four memsets before this kernel a clear at capacity 1000 took 8.9 us (back to back on the device), now 4.1.
+// four memsets before this kernel a clear at capacity 1000 took 8.9 us (back to back on the device), one
+// plain launch 4.1, and behind another early launch it takes 1.5.
 template <int KIND>
 __global__ void __launch_bounds__(kThreads)
 k_init(dview t, accounting_init acc)
@@ -831,12 +832,12 @@ constexpr unsigned int kCountedImmediate = 1u; // one thread per key, stripe loc
 constexpr unsigned int kCountedInOrder = 2u;   // one thread
 
 // A call of at most this many keys runs its three passes in one launch, a cluster of blocks with hardware
-// barriers between the passes: such a call is bound by its launches (4.1 us each, back to back) and by the chain
-// of dependent reads.  700 keys, capacity 1000: one cluster 10.2 us; a memset and three launches, the inserts one
-// thread per key in one block and every key racing for its group's first free slot, 21.0 us.  Above it, the three
-// launches: 45 K keys of a map<u32,u32> 16.4 us, 22.2 us before with the memset and one thread per key.  The line
-// is the size up to which a call that could reach the refusal takes its keys in input order; the largest call
-// below it gives each thread of the cluster two keys.
+// barriers between the passes: such a call is bound by its launches (a plain one takes 4.1 us, back to back)
+// and by the chain of dependent reads.  700 keys, capacity 1000: one cluster 10.2 us (7.3 by launch_early); a memset
+// and three launches, the inserts one thread per key in one block and every key racing for its group's first free
+// slot, 21.0 us.  Above it, the three launches: 45 K keys of a map<u32,u32> 16.4 us (10.0 by launch_early), 22.2 us
+// before with the memset and one thread per key.  The line is the size up to which a call that could reach the
+// refusal takes its keys in input order; the largest call below it gives each thread of the cluster two keys.
 constexpr int kCountedClusterBlocks = 8;
 constexpr int64_t kCountedClusterMax = 4096;
 
