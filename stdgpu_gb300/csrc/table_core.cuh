@@ -347,10 +347,25 @@ special_erase(const dview& t, typename kind_consts<KIND>::K key)
 
 constexpr int kTile = 4;
 
+// CACHED: the line may come from the SM's own cache, for launches that change no slot.  Queries that repeat hot keys
+// otherwise all go to the L2 slices that hold those keys' lines and wait there: four calls with 2^22 Zipf keys (0.99)
+// on a live map 445 -> 392 us, while lookups of distinct keys, which find nothing in that cache, lose nothing (a step
+// with 2^27 queries 10036 and 10040 us, with 2^20 in L2 77.1 and 77.0).  Lookups of a batch of tables stay without:
+// with it 1054.8 -> 1060.2 us, and 1159 us with a range of queries to each block, so that small tables would be
+// cached.  Not for inserts and erases: a line kept there misses what other SMs stored or erased, so that copies of a
+// hot key would each go to the compare-and-swap.
+template <bool CACHED = false>
 SG_D void
 load_sector(const dview& t, uint32_t g, int q, uint32_t (&w)[8])
 {
     const char* p = t.slots + (static_cast<uint64_t>(g) << 7) + 32 * q;
+    if constexpr (CACHED)
+    {
+        asm volatile("ld.global.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                     : "l"(p));
+        return;
+    }
     asm volatile("ld.global.cg.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                  : "l"(p));
@@ -773,7 +788,7 @@ tile_pick(const V (&v)[kTile], const tile_lanes& L)
 
 // Loads the home groups of the tile's 4 keys and returns the lane's own home group; a lane with nothing to probe has
 // home 0 (a valid group, read and ignored).
-template <int KIND>
+template <int KIND, bool CACHED = false>
 SG_D uint32_t
 load_homes(const dview& t, const tile_lanes& L, uint64_t hash, bool probe, uint32_t (&pre)[kTile][8])
 {
@@ -781,7 +796,7 @@ load_homes(const dview& t, const tile_lanes& L, uint64_t hash, bool probe, uint3
 #pragma unroll
     for (int r = 0; r < kTile; ++r)
     {
-        load_sector(t, __shfl_sync(0xffffffffu, home, L.tbase + r), L.q, pre[r]);
+        load_sector<CACHED>(t, __shfl_sync(0xffffffffu, home, L.tbase + r), L.q, pre[r]);
     }
     return home;
 }
@@ -950,7 +965,7 @@ insert_step(const dview& t, const tile_lanes& L, const void* in0, const void* in
 
 // Locates the slot of each lane's key (-1 when absent); with WANT_VALUE the mapped value comes back in
 // val.  Keys not decided in their home group (group full of other keys) continue with tile_find.
-template <int KIND, bool WANT_VALUE>
+template <int KIND, bool WANT_VALUE, bool CACHED = false>
 SG_D int32_t
 locate_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K key, uint64_t hash, bool probe,
             typename kind_consts<KIND>::V& val)
@@ -961,7 +976,7 @@ locate_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K k
     constexpr uint32_t G = C::slots_per_group;
     constexpr uint32_t S = sector_consts<KIND>::slots;
     uint32_t pre[kTile][8];
-    const uint32_t home = load_homes<KIND>(t, L, hash, probe, pre);
+    const uint32_t home = load_homes<KIND, CACHED>(t, L, hash, probe, pre);
     uint32_t match = 0u, never = 0u; // what the lane's sector of key r's group holds, in byte r
     V vals[kTile];
 #pragma unroll
@@ -1114,7 +1129,7 @@ erase_step(const dview& t, const tile_lanes& L, const void* keys, int64_t i, boo
 // Find / contains step.  zero_absent: an absent key's mapped value is written as 0 (else left alone), so a caller
 // that wants it so needs no pass over the output before the call (which cost 70 us of a 3.73 ms find of 2^27
 // queries, and a launch of 4 us and 16 us of host time before a find of 60 K queries).
-template <int KIND, bool WANT_VALUES>
+template <int KIND, bool WANT_VALUES, bool CACHED = false>
 SG_D void
 find_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K key, int64_t i, bool valid,
               void* out_vals, uint8_t* out_found, const uint64_t* hashes = nullptr, bool zero_absent = false)
@@ -1132,7 +1147,7 @@ find_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K
     const bool probe = valid && !special;
     V pv{};
     const uint64_t hash = hashes != nullptr && probe ? __ldcs(hashes + i) : static_cast<uint64_t>(key);
-    const int32_t slot = locate_step<KIND, WANT_VALUES>(t, L, key, hash, probe, pv);
+    const int32_t slot = locate_step<KIND, WANT_VALUES, CACHED>(t, L, key, hash, probe, pv);
     if (probe)
     {
         found = slot >= 0;
@@ -1155,14 +1170,14 @@ find_key_step(const dview& t, const tile_lanes& L, typename kind_consts<KIND>::K
     step_end();
 }
 
-template <int KIND, bool WANT_VALUES>
+template <int KIND, bool WANT_VALUES, bool CACHED = false>
 SG_D void
 find_step(const dview& t, const tile_lanes& L, const void* keys, int64_t i, bool valid, void* out_vals,
           uint8_t* out_found, const uint64_t* hashes = nullptr, bool zero_absent = false)
 {
     using K = typename kind_consts<KIND>::K;
     const K key = valid ? __ldcs(reinterpret_cast<const K*>(keys) + i) : kind_consts<KIND>::empty_key;
-    find_key_step<KIND, WANT_VALUES>(t, L, key, i, valid, out_vals, out_found, hashes, zero_absent);
+    find_key_step<KIND, WANT_VALUES, CACHED>(t, L, key, i, valid, out_vals, out_found, hashes, zero_absent);
 }
 
 } // namespace detail

@@ -1210,7 +1210,7 @@ k_find(dview t, const void* keys, int64_t n, void* out_vals, uint8_t* out_found,
     for (int64_t base = warp * 32; base < n; base += nwarps * 32)
     {
         const int64_t i = base + L.lane;
-        find_step<KIND, WANT_VALUES>(t, L, keys, i, i < n, out_vals, out_found, hashes, zero_absent);
+        find_step<KIND, WANT_VALUES, true>(t, L, keys, i, i < n, out_vals, out_found, hashes, zero_absent);
     }
 }
 

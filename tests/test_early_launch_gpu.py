@@ -111,3 +111,24 @@ def test_batched_calls_see_the_stream_before_them():
         buf.zero_()
         assert int(none.sum()) == 0 and int(every.sum()) == per * tables
     sg.table_batch.destroyDeviceObjects(b)
+
+
+@pytest.mark.parametrize("n", [32, 4097, 300000])
+def test_lookups_of_hot_keys_see_the_last_calls(n):
+    """Queries that repeat few keys, which a lookup may read from the SM's own cache, between calls that store and
+    erase those keys."""
+    t = sg.unordered_map.createDeviceObject(3000, key="u64", mapped="u32")
+    hot = torch.arange(1, 101, dtype=torch.int64, device="cuda") * 0x9E3779B97F4A7C1
+    pick = torch.arange(n, device="cuda").remainder(100)
+    for call in range(1, 4):
+        stored = hot[: 30 * call]
+        t.insert(stored, torch.full((30 * call,), call, dtype=torch.int32, device="cuda"))
+        vals, found = t.find(hot[pick])
+        assert torch.equal(found.bool(), pick < 30 * call)
+        assert torch.equal(vals != 0, pick < 30 * call)
+        t.erase(stored[:10])
+        assert torch.equal(t.contains(hot[pick]).bool(), (pick >= 10) & (pick < 30 * call))
+        t.insert(stored[:10], torch.full((10,), 9, dtype=torch.int32, device="cuda"))
+        vals, _ = t.find(hot[pick])
+        assert torch.equal(vals[pick < 10], torch.full_like(vals[pick < 10], 9))
+    sg.unordered_map.destroyDeviceObject(t)
