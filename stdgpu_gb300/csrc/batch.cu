@@ -102,7 +102,7 @@ tile_table(const int64_t* prefix, int32_t n, int64_t x)
         while (hi - lo > 1)
         {
             const int32_t mid = (lo + hi) >> 1;
-            if (__ldg(prefix + mid) <= x)
+            if (prefix[mid] <= x)
             {
                 lo = mid;
             }
@@ -187,7 +187,7 @@ k_batch_lists(const dview* views, const int64_t* offsets, const int64_t* prefix,
     auto& s = *reinterpret_cast<list_tile<E, PER>*>(smem);
     __shared__ int32_t s_table;
     // a block takes consecutive tiles: one search, then the tables in order
-    const int64_t tiles = __ldg(prefix + n);
+    const int64_t tiles = prefix[n];
     const int64_t x_lo = tiles * blockIdx.x / gridDim.x, x_hi = tiles * (blockIdx.x + 1) / gridDim.x;
     if (x_lo == x_hi)
     {
@@ -205,15 +205,15 @@ k_batch_lists(const dview* views, const int64_t* offsets, const int64_t* prefix,
     int32_t tb = s_table;
     for (int64_t x = x_lo; x < x_hi; ++x)
     {
-        while (__ldg(prefix + tb + 1) <= x)
+        while (prefix[tb + 1] <= x)
         {
             ++tb;
         }
         const dview t = views[tb];
-        const int32_t i0 = __ldg(first_item + tb);
-        const int regions = __ldg(first_item + tb + 1) - i0;
-        const int64_t lo = __ldg(offsets + tb) + (x - __ldg(prefix + tb)) * kTile;
-        const int64_t hi = __ldg(offsets + tb + 1);
+        const int32_t i0 = first_item[tb];
+        const int regions = first_item[tb + 1] - i0;
+        const int64_t lo = offsets[tb] + (x - prefix[tb]) * kTile;
+        const int64_t hi = offsets[tb + 1];
         E elem[PER];
         int rid[PER];
 #pragma unroll
@@ -273,9 +273,9 @@ k_batch_build(const dview* views, const int64_t* offsets, const build_item* item
     extern __shared__ __align__(128) unsigned char smem[];
     const build_item it = items[blockIdx.x];
     const dview t = views[it.table];
-    const int64_t lo = __ldg(offsets + it.table), hi = __ldg(offsets + it.table + 1);
+    const int64_t lo = offsets[it.table], hi = offsets[it.table + 1];
     const unsigned int listed = fill[blockIdx.x];
-    if (__ldg(build + it.table) == 0)
+    if (build[it.table] == 0)
     {
         return;
     }
@@ -372,7 +372,7 @@ k_batch(const dview* views, const int64_t* offsets, const int64_t* prefix, int32
     const tile_lanes L;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    const int64_t tiles = __ldg(prefix + n);
+    const int64_t tiles = prefix[n];
     unsigned long long retry = 0;
     const int64_t share = tiles / nwarps;
     tiles_per_step = share < tiles_per_step ? (share < 1 ? 1 : static_cast<int>(share)) : tiles_per_step;
@@ -381,17 +381,17 @@ k_batch(const dview* views, const int64_t* offsets, const int64_t* prefix, int32
         const int64_t x1 = x0 + tiles_per_step < tiles ? x0 + tiles_per_step : tiles;
         // one search per step, then the tables in order; a table's counts are added once per step
         int32_t tb = tile_table(prefix, n, x0);
-        int64_t next = __ldg(prefix + tb + 1); // first tile of the table after
+        int64_t next = prefix[tb + 1]; // first tile of the table after
         for (int64_t x = x0; x < x1;)
         {
             while (next <= x)
             {
                 ++tb;
-                next = __ldg(prefix + tb + 1);
+                next = prefix[tb + 1];
             }
             const dview t = views[tb];
-            const int64_t end = __ldg(offsets + tb + 1);
-            int64_t i = __ldg(offsets + tb) + (x - __ldg(prefix + tb)) * 32 + L.lane;
+            const int64_t end = offsets[tb + 1];
+            int64_t i = offsets[tb] + (x - prefix[tb]) * 32 + L.lane;
             step_counts c;
             for (const int64_t stop = next < x1 ? next : x1; x < stop; ++x, i += 32)
             {

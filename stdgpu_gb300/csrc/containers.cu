@@ -193,15 +193,15 @@ k_vector_push_back(T* data, long long* size, int64_t cap, const T* values, const
         {
             if constexpr (ROWS == 32)
             {
-                const uint4 a = __ldg(reinterpret_cast<const uint4*>(pred + mine));
-                const uint4 b = __ldg(reinterpret_cast<const uint4*>(pred + mine) + 1);
+                const uint4 a = __ldcs(reinterpret_cast<const uint4*>(pred + mine));
+                const uint4 b = __ldcs(reinterpret_cast<const uint4*>(pred + mine) + 1);
                 bits = nonzero_bytes(a.x) | nonzero_bytes(a.y) << 4 | nonzero_bytes(a.z) << 8 |
                        nonzero_bytes(a.w) << 12 | nonzero_bytes(b.x) << 16 | nonzero_bytes(b.y) << 20 |
                        nonzero_bytes(b.z) << 24 | nonzero_bytes(b.w) << 28;
             }
             else
             {
-                bits = nonzero_bytes(__ldg(reinterpret_cast<const unsigned*>(pred + mine)));
+                bits = nonzero_bytes(__ldcs(reinterpret_cast<const unsigned*>(pred + mine)));
             }
         }
         else
@@ -407,7 +407,7 @@ k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters
 #pragma unroll
             for (int k = 0; k < kPlanTile / 512; ++k)
             {
-                const uint4 x = __ldg(p + k * 32 + lane);
+                const uint4 x = p[k * 32 + lane];
                 count += __popc(__vsetne4(x.x, 0u)) + __popc(__vsetne4(x.y, 0u)) + __popc(__vsetne4(x.z, 0u)) +
                          __popc(__vsetne4(x.w, 0u));
             }
@@ -599,7 +599,7 @@ k_deque_move(T* data, const unsigned* before, unsigned ucap, const uint8_t* is_p
             s_warp[buf][warp] = total;
         }
         __syncthreads();
-        unsigned rank = __ldg(before + tile); // pushes before the tile, then before the row
+        unsigned rank = before[tile]; // pushes before the tile, then before the row
         for (int w = 0; w < warp; ++w)
         {
             rank += s_warp[buf][w];

@@ -160,7 +160,9 @@ persistent_grid(Kernel kernel, int threads, std::size_t smem = 0)
     return sms * per_sm;
 }
 
-// First statement of a kernel started by launch_early.
+// First statement of a kernel started by launch_early.  No such kernel reads by __ldg or through a __restrict__
+// pointer: those promise that nothing writes the data while the kernel runs, which the work before it on the stream
+// still does until the wait returns, so a compiler may move such a load above the wait.
 __device__ __forceinline__ void
 wait_for_stream()
 {

@@ -858,7 +858,7 @@ template <int KIND>
 SG_D uint64_t
 counted_hash(typename kind_consts<KIND>::K key, const uint64_t* hashes, int64_t i)
 {
-    return hashes != nullptr ? __ldg(hashes + i) : identity_word_hash{}(key);
+    return hashes != nullptr ? hashes[i] : identity_word_hash{}(key);
 }
 
 // Pass 1: candidate per bucket (atomic minimum of the input indices of keys not stored) and the call's bounds.
@@ -1151,7 +1151,7 @@ k_erase_counted(dview t, sg_unordered_view v, const void* keys, int64_t n, uint8
         uint64_t hash = 0;
         if (valid)
         {
-            key = __ldg(static_cast<const K*>(keys) + i);
+            key = static_cast<const K*>(keys)[i];
             hash = counted_hash<KIND>(key, hashes, i);
         }
         const bool special = valid && key >= C::tomb_key;
