@@ -1,0 +1,191 @@
+"""Batched inserts without per-key flags, where tables of several regions (256 probe groups each) are built from lists
+of their regions' keys: every kind of table around one region, several regions, 1024 regions (the most that are built)
+and above; out-of-band keys; keys that spill over a region's end, into the next region and around the table's end, and
+more of them than the spill buffer takes; a key repeated past a list's length.  What every slot of a table holds, the
+sizes and the lookups are those of a dict per table."""
+
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+import stdgpu_gb300 as sg
+from stdgpu_gb300.containers import _DeviceArray
+
+from gpu_util import dev, host
+
+pytestmark = pytest.mark.gpu
+
+REGION, REGIONS, SPILLS = 256, 1024, 1 << 15  # kRegionGroups, kListRegions, kSpillMax
+KINDS = [O.SET_U32, O.SET_U64, O.MAP_U64_U32, O.MAP_U64_U64, O.MAP_U32_U32, O.MAP_U32_U64]
+SLOT = {O.SET_U32: 4, O.SET_U64: 8, O.MAP_U64_U32: 16, O.MAP_U64_U64: 16, O.MAP_U32_U32: 8, O.MAP_U32_U64: 16}
+NAME = {np.dtype(np.uint32): "u32", np.dtype(np.uint64): "u64"}
+
+
+def _names(kind):
+    vd = O.VAL_DTYPE[kind]
+    return NAME[np.dtype(O.KEY_DTYPE[kind])], (None if vd is None else NAME[np.dtype(vd)])
+
+
+def _geometry(kind, cap):
+    return sg.geometry_for(sg.KINDS[_names(kind)], int(cap))
+
+
+def _cap_with_groups(kind, groups):
+    """The smallest capacity whose table has at least `groups` probe groups."""
+    lo, hi = 1, groups * 128 // SLOT[kind]
+    while lo < hi:
+        mid = (lo + hi) // 2
+        if _geometry(kind, mid).num_groups >= groups:
+            hi = mid
+        else:
+            lo = mid + 1
+    return lo
+
+
+def _home(kind, cap, keys):
+    """Home probe group of each key."""
+    g = _geometry(kind, cap)
+    bits = int(g.bucket_count).bit_length() - 1
+    k = keys.astype(np.uint64)
+    if bits == 0:
+        return np.zeros(len(k), np.int64)
+    drop = np.uint64(64 - bits)
+    with np.errstate(over="ignore"):
+        bucket = ((k ^ (k >> drop)) * np.uint64(11400714819323198485)) >> drop
+    return ((bucket * np.uint64(g.num_groups)) >> np.uint64(bits)).astype(np.int64)
+
+
+def _random(kind, n, rng):
+    kd = np.dtype(O.KEY_DTYPE[kind])
+    return np.unique(rng.integers(1, np.iinfo(kd).max - 1, size=n + n // 8 + 8, dtype=np.uint64).astype(kd))[:n]
+
+
+def _near(kind, cap, first, last, count, rng):
+    """`count` distinct keys whose home group lies in [first, last)."""
+    out = np.zeros(0, O.KEY_DTYPE[kind])
+    while len(out) < count:
+        k = _random(kind, 1 << 20, rng)
+        h = _home(kind, cap, k)
+        out = np.unique(np.concatenate([out, k[(h >= first) & (h < last)]]))
+    return rng.permutation(out)[:count]
+
+
+def _stored(b, kind, t):
+    """{key: mapped value} of table t's slot image; a key stored twice fails."""
+    v = b.view(t)
+    raw = torch.as_tensor(_DeviceArray(v.slots, (int(v.num_groups) + 1) * 16, 8), device="cuda").cpu().numpy()
+    sb = SLOT[kind]
+    rows = raw.view(np.uint8).reshape(-1, sb)
+    kd, vd = np.dtype(O.KEY_DTYPE[kind]), O.VAL_DTYPE[kind]
+    top = np.iinfo(kd).max
+    keys = np.ascontiguousarray(rows[:, : kd.itemsize]).view(kd).ravel()
+    n = int(v.num_groups) * (128 // sb)
+    live = np.nonzero(keys[:n] < top - kd.type(1))[0]
+    vals = keys[live]
+    if vd is not None:
+        at = 4 if sb == 8 else 8
+        vals = np.ascontiguousarray(rows[:, at: at + np.dtype(vd).itemsize]).view(vd).ravel()[live]
+    assert len(np.unique(keys[live])) == len(live), t
+    assert (keys[int(v.total_count):n] == top - kd.type(1)).all(), t  # the erased marker at and above total_count
+    return dict(zip(keys[live].tolist(), vals.tolist()))
+
+
+def _refused(b, t):
+    return int(torch.as_tensor(_DeviceArray(b.view(t).header, 8, 8), device="cuda")[1].item())
+
+
+def _value(kind, keys):
+    vd = O.VAL_DTYPE[kind]
+    return None if vd is None else (keys >> keys.dtype.type(1)).astype(vd)
+
+
+def _insert_and_check(kind, caps, keys, full=()):
+    """One insert into fresh tables without flags; tables in `full` get more distinct keys than they take."""
+    ks, ms = _names(kind)
+    kd, vd = np.dtype(O.KEY_DTYPE[kind]), O.VAL_DTYPE[kind]
+    top = np.iinfo(kd).max
+    b = sg.table_batch.createDeviceObjects(caps, key=ks, mapped=ms)
+    flat = np.concatenate(keys).astype(kd)
+    off = np.concatenate([[0], np.cumsum([len(k) for k in keys])]).astype(np.int64)
+    vals = _value(kind, flat)
+    for _ in range(2):  # again after a clear
+        b.insert(dev(flat), dev(off), dev(vals) if vals is not None else None)
+        sizes = b.sizes()
+        got, found = b.find(dev(flat), dev(off))
+        found = found.cpu().numpy()
+        for t, cap in enumerate(caps):
+            k = keys[t]
+            lo, hi = off[t], off[t + 1]
+            want = {int(x): int(y) for x, y in zip(k, k if vd is None else _value(kind, k)) if x < top - kd.type(1)}
+            special = len(set(k.tolist()) & {int(top), int(top) - 1})
+            held = _stored(b, kind, t)
+            if t in full:
+                room = _geometry(kind, cap).max_size
+                assert len(held) == room and sizes[t] == room + special, t
+                assert all(want[x] == y for x, y in held.items()), t
+                assert _refused(b, t) == len(want) - room, t
+                assert np.array_equal(found[lo:hi].astype(bool), [x in held or x >= top - 1 for x in k.tolist()]), t
+            else:
+                assert held == want and sizes[t] == len(want) + special, t
+                assert found[lo:hi].all() and _refused(b, t) == 0, t
+                if vd is not None:
+                    assert np.array_equal(host(got, vd)[lo:hi], _value(kind, k)), t
+        b.clear()
+        assert b.sizes().sum() == 0
+    sg.table_batch.destroyDeviceObjects(b)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_tables_around_one_region_and_several(kind):
+    rng = np.random.default_rng(kind)
+    above = _cap_with_groups(kind, REGION + 1)  # (a table of exactly 256 groups does not exist)
+    caps = [1, 40, above - 1, above] + [_cap_with_groups(kind, g) for g in (3 * REGION, 5 * REGION - 3, 9 * REGION + 1)]
+    assert _geometry(kind, above - 1).num_groups <= REGION
+    keys = []
+    for c in caps:
+        k = _random(kind, max(1, c // 2), rng)
+        top = np.iinfo(k.dtype).max
+        k = np.concatenate([k, k[: len(k) // 4], np.array([top, top - 1, top], k.dtype)])  # copies, out-of-band keys
+        keys.append(rng.permutation(k))
+    _insert_and_check(kind, caps, keys)
+
+
+@pytest.mark.parametrize("kind", [O.SET_U64, O.MAP_U64_U64])
+@pytest.mark.parametrize("built", [True, False])
+def test_tables_of_the_most_regions_that_are_built(kind, built):
+    cap = _cap_with_groups(kind, REGIONS * REGION + 1) - int(built)
+    assert (_geometry(kind, cap).num_groups <= REGIONS * REGION) == built
+    rng = np.random.default_rng(50)
+    _insert_and_check(kind, [cap, 5000], [_random(kind, cap // 3, rng), _random(kind, 3000, rng)])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_keys_that_spill_out_of_built_regions(kind):
+    rng = np.random.default_rng(10 + kind)
+    cap = _cap_with_groups(kind, 3 * REGION + 7)
+    groups = _geometry(kind, cap).num_groups
+    slots = 8 * 128 // SLOT[kind]  # of eight groups
+    crowd = _near(kind, cap, REGION - 8, REGION, 3 * slots, rng)       # on into region 1
+    end = _near(kind, cap, groups - 5, groups, 3 * slots, rng)         # around the table's end, into group 0
+    rest = _random(kind, cap // 4, rng)
+    keys = [rng.permutation(np.concatenate([rest, crowd, end, crowd])), rest[:1000].copy()]
+    _insert_and_check(kind, [cap, _cap_with_groups(kind, REGION)], keys)
+
+
+def test_more_spilled_keys_than_the_buffer_takes():
+    kind = O.SET_U64
+    rng = np.random.default_rng(20)
+    cap = _cap_with_groups(kind, 3 * REGION)
+    crowd = _near(kind, cap, REGION - 8, REGION, REGION * 16, rng)  # a list's length; 128 of them fit the region
+    tables = SPILLS // (len(crowd) - 8 * 16) + 3
+    _insert_and_check(kind, [cap] * tables, [rng.permutation(crowd) for _ in range(tables)])
+
+
+@pytest.mark.parametrize("kind", [O.SET_U32, O.SET_U64, O.MAP_U64_U32, O.MAP_U32_U32])
+def test_a_key_repeated_past_a_lists_length(kind):
+    rng = np.random.default_rng(30)
+    cap = _cap_with_groups(kind, 3 * REGION)
+    k = _random(kind, cap // 3, rng)
+    length = REGION * 128 // SLOT[kind]
+    _insert_and_check(kind, [cap, cap], [rng.permutation(np.concatenate([k, np.full(2 * length, k[0])])), k])
