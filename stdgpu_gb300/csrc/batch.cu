@@ -365,7 +365,7 @@ enum batch_op : int
 template <int KIND, int OP, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 k_batch(const dview* views, const int64_t* offsets, const int64_t* prefix, int32_t n, int tiles_per_step,
-        const void* in0, const void* in1, void* out_vals, uint8_t* out_flags, const uint8_t* built,
+        const void* in0, const void* in1, void* out_vals, uint8_t* out_flags, const uint8_t* todo,
         spill_list spills)
 {
     wait_for_stream();
@@ -445,11 +445,16 @@ k_batch(const dview* views, const int64_t* offsets, const int64_t* prefix, int32
     }
     if constexpr (OP == kOpInsertAos || OP == kOpInsertSoa)
     {
-        // keys that found no room in their region, one per warp step (their tables differ)
-        const int64_t spilled = built != nullptr ? min(*spills.count, kSpillMax) : 0u;
+        // keys that found no room in their region, one per warp step (their tables differ); those of a table marked
+        // todo are among the keys walked above, and a full table counts each refused key once
+        const int64_t spilled = todo != nullptr ? min(*spills.count, kSpillMax) : 0u;
         for (int64_t e = warp; e < spilled; e += nwarps)
         {
             const spill_entry x = spills.entry[e];
+            if (todo[x.table] != 0)
+            {
+                continue;
+            }
             const dview t = views[x.table];
             typename kind_consts<KIND>::K key;
             typename kind_consts<KIND>::V val;
@@ -565,14 +570,14 @@ struct batch_launch
     template <int OP, int THREADS>
     static sg_status
     go(sg_table_batch* b, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
-       uint8_t* out_flags, const uint8_t* built, cudaStream_t s)
+       uint8_t* out_flags, const uint8_t* todo, cudaStream_t s)
     {
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<KIND, OP, THREADS>, THREADS, 0);
         per_sm = per_sm < 1 ? 1 : per_sm;
         const int want = b->blocks_per_sm > 0 ? (b->blocks_per_sm < per_sm ? b->blocks_per_sm : per_sm) : per_sm;
         SG_CUDA_TRY(launch_early(k_batch<KIND, OP, THREADS>, b->sms * want, THREADS, s, b->views, offsets, b->prefix,
-                                 b->n, b->tiles_per_step, in0, in1, out_vals, out_flags, built, b->spills));
+                                 b->n, b->tiles_per_step, in0, in1, out_vals, out_flags, todo, b->spills));
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -580,35 +585,35 @@ struct batch_launch
     template <int OP>
     static sg_status
     run_op(sg_table_batch* b, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
-           uint8_t* out_flags, const uint8_t* built, cudaStream_t s)
+           uint8_t* out_flags, const uint8_t* todo, cudaStream_t s)
     {
         switch (b->threads)
         {
             case 128:
-                return go<OP, 128>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return go<OP, 128>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
             case 512:
-                return go<OP, 512>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return go<OP, 512>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
             default:
-                return go<OP, 256>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return go<OP, 256>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
         }
     }
 
     static sg_status
     run(sg_table_batch* b, int op, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
-        uint8_t* out_flags, const uint8_t* built, cudaStream_t s)
+        uint8_t* out_flags, const uint8_t* todo, cudaStream_t s)
     {
         switch (op)
         {
             case kOpInsertAos:
-                return run_op<kOpInsertAos>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return run_op<kOpInsertAos>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
             case kOpInsertSoa:
-                return run_op<kOpInsertSoa>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return run_op<kOpInsertSoa>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
             case kOpErase:
-                return run_op<kOpErase>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return run_op<kOpErase>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
             case kOpFind:
-                return run_op<kOpFind>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return run_op<kOpFind>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
             default:
-                return run_op<kOpContains>(b, offsets, in0, in1, out_vals, out_flags, built, s);
+                return run_op<kOpContains>(b, offsets, in0, in1, out_vals, out_flags, todo, s);
         }
     }
 
@@ -700,25 +705,25 @@ dispatch_op(sg_table_batch* b, int op, const int64_t* offsets, const void* in0, 
             return st;
         }
     }
-    const uint8_t* built = build ? b->marks : nullptr;
+    // the tables whose keys are walked (all, without a build)
+    const uint8_t* todo = build ? b->marks + b->n : nullptr;
     // a NULL key array (all ranges empty, as an empty tensor gives) walks no tile
-    SG_CUDA_TRY(launch_early(k_batch_tiles, 1, 1024, s, offsets, b->n, b->prefix, in0 != nullptr,
-                             build ? b->marks + b->n : nullptr));
+    SG_CUDA_TRY(launch_early(k_batch_tiles, 1, 1024, s, offsets, b->n, b->prefix, in0 != nullptr, todo));
     SG_LAUNCH_CHECK();
     switch (b->kind)
     {
         case 0:
-            return batch_launch<0>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
+            return batch_launch<0>::run(b, op, offsets, in0, in1, out_vals, out_flags, todo, s);
         case 1:
-            return batch_launch<1>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
+            return batch_launch<1>::run(b, op, offsets, in0, in1, out_vals, out_flags, todo, s);
         case 2:
-            return batch_launch<2>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
+            return batch_launch<2>::run(b, op, offsets, in0, in1, out_vals, out_flags, todo, s);
         case 3:
-            return batch_launch<3>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
+            return batch_launch<3>::run(b, op, offsets, in0, in1, out_vals, out_flags, todo, s);
         case 4:
-            return batch_launch<4>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
+            return batch_launch<4>::run(b, op, offsets, in0, in1, out_vals, out_flags, todo, s);
         case 5:
-            return batch_launch<5>::run(b, op, offsets, in0, in1, out_vals, out_flags, built, s);
+            return batch_launch<5>::run(b, op, offsets, in0, in1, out_vals, out_flags, todo, s);
         default:
             return SG_ERR_BAD_ARG;
     }

@@ -1,8 +1,8 @@
 """Batched inserts without per-key flags, where tables of several regions (256 probe groups each) are built from lists
 of their regions' keys: every kind of table around one region, several regions, 1024 regions (the most that are built)
 and above; out-of-band keys; keys that spill over a region's end, into the next region and around the table's end, and
-more of them than the spill buffer takes; a key repeated past a list's length.  What every slot of a table holds, the
-sizes and the lookups are those of a dict per table."""
+more of them than the spill buffer takes; a key repeated past a list's length; tables filled past max_size().
+What every slot of a table holds, the sizes, the refused inserts and the lookups are those of a dict per table."""
 
 import numpy as np
 import pytest
@@ -189,3 +189,13 @@ def test_a_key_repeated_past_a_lists_length(kind):
     k = _random(kind, cap // 3, rng)
     length = REGION * 128 // SLOT[kind]
     _insert_and_check(kind, [cap, cap], [rng.permutation(np.concatenate([k, np.full(2 * length, k[0])])), k])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("groups", [3, REGION, 2 * REGION + 9])
+def test_tables_filled_past_max_size_count_each_refused_key_once(kind, groups):
+    rng = np.random.default_rng(40 + groups)
+    cap = _cap_with_groups(kind, groups)
+    room = _geometry(kind, cap).max_size
+    more = _random(kind, room + 20, rng)
+    _insert_and_check(kind, [cap, cap], [rng.permutation(more), rng.permutation(more[: room // 2])], full=(0,))
