@@ -146,22 +146,27 @@ struct spill_list
 };
 
 // First launch of an insert into a batch that may be empty (one block): build[t] = 1 for a table that holds nothing
-// and gets at least a key per two groups (a region is written whole, so fewer keys are cheaper to insert one by one);
-// todo[t] = 1 for the others that get keys.  Tables of several regions get lists (prefix: their
-// tiles of list_tile elements), which leave no room for an element's index: with per-key flags they go to the probe
-// kernel.
+// and gets at least a key per two groups (a region is written whole, so fewer keys are cheaper to insert one by one)
+// and not many more than it has slots; todo[t] = 1 for the others that get keys.  A table of several regions with more
+// keys than slots is left to the walk, since a list would overflow.  A table of one region is built by one block,
+// whatever copies its keys hold, while that block gets at most twice an even share of the call's keys among
+// `resident` blocks: 697 tables of 1000 with 5000 distinct keys each take 6680 us so, 9074 by the walk, and one table
+// of 1000 with 2^22 copies of 500 keys takes 127 us by the walk, 9270 by one block.  Tables of several regions get
+// lists (prefix: their tiles of list_tile elements), which leave no room for an element's index: with per-key flags
+// they go to the probe kernel.
 __global__ void __launch_bounds__(1024)
 k_batch_choose(const dview* views, const int64_t* offsets, int32_t n, const int32_t* first_item, bool flags, int tile,
-               uint8_t* build, uint8_t* todo, int64_t* prefix)
+               int resident, uint8_t* build, uint8_t* todo, int64_t* prefix)
 {
     wait_for_stream();
+    const int64_t share = 2 * (offsets[n] - offsets[0]) / resident;
     for (int32_t t = threadIdx.x; t < n; t += blockDim.x)
     {
         const dview v = views[t];
         const int64_t cnt = offsets[t + 1] - offsets[t];
         const int32_t regions = first_item[t + 1] - first_item[t];
-        const bool ok = cnt > 0 && 2 * cnt >= v.num_groups && regions > 0 && (regions == 1 || !flags) &&
-                        v.hdr->size == 0 && v.hdr->tombstones == 0;
+        const bool ok = cnt > 0 && 2 * cnt >= v.num_groups && (cnt <= v.total || (regions == 1 && cnt <= share)) &&
+                        regions > 0 && (regions == 1 || !flags) && v.hdr->size == 0 && v.hdr->tombstones == 0;
         build[t] = ok ? 1 : 0;
         todo[t] = cnt > 0 && !ok ? 1 : 0;
     }
@@ -628,7 +633,8 @@ struct batch_launch
         // the lists' lengths, and the spill count behind them
         SG_CUDA_TRY(cudaMemsetAsync(b->fill, 0, sizeof(unsigned int) * static_cast<size_t>(b->n_items + 1), s));
         SG_CUDA_TRY(launch_early(k_batch_choose, 1, 1024, s, b->views, offsets, b->n, b->first_item,
-                                 out_flags != nullptr, kListPer * kListThreads, b->marks, todo, b->list_prefix));
+                                 out_flags != nullptr, kListPer * kListThreads, b->sms * kRegionBlocks, b->marks, todo,
+                                 b->list_prefix));
         SG_LAUNCH_CHECK();
         SG_CUDA_TRY(cudaFuncSetAttribute(k_batch_lists<KIND, AOS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(sizeof(Lists))));

@@ -199,3 +199,31 @@ def test_tables_filled_past_max_size_count_each_refused_key_once(kind, groups):
     room = _geometry(kind, cap).max_size
     more = _random(kind, room + 20, rng)
     _insert_and_check(kind, [cap, cap], [rng.permutation(more), rng.permutation(more[: room // 2])], full=(0,))
+
+
+def _microseconds(call, before):
+    best = float("inf")
+    for _ in range(5):
+        before()
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        call()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("tables", [1, 8])
+def test_many_copies_for_few_small_tables_are_not_left_to_one_block_each(tables):
+    """The first insert into a cleared table costs about what the same insert costs on a table that holds the keys:
+    one block that took all of a table's keys by itself would take far longer than the whole chip."""
+    per = (1 << 22) // tables
+    keys = torch.arange(1, 501, device="cuda").repeat(1 + per // 500)[:per].repeat(tables)
+    off = torch.arange(tables + 1, dtype=torch.int64, device="cuda") * per
+    b = sg.table_batch.createDeviceObjects([1000] * tables, key="u64")
+    first = _microseconds(lambda: b.insert(keys, off), b.clear)
+    assert b.sizes().tolist() == [500] * tables
+    again = _microseconds(lambda: b.insert(keys, off), lambda: None)
+    sg.table_batch.destroyDeviceObjects(b)
+    assert first < 5 * again + 50, (first, again)
