@@ -27,49 +27,64 @@ namespace sg
 namespace detail
 {
 
-// Exclusive scan over the tables t < n of count(t) into prefix[0, n], prefix[n] = the sum, by one block of 1024
-// threads.  The threads' sums go through warp shuffles (one thread walking all 1024 of them took most of the 12 us
-// that the tiles of 4096 tables took; now 6).
-template <typename Count>
+// Exclusive scan over the tables t < n of count(t), handed to put(t, sum before t) for t <= n, by one block of 1024
+// threads, four consecutive tables per thread at a time.  What bounds it is the chain from a round's loads to the
+// next round's: 4 us for up to 4096 tables, 19 for 16384, 71 for 65536.  With a run of tables per thread, read twice
+// and one after another, an insert of 3 keys each into 65536 tables takes 210 us instead of 126.
+template <typename Count, typename Put>
 SG_D void
-scan_tables(int32_t n, int64_t* prefix, Count count)
+scan_tables(int32_t n, Count count, Put put)
 {
-    __shared__ long long warp_sums[32];
+    constexpr int kPer = 4;
+    __shared__ long long warp_sums[2][32];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int64_t per = (static_cast<int64_t>(n) + blockDim.x - 1) / blockDim.x;
-    const int64_t lo = threadIdx.x * per;
-    const int64_t hi = lo + per < n ? lo + per : n;
-    long long s = 0;
-    for (int64_t t = lo; t < hi; ++t)
+    long long carry = 0;
+    int buf = 0;
+    for (int64_t base = 0; base < n; base += kPer * 1024, buf ^= 1)
     {
-        s += count(t);
-    }
-    long long incl = s;
+        const int64_t t0 = base + kPer * static_cast<int64_t>(threadIdx.x);
+        long long c[kPer];
+        long long s = 0;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1)
-    {
-        const long long x = __shfl_up_sync(0xffffffffu, incl, d);
-        incl += lane >= d ? x : 0;
-    }
-    if (lane == 31)
-    {
-        warp_sums[warp] = incl;
-    }
-    __syncthreads();
-    long long run = incl - s;
-    for (int w = 0; w < warp; ++w)
-    {
-        run += warp_sums[w];
-    }
-    for (int64_t t = lo; t < hi; ++t)
-    {
-        prefix[t] = run;
-        run += count(t);
-    }
-    if (threadIdx.x == blockDim.x - 1)
-    {
-        prefix[n] = run;
+        for (int k = 0; k < kPer; ++k)
+        {
+            c[k] = t0 + k < n ? count(t0 + k) : 0;
+            s += c[k];
+        }
+        long long incl = s;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+            const long long x = __shfl_up_sync(0xffffffffu, incl, d);
+            incl += lane >= d ? x : 0;
+        }
+        if (lane == 31)
+        {
+            warp_sums[buf][warp] = incl;
+        }
+        __syncthreads(); // one per round: the next one fills the other buffer
+        const bool more = base + kPer * 1024 < n;
+        long long run = carry + incl - s;
+        for (int w = 0; w < (more ? 32 : warp); ++w)
+        {
+            const long long x = warp_sums[buf][w];
+            run += w < warp ? x : 0;
+            carry += x;
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k)
+        {
+            if (t0 + k < n)
+            {
+                put(t0 + k, run);
+            }
+            run += c[k];
+        }
+        if (!more && threadIdx.x == 1023)
+        {
+            put(n, run);
+        }
     }
 }
 
@@ -82,13 +97,16 @@ tiles_of(const int64_t* offsets, int64_t t, int tile)
 
 // Prefix of tile counts: prefix[t] = sum over u < t of ceil(n_u / 32); prefix[n] = all tiles.  Tables whose `todo`
 // (nullable) is 0 have no tiles.
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(1024, 2)
 k_batch_tiles(const int64_t* offsets, int32_t n, int64_t* prefix, bool has_keys, const uint8_t* todo)
 {
     wait_for_stream();
-    scan_tables(n, prefix, [&](int64_t t) -> long long {
-        return has_keys && (todo == nullptr || todo[t] != 0) ? tiles_of(offsets, t, 32) : 0;
-    });
+    scan_tables(
+            n,
+            [&](int64_t t) -> long long {
+                return has_keys && (todo == nullptr || todo[t] != 0) ? tiles_of(offsets, t, 32) : 0;
+            },
+            [&](int64_t t, long long x) { prefix[t] = x; });
 }
 
 // Table of tile x: the last t with prefix[t] <= x (binary search by lane 0, broadcast to the warp).
@@ -124,10 +142,19 @@ struct build_item
     int32_t table;
     uint32_t first; // groups
     uint32_t count;
-    int32_t whole; // the table's only region: its keys are read from the input, not from a list
+    int32_t list; // its list, or -1 for a table's only region: the keys are read from the input
 };
 
 constexpr int kListPer = 4; // elements per thread and tile of the lists
+
+// Counts of a call, behind the lists' lengths; all zero when it starts.
+struct build_words
+{
+    unsigned int spilled; // keys offered to the spill list
+    unsigned int taken;   // items that blocks have taken beyond their first
+    unsigned int arrived; // blocks of k_batch_choose that are done
+    unsigned int any;     // 1: a table is built
+};
 
 // A key that found no room in its region, for the probe kernel.  More of them than the buffer holds mark their
 // tables todo.
@@ -145,45 +172,103 @@ struct spill_list
     spill_entry* entry;
 };
 
-// First launch of an insert into a batch that may be empty (one block): build[t] = 1 for a table that holds nothing
-// and gets at least a key per two groups (a region is written whole, so fewer keys are cheaper to insert one by one)
-// and not many more than it has slots; todo[t] = 1 for the others that get keys.  A table of several regions with more
+// First launch of an insert into a batch that may be empty: build[t] = 1 for a table that holds nothing and gets at
+// least a key per two groups (a region is written whole, so fewer keys are cheaper to insert one by one) and not many more than it has slots; todo[t] = 1 for the others that get keys.  A table of several regions with more
 // keys than slots is left to the walk, since a list would overflow.  A table of one region is built by one block,
 // whatever copies its keys hold, while that block gets at most twice an even share of the call's keys among
 // `resident` blocks: 697 tables of 1000 with 5000 distinct keys each take 6680 us so, 9074 by the walk, and one table
 // of 1000 with 2^22 copies of 500 keys takes 127 us by the walk, 9270 by one block.  Tables of several regions get
-// lists (prefix: their tiles of list_tile elements), which leave no room for an element's index: with per-key flags
-// they go to the probe kernel.
+// lists (prefix: their tiles of `tile` elements; item_prefix: the regions of the tables before that are built), which
+// leave no room for an element's index: with per-key flags they go to the probe kernel.  The last block to finish adds
+// up the tables, unless none is built: 3 keys each into 65536 cleared tables of 2100 take 155 us, 520 when one block
+// did all of it and each region had its block, 244 with no table ever built.
 __global__ void __launch_bounds__(1024)
 k_batch_choose(const dview* views, const int64_t* offsets, int32_t n, const int32_t* first_item, bool flags, int tile,
-               int resident, uint8_t* build, uint8_t* todo, int64_t* prefix)
+               int resident, uint8_t* build, uint8_t* todo, int64_t* prefix, int64_t* item_prefix, build_words* words)
 {
     wait_for_stream();
-    const int64_t share = 2 * (offsets[n] - offsets[0]) / resident;
-    for (int32_t t = threadIdx.x; t < n; t += blockDim.x)
+    __shared__ unsigned int s_last;
+    const bool alone = gridDim.x == 1;
+    const int64_t twice = 2 * (offsets[n] - offsets[0]);
+    bool any = false;
+    for (int32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
     {
         const dview v = views[t];
         const int64_t cnt = offsets[t + 1] - offsets[t];
         const int32_t regions = first_item[t + 1] - first_item[t];
-        const bool ok = cnt > 0 && 2 * cnt >= v.num_groups && (cnt <= v.total || (regions == 1 && cnt <= share)) &&
-                        regions > 0 && (regions == 1 || !flags) && v.hdr->size == 0 && v.hdr->tombstones == 0;
+        const bool ok = cnt > 0 && 2 * cnt >= v.num_groups &&
+                        (cnt <= v.total || (regions == 1 && cnt * resident <= twice)) && regions > 0 &&
+                        (regions == 1 || !flags) && v.hdr->size == 0 && v.hdr->tombstones == 0;
         build[t] = ok ? 1 : 0;
         todo[t] = cnt > 0 && !ok ? 1 : 0;
+        any = any || ok;
     }
-    __syncthreads();
-    scan_tables(n, prefix, [&](int64_t t) -> long long {
-        return build[t] != 0 && first_item[t + 1] - first_item[t] > 1 ? tiles_of(offsets, t, tile) : 0;
-    });
+    any = __syncthreads_or(any) != 0;
+    if (!alone)
+    {
+        if (threadIdx.x == 0)
+        {
+            if (any)
+            {
+                atomicOr(&words->any, 1u);
+            }
+            __threadfence();
+            s_last = atomicAdd(&words->arrived, 1u) == gridDim.x - 1 ? 1u : 0u;
+            __threadfence();
+        }
+        __syncthreads();
+        if (s_last == 0u)
+        {
+            return;
+        }
+        // the last block has all tables' marks
+        any = __ldcg(&words->any) != 0u;
+    }
+    if (!any)
+    {
+        if (threadIdx.x == 0)
+        {
+            prefix[n] = 0;
+            item_prefix[n] = 0;
+        }
+        return;
+    }
+    // both sums in one scan: tiles in the upper half, items (fewer than 2^31) in the lower
+    scan_tables(
+            n,
+            [&](int64_t t) -> long long {
+                const uint8_t mark = alone ? build[t] : __ldcg(build + t);
+                const long long regions = mark != 0 ? first_item[t + 1] - first_item[t] : 0;
+                return (regions > 1 ? tiles_of(offsets, t, tile) << 32 : 0) + regions;
+            },
+            [&](int64_t t, long long x) {
+                prefix[t] = x >> 32;
+                item_prefix[t] = x & 0xffffffffll;
+            });
 }
 
-// Second launch: the keys of the tables that are built and have several regions, appended to the lists in their
-// regions' slots.
+// Second launch: the items that are built in `order` (nullable: the build looks at every item), and the keys of the
+// tables that are built and have several regions, appended to the lists in their regions' slots.
 template <int KIND, bool AOS>
 __global__ void __launch_bounds__(kListThreads, 3)
 k_batch_lists(const dview* views, const int64_t* offsets, const int64_t* prefix, int32_t n, const int32_t* first_item,
-              unsigned int* fill, uint8_t* todo, const void* in0, const void* in1)
+              const build_item* items, int32_t n_items, const uint8_t* build, const int64_t* item_prefix,
+              build_item* order, unsigned int* fill, uint8_t* todo, const void* in0, const void* in1)
 {
     wait_for_stream();
+    if (order != nullptr && item_prefix[n] == 0)
+    {
+        return;
+    }
+    for (int32_t i = order != nullptr ? blockIdx.x * kListThreads + threadIdx.x : n_items; i < n_items;
+         i += gridDim.x * kListThreads)
+    {
+        const build_item it = items[i];
+        if (build[it.table] != 0)
+        {
+            order[item_prefix[it.table] + i - first_item[it.table]] = it;
+        }
+    }
     using C = kind_consts<KIND>;
     using E = typename slot_image<KIND>::type;
     constexpr int PER = kListPer;
@@ -261,14 +346,18 @@ k_batch_lists(const dview* views, const int64_t* offsets, const int64_t* prefix,
     }
 }
 
-// Third launch: one region per block.  Spilled keys go to the probe kernel one by one.  A table some of whose keys
-// found no room in a list is marked todo: the probe kernel then runs over all its keys, which changes nothing for
-// those stored here.
-template <int KIND, bool AOS>
+// Third launch: the items that are built, one region at a time per block.  A batch of more items than blocks that are
+// resident at once (ORDERED) gives the built ones in `items`, `built` of them, and the blocks take the next one from a counter: a
+// block for each of its regions, built or not, made an insert of 3 keys each into 4096 cleared tables of 8192 take
+// 46 us, 26 so.  Else each item has its block, which looks whether it is built: two reads less to
+// wait for, 13.2 us against 14.2 for 697 tables of 817 regions.  Spilled keys go to the probe kernel one by one.  A table
+// some of whose keys found no room in a list is marked todo: the probe kernel then runs over all its keys, which
+// changes nothing for those stored here.
+template <int KIND, bool AOS, bool ORDERED>
 __global__ void __launch_bounds__(kRegionThreads, kRegionBlocks)
-k_batch_build(const dview* views, const int64_t* offsets, const build_item* items, const uint8_t* build,
-              const unsigned int* fill, uint8_t* todo, const void* in0, const void* in1, uint8_t* out_flags,
-              spill_list spills)
+k_batch_build(const dview* views, const int64_t* offsets, const build_item* items, const int64_t* built,
+              const uint8_t* build, unsigned int* next, const unsigned int* fill, uint8_t* todo, const void* in0,
+              const void* in1, uint8_t* out_flags, spill_list spills)
 {
     wait_for_stream();
     using C = kind_consts<KIND>;
@@ -276,82 +365,93 @@ k_batch_build(const dview* views, const int64_t* offsets, const build_item* item
     using V = typename C::V;
     using E = typename slot_image<KIND>::type;
     extern __shared__ __align__(128) unsigned char smem[];
-    const build_item it = items[blockIdx.x];
-    const dview t = views[it.table];
-    const int64_t lo = offsets[it.table], hi = offsets[it.table + 1];
-    const unsigned int listed = fill[blockIdx.x];
-    if (build[it.table] == 0)
+    __shared__ unsigned int s_next;
+    const int64_t n_built = ORDERED ? *built : gridDim.x;
+    for (int64_t w = blockIdx.x; w < n_built; w = ORDERED ? s_next : n_built)
     {
-        return;
-    }
-    const region r{ reinterpret_cast<char*>(smem), it.first, it.count, it.whole != 0 };
-    region_start<KIND>(t, r);
-    __syncthreads();
-    const E* const list = reinterpret_cast<const E*>(t.slots + (static_cast<uint64_t>(it.first) << 7));
-    const int64_t count = it.whole != 0 ? hi - lo
-                                        : static_cast<int64_t>(min(listed, it.count * C::slots_per_group));
-    unsigned int done = 0, refused = 0;
-    constexpr int kAhead = 4; // keys loaded before any is inserted
-    for (int64_t base = threadIdx.x; base < count; base += kAhead * kRegionThreads)
-    {
-        K key[kAhead];
-        V val[kAhead];
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j)
+        const build_item it = items[w];
+        const bool whole = it.list < 0;
+        const dview t = views[it.table];
+        const int64_t lo = offsets[it.table], hi = offsets[it.table + 1];
+        const unsigned int listed = whole ? 0u : fill[it.list];
+        if (!ORDERED && build[it.table] == 0)
         {
-            const int64_t i = base + j * kRegionThreads;
-            if (i < count)
+            return;
+        }
+        const region r{ reinterpret_cast<char*>(smem), it.first, it.count, whole };
+        region_start<KIND>(t, r);
+        __syncthreads();
+        if (ORDERED && threadIdx.x == 0)
+        {
+            s_next = gridDim.x + atomicAdd(next, 1u); // there by the time the region is built
+        }
+        const E* const list = reinterpret_cast<const E*>(t.slots + (static_cast<uint64_t>(it.first) << 7));
+        const int64_t count = whole ? hi - lo
+                                            : static_cast<int64_t>(min(listed, it.count * C::slots_per_group));
+        unsigned int done = 0, refused = 0;
+        constexpr int kAhead = 4; // keys loaded before any is inserted
+        for (int64_t base = threadIdx.x; base < count; base += kAhead * kRegionThreads)
+        {
+            K key[kAhead];
+            V val[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
             {
-                if (it.whole != 0)
+                const int64_t i = base + j * kRegionThreads;
+                if (i < count)
                 {
-                    load_input<KIND, AOS>(in0, in1, lo + i, key[j], val[j]);
+                    if (whole)
+                    {
+                        load_input<KIND, AOS>(in0, in1, lo + i, key[j], val[j]);
+                    }
+                    else
+                    {
+                        unpack_element<KIND>(__ldcg(list + i), key[j], val[j]);
+                    }
                 }
-                else
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
+            {
+                const int64_t i = base + j * kRegionThreads;
+                if (i >= count)
                 {
-                    unpack_element<KIND>(__ldcg(list + i), key[j], val[j]);
+                    break;
+                }
+                const int res = key[j] >= C::tomb_key
+                                        ? special_insert<KIND>(t, key[j], val[j])
+                                        : region_insert<KIND>(r, home_of<KIND>(t, key[j]) - it.first,
+                                                              rot_of(static_cast<uint64_t>(key[j])), key[j], val[j]);
+                done += (res == kRegionInserted);
+                refused += (res == kRegionRefused);
+                if (res == kRegionSpill)
+                {
+                    const unsigned int k = atomicAdd(spills.count, 1u);
+                    if (k < kSpillMax)
+                    {
+                        spill_entry x{};
+                        *reinterpret_cast<E*>(&x.image) = pack_element<KIND>(key[j], val[j]);
+                        x.table = it.table;
+                        spills.entry[k] = x;
+                    }
+                    else
+                    {
+                        todo[it.table] = 1;
+                    }
+                }
+                if (out_flags != nullptr)
+                {
+                    out_flags[lo + i] = static_cast<uint8_t>(res == kRegionInserted);
                 }
             }
         }
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j)
-        {
-            const int64_t i = base + j * kRegionThreads;
-            if (i >= count)
-            {
-                break;
-            }
-            const int res = key[j] >= C::tomb_key
-                                    ? special_insert<KIND>(t, key[j], val[j])
-                                    : region_insert<KIND>(r, home_of<KIND>(t, key[j]) - it.first,
-                                                          rot_of(static_cast<uint64_t>(key[j])), key[j], val[j]);
-            done += (res == kRegionInserted);
-            refused += (res == kRegionRefused);
-            if (res == kRegionSpill)
-            {
-                const unsigned int k = atomicAdd(spills.count, 1u);
-                if (k < kSpillMax)
-                {
-                    spill_entry x{};
-                    *reinterpret_cast<E*>(&x.image) = pack_element<KIND>(key[j], val[j]);
-                    x.table = it.table;
-                    spills.entry[k] = x;
-                }
-                else
-                {
-                    todo[it.table] = 1;
-                }
-            }
-            if (out_flags != nullptr)
-            {
-                out_flags[lo + i] = static_cast<uint8_t>(res == kRegionInserted);
-            }
-        }
+        __syncthreads(); // the list, which lies in the region's slots, is read
+        region_write(t, r);
+        unsigned int c[2] = { done, refused };
+        unsigned long long* const dst[2] = { &t.hdr->size, &t.hdr->refused };
+        region_add<2>(c, dst);
+        __syncthreads(); // the region is written out, and the next item is there
     }
-    __syncthreads(); // the list, which lies in the region's slots, is read
-    region_write(t, r);
-    unsigned int c[2] = { done, refused };
-    unsigned long long* const dst[2] = { &t.hdr->size, &t.hdr->refused };
-    region_add<2>(c, dst);
 }
 
 enum batch_op : int
@@ -546,11 +646,24 @@ struct sg_table_batch
     int64_t n_items;
     int32_t* first_item;     // device, n + 1
     uint8_t* marks;          // device, 2 n
-    unsigned int* fill;      // device, n_items
+    build_item* order;       // device, n_items: a call's items that are built
+    unsigned int* fill;      // device, n_items, and the build_words behind them
     int64_t* list_prefix;    // device, n + 1
     spill_list spills;       // device
     bool maybe_empty;        // cleared or created since the last insert: tries the build (the device decides per table)
 };
+
+size_t
+fill_bytes(int64_t n_items)
+{
+    return sizeof(unsigned int) * static_cast<size_t>(n_items) + sizeof(build_words);
+}
+
+build_words*
+words_of(unsigned int* fill, int64_t n_items)
+{
+    return reinterpret_cast<build_words*>(fill + n_items);
+}
 
 constexpr int64_t kBatchInsertLocks = int64_t{ 1 } << 16;
 
@@ -629,24 +742,46 @@ struct batch_launch
           cudaStream_t s)
     {
         using Lists = list_tile<typename slot_image<KIND>::type, kListPer>;
+        // once: a call to set an attribute takes a microsecond of the host's time
+        static const cudaError_t shared_set = [] {
+            constexpr cudaFuncAttribute kShared = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            cudaError_t e = cudaFuncSetAttribute(k_batch_lists<KIND, AOS>, kShared, static_cast<int>(sizeof(Lists)));
+            e = e != cudaSuccess ? e
+                                 : cudaFuncSetAttribute(k_batch_build<KIND, AOS, true>, kShared,
+                                                        static_cast<int>(kRegionBytes));
+            return e != cudaSuccess ? e
+                                    : cudaFuncSetAttribute(k_batch_build<KIND, AOS, false>, kShared,
+                                                           static_cast<int>(kRegionBytes));
+        }();
+        SG_CUDA_TRY(shared_set);
         uint8_t* const todo = b->marks + b->n;
-        // the lists' lengths, and the spill count behind them
-        SG_CUDA_TRY(cudaMemsetAsync(b->fill, 0, sizeof(unsigned int) * static_cast<size_t>(b->n_items + 1), s));
-        SG_CUDA_TRY(launch_early(k_batch_choose, 1, 1024, s, b->views, offsets, b->n, b->first_item,
+        build_words* const words = words_of(b->fill, b->n_items);
+        SG_CUDA_TRY(cudaMemsetAsync(b->fill, 0, fill_bytes(b->n_items), s));
+        SG_CUDA_TRY(launch_early(k_batch_choose, grid_for(b->n, 1024, b->sms), 1024, s, b->views, offsets, b->n, b->first_item,
                                  out_flags != nullptr, kListPer * kListThreads, b->sms * kRegionBlocks, b->marks, todo,
-                                 b->list_prefix));
+                                 b->list_prefix, b->prefix, words));
         SG_LAUNCH_CHECK();
-        SG_CUDA_TRY(cudaFuncSetAttribute(k_batch_lists<KIND, AOS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(sizeof(Lists))));
         static const int lists_grid = persistent_grid(k_batch_lists<KIND, AOS>, kListThreads, sizeof(Lists));
+        static const int build_grid =
+                persistent_grid(k_batch_build<KIND, AOS, true>, kRegionThreads, kRegionBytes);
+        const bool ordered = b->n_items > build_grid;
         SG_CUDA_TRY(launch_early_shared(k_batch_lists<KIND, AOS>, lists_grid, kListThreads, sizeof(Lists), s, b->views,
-                                        offsets, b->list_prefix, b->n, b->first_item, b->fill, todo, in0, in1));
+                                        offsets, b->list_prefix, b->n, b->first_item, b->items,
+                                        static_cast<int32_t>(b->n_items), b->marks, b->prefix,
+                                        ordered ? b->order : nullptr, b->fill, todo, in0, in1));
         SG_LAUNCH_CHECK();
-        SG_CUDA_TRY(cudaFuncSetAttribute(k_batch_build<KIND, AOS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(kRegionBytes)));
-        SG_CUDA_TRY(launch_early_shared(k_batch_build<KIND, AOS>, static_cast<unsigned>(b->n_items), kRegionThreads,
-                                        kRegionBytes, s, b->views, offsets, b->items, b->marks, b->fill, todo, in0, in1,
-                                        out_flags, b->spills));
+        if (ordered)
+        {
+            SG_CUDA_TRY(launch_early_shared(k_batch_build<KIND, AOS, true>, build_grid, kRegionThreads, kRegionBytes, s,
+                                            b->views, offsets, b->order, b->prefix + b->n, b->marks, &words->taken,
+                                            b->fill, todo, in0, in1, out_flags, b->spills));
+        }
+        else
+        {
+            SG_CUDA_TRY(launch_early_shared(k_batch_build<KIND, AOS, false>, static_cast<int>(b->n_items),
+                                            kRegionThreads, kRegionBytes, s, b->views, offsets, b->items, nullptr,
+                                            b->marks, nullptr, b->fill, todo, in0, in1, out_flags, b->spills));
+        }
         SG_LAUNCH_CHECK();
         return SG_OK;
     }
@@ -822,7 +957,7 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
             const int64_t g = k * kRegionGroups;
             items.push_back(build_item{ t, static_cast<uint32_t>(g),
                                         static_cast<uint32_t>(std::min<int64_t>(groups[t] - g, kRegionGroups)),
-                                        regions == 1 ? 1 : 0 });
+                                        regions == 1 ? -1 : static_cast<int32_t>(items.size()) });
         }
         first_item[t + 1] = static_cast<int32_t>(items.size());
     }
@@ -858,8 +993,12 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
     }
     if (e == cudaSuccess && !items.empty())
     {
-        e = sg::detail::dev_malloc(&b->fill, sizeof(unsigned int) * (items.size() + 1));
-        b->spills.count = b->fill + items.size();
+        e = sg::detail::dev_malloc(&b->fill, fill_bytes(b->n_items));
+        b->spills.count = &words_of(b->fill, b->n_items)->spilled;
+    }
+    if (e == cudaSuccess && !items.empty())
+    {
+        e = sg::detail::dev_malloc(&b->order, sizeof(build_item) * items.size());
     }
     if (e == cudaSuccess && !items.empty())
     {
@@ -940,6 +1079,7 @@ sg_batch_destroy(sg_table_batch* b)
     sg::detail::dev_free(b->locks);
     sg::detail::dev_free(b->items);
     sg::detail::dev_free(b->fill);
+    sg::detail::dev_free(b->order);
     sg::detail::dev_free(b->spills.entry);
     sg::detail::dev_free(b->first_item);
     sg::detail::dev_free(b->list_prefix);

@@ -227,3 +227,16 @@ def test_many_copies_for_few_small_tables_are_not_left_to_one_block_each(tables)
     again = _microseconds(lambda: b.insert(keys, off), lambda: None)
     sg.table_batch.destroyDeviceObjects(b)
     assert first < 5 * again + 50, (first, again)
+
+
+def test_a_first_insert_that_builds_nothing_costs_little_more_than_the_next():
+    """Three keys into each of very many cleared tables: deciding that none is built is a small part of the call."""
+    tables = 1 << 16
+    keys = torch.arange(1, 3 * tables + 1, device="cuda")
+    off = torch.arange(tables + 1, dtype=torch.int64, device="cuda") * 3
+    b = sg.table_batch.createDeviceObjects([2100] * tables, key="u64")
+    first = _microseconds(lambda: b.insert(keys, off), b.clear)
+    assert (b.sizes() == 3).all()
+    again = _microseconds(lambda: b.insert(keys, off), lambda: None)
+    sg.table_batch.destroyDeviceObjects(b)
+    assert first < 1.9 * again, (first, again)
