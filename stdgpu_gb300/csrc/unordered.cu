@@ -53,7 +53,7 @@ struct accounting_init
 };
 
 // Words of a counted bulk insert (k_counted_*), in the 256 bytes that the device header is given of its own,
-// behind its fields.  All zero between calls.
+// behind its fields.  All zero between calls (sg_unordered::counted_open: after a call that broke off they are not).
 struct counted_control
 {
     unsigned long long absent; // keys of the call that are not stored
@@ -1696,6 +1696,7 @@ struct sg_unordered
     uint32_t* bucket_heads;        // the reference's excess-list accounting (sg_unordered_view), nullptr: off
     uint32_t* slot_heads;
     uint32_t* bucket_cand;         // a bulk insert's candidate per bucket (k_counted_candidates)
+    bool counted_open;             // a counted insert's first launch was queued, its last one (k_counted_reset) not
     char* heads_block;             // their own block when switched on after creation, else nullptr (in `block`)
     char* call_scratch;            // sg_unordered_call_scratch: the caller-side staging of the C++ API's bulk calls
     int64_t call_scratch_bytes;
@@ -1972,6 +1973,16 @@ use_partitioned_erase(const sg_unordered* t, int64_t n, const uint8_t* flags)
 }
 
 // Bulk insert of a table with the accounting on: candidates, the inserts, candidates reset.
+// What a counted insert keeps between its launches as it is between calls: no candidates, the control words zero.
+cudaError_t
+reset_counted_call(sg_unordered* t, cudaStream_t s)
+{
+    const cudaError_t e = cudaMemsetAsync(t->bucket_cand, 0xFF, bucket_cand_bytes(t->bucket_count), s);
+    return e != cudaSuccess ? e
+                            : cudaMemsetAsync(reinterpret_cast<char*>(t->hdr) + kCountedControlOffset, 0,
+                                              sizeof(counted_control), s);
+}
+
 template <int KIND, bool AOS>
 sg_status
 insert_counted(sg_unordered* t, const void* in0, const void* in1, int64_t n, uint8_t* flags, cudaStream_t s,
@@ -1983,6 +1994,12 @@ insert_counted(sg_unordered* t, const void* in0, const void* in1, int64_t n, uin
     }
     const dview d = view_of(t);
     const sg_unordered_view v = public_view(t);
+    if (t->counted_open)
+    {
+        // a launch of an earlier call was refused: its candidates and bounds are still there
+        SG_CUDA_TRY(reset_counted_call(t, s));
+        t->counted_open = false;
+    }
     if (n <= kCountedClusterMax)
     {
         int blocks = 1;
@@ -2011,6 +2028,7 @@ insert_counted(sg_unordered* t, const void* in0, const void* in1, int64_t n, uin
     static const int g_cand = persistent_grid(k_counted_candidates<KIND, AOS>, kThreads);
     static const int g_ins = persistent_grid(k_insert_counted<KIND, AOS>, kThreads);
     static const int g_reset = persistent_grid(k_counted_reset<KIND, AOS>, kThreads);
+    t->counted_open = true;
     SG_CUDA_TRY(launch_early(k_counted_candidates<KIND, AOS>, grid_for(n, kThreads, g_cand), kThreads, s, d, v, in0,
                              in1, n, hashes, t->bucket_cand));
     SG_LAUNCH_CHECK();
@@ -2020,6 +2038,7 @@ insert_counted(sg_unordered* t, const void* in0, const void* in1, int64_t n, uin
     SG_CUDA_TRY(launch_early(k_counted_reset<KIND, AOS>, grid_for(n, kThreads, g_reset), kThreads, s, d, v, in0, in1, n,
                              hashes, t->bucket_cand));
     SG_LAUNCH_CHECK();
+    t->counted_open = false;
     return SG_OK;
 }
 
@@ -2375,9 +2394,8 @@ reset_accounting(sg_unordered* t, cudaStream_t s)
     }
     SG_CUDA_TRY(cudaMemsetAsync(t->bucket_heads, 0, bucket_heads_bytes(t->bucket_count), s));
     SG_CUDA_TRY(cudaMemsetAsync(t->slot_heads, 0, slot_heads_bytes(t->num_groups, t->slot_bytes), s));
-    SG_CUDA_TRY(cudaMemsetAsync(t->bucket_cand, 0xFF, bucket_cand_bytes(t->bucket_count), s));
     SG_CUDA_TRY(cudaMemsetAsync(&t->hdr->excess_used, 0, sizeof(unsigned long long), s));
-    SG_CUDA_TRY(cudaMemsetAsync(reinterpret_cast<char*>(t->hdr) + kCountedControlOffset, 0, sizeof(counted_control), s));
+    SG_CUDA_TRY(reset_counted_call(t, s));
     return SG_OK;
 }
 
