@@ -346,7 +346,8 @@ reserve(long long* counter, long long bound, long long want, bool grow)
 #define SG_DEQUE_FAST 1
 #endif
 
-// What a mixed call does, settled on the device by k_deque_plan; behind the sync words of the device calls.
+// What a mixed call does, settled on the device by k_deque_plan; behind the sync words of the device calls.  pushes
+// and arrived are 0 between calls.
 struct deque_control
 {
     unsigned long long pushes;  // of the call
@@ -377,11 +378,12 @@ static_assert(kPlanTile == kTileElems, "one count per tile of the move");
 // block into the pushes before each tile; that block then settles the call.  The order it stands for runs pushes
 // while there is room and pops while there are elements, in turn, so a push fails only where the deque ends full and
 // a pop only where it ends empty; pushes take the tickets from `end` on and pops those from `begin` on, in element
-// order, and the counters are moved here.  The launches that follow need neither turn words nor reservations.
+// order.  The launches that follow need neither turn words nor reservations; the last one moves the counters, so a
+// call that breaks off between its launches leaves the deque as it was.
 // counts: room for a word per tile (the turn words' array, which is marked dirty).
 __global__ void __launch_bounds__(kCThreads)
-k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters* c, int64_t cap, sg_deque_sync* sync,
-             uint32_t epoch, deque_control* ctl)
+k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, const deque_counters* c, int64_t cap,
+             sg_deque_sync* sync, deque_control* ctl)
 {
     wait_for_stream();
     __shared__ unsigned long long s_block;
@@ -502,11 +504,7 @@ k_deque_plan(const uint8_t* is_push, int64_t n, unsigned* counts, deque_counters
         ctl->push_t0 = c->end;
         ctl->pop_t0 = c->begin;
         ctl->apart = push_ok <= room && pop_ok <= held ? 1u : 0u;
-        c->end += static_cast<unsigned long long>(push_ok);
-        c->begin += static_cast<unsigned long long>(pop_ok);
-        c->size += push_ok - pop_ok;
-        c->avail += push_ok - pop_ok;
-        deque_call_ends(c, sync, epoch, 1u);
+        sync->dirty = 1u; // the counts lie where the turn words were
     }
 }
 
@@ -565,9 +563,19 @@ enum move_phase : int
 template <typename T, int PHASE>
 __global__ void __launch_bounds__(kCThreads, 8)
 k_deque_move(T* data, const unsigned* before, unsigned ucap, const uint8_t* is_push, const T* values, unsigned n,
-             T* out_popped, uint8_t* out_ok, bool zero_rest, const deque_control* ctl)
+             T* out_popped, uint8_t* out_ok, bool zero_rest, const deque_control* ctl, deque_counters* c,
+             sg_deque_sync* sync, uint32_t epoch)
 {
     wait_for_stream();
+    if (PHASE == kMoveLate && blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        // nothing of the call reads the counters any more
+        c->end += static_cast<unsigned long long>(ctl->push_ok);
+        c->begin += static_cast<unsigned long long>(ctl->pop_ok);
+        c->size += ctl->push_ok - ctl->pop_ok;
+        c->avail += ctl->push_ok - ctl->pop_ok;
+        deque_call_ends(c, sync, epoch, 1u);
+    }
     const bool apart = ctl->apart != 0u;
     if (PHASE != kMoveFirst && apart)
     {
@@ -1444,7 +1452,7 @@ deque_mixed(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, 
     const int64_t tiles = (n + kPlanTile - 1) / kPlanTile;
     static const int mp = persistent_grid(k_deque_plan, kCThreads);
     SG_CUDA_TRY(launch_early(k_deque_plan, grid_for(tiles, kWarps, mp), kCThreads, s, is_push, n, d->seq, d->counters,
-                             d->capacity, d->sync, d->epoch, control_of(d)));
+                             d->capacity, d->sync, control_of(d)));
     SG_LAUNCH_CHECK();
     // at most `capacity` elements, below 2^31: 32-bit ranks
     const unsigned ucap = static_cast<unsigned>(d->capacity);
@@ -1453,13 +1461,13 @@ deque_mixed(sg_deque* d, const uint8_t* is_push, const void* values, int64_t n, 
     static const int m1 = persistent_grid(k_deque_move<T, kMovePush>, kCThreads);
     static const int m2 = persistent_grid(k_deque_move<T, kMoveLate>, kCThreads);
     SG_CUDA_TRY(launch_early(k_deque_move<T, kMoveFirst>, grid_for(tiles, 1, m0), kCThreads, s, data, d->seq, ucap,
-                             is_push, in, un, out, out_ok, zero_rest, control_of(d)));
+                             is_push, in, un, out, out_ok, zero_rest, control_of(d), d->counters, d->sync, d->epoch));
     SG_LAUNCH_CHECK();
     SG_CUDA_TRY(launch_early(k_deque_move<T, kMovePush>, grid_for(tiles, 1, m1), kCThreads, s, data, d->seq, ucap,
-                             is_push, in, un, out, out_ok, zero_rest, control_of(d)));
+                             is_push, in, un, out, out_ok, zero_rest, control_of(d), d->counters, d->sync, d->epoch));
     SG_LAUNCH_CHECK();
     SG_CUDA_TRY(launch_early(k_deque_move<T, kMoveLate>, grid_for(tiles, 1, m2), kCThreads, s, data, d->seq, ucap,
-                             is_push, in, un, out, out_ok, zero_rest, control_of(d)));
+                             is_push, in, un, out, out_ok, zero_rest, control_of(d), d->counters, d->sync, d->epoch));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }

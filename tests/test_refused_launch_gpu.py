@@ -74,3 +74,32 @@ for at in (0, 1, 2):
     a.insert(keys(300000, 100))     # a call of one launch
     assert a.size() == b.size() + 100
 ''')
+
+
+def test_mixed_deque_call_that_broke_off_leaves_the_deque_as_it_was():
+    """A ring too large for turn words, whose mixed calls are a plan and three moves: with any of the four refused the
+    counters are as before the call, and the elements are there in order."""
+    _run(r'''
+cap, n = (1 << 17) + 5, 50000
+d = sg.deque.createDeviceObject(cap, elem_bytes=8)
+first = torch.arange(1, 30001, device="cuda")
+some = torch.arange(n, device="cuda").remainder(3).eq(0).to(torch.uint8)  # more pops than pushes
+for kind in (some, 1 - some):
+    for at in (0, 1, 2, 3):
+        d.clear()
+        d.push_back(first)
+        assert refused(at, lambda: d.ops(kind, torch.arange(n, device="cuda")))
+        assert d.size() == 30000
+        vals, ok = d.pop_front(30001)
+        assert torch.equal(vals[:30000], first) and int(ok.sum()) == 30000 and d.size() == 0
+        d.push_back(first)
+        popped, done = d.ops(kind, torch.arange(n, device="cuda") + 10 ** 6)
+        pushes, pops = int(kind.sum()), n - int(kind.sum())
+        assert d.size() == max(0, 30000 + pushes - pops)
+        # more elements than slots, by turn words, which the plan's counts have lain over
+        d.clear()
+        big = torch.ones(cap + 100, dtype=torch.uint8, device="cuda")
+        big[: 60] = 0
+        popped, done = d.ops(big, torch.arange(cap + 100, device="cuda"))
+        assert d.size() <= cap and d.size() >= cap - 60
+''')
