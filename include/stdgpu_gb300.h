@@ -326,7 +326,8 @@ SG_API sg_status sg_unordered_contains_host(sg_unordered* table, sg_stager* stag
  * offsets[t+1]) of the input (offsets: DEVICE array of n_tables + 1 int64), and runs as one
  * persistent launch over (table, 32-key range) tiles.  A NULL key array (all ranges empty, as an empty
  * tensor gives) walks no tile.  No host work depends on the sizes, so a sequence of batched calls can be
- * captured in a CUDA graph. */
+ * captured in a CUDA graph.  An insert that the CUDA runtime refuses half way (SG_ERR_CUDA) can leave tables
+ * that were empty without their keys in place: inserts, erases and lookups return SG_ERR_CUDA until clear(). */
 typedef struct sg_table_batch sg_table_batch;
 
 /* capacities: HOST array of n_tables capacities (createDeviceObject(capacity) of each table). */

@@ -652,6 +652,7 @@ struct sg_table_batch
     unsigned int* fill;      // device, n_items, and the build_words behind them
     int64_t* list_prefix;    // device, n + 1
     spill_list spills;       // device
+    bool torn;               // lists were queued into tables' slots, but the launch that builds from them was refused
     bool maybe_empty;        // cleared or created since the last insert: tries the build (the device decides per table)
 };
 
@@ -771,6 +772,7 @@ struct batch_launch
                                         offsets, b->list_prefix, b->n, b->first_item, b->items,
                                         static_cast<int32_t>(b->n_items), b->marks, b->prefix,
                                         ordered ? b->order : nullptr, b->fill, todo, in0, in1));
+        b->torn = true;
         SG_LAUNCH_CHECK();
         if (ordered)
         {
@@ -785,6 +787,7 @@ struct batch_launch
                                             b->marks, nullptr, b->fill, todo, in0, in1, out_flags, b->spills));
         }
         SG_LAUNCH_CHECK();
+        b->torn = false;
         return SG_OK;
     }
 
@@ -834,6 +837,10 @@ sg_status
 dispatch_op(sg_table_batch* b, int op, const int64_t* offsets, const void* in0, const void* in1, void* out_vals,
             uint8_t* out_flags, cudaStream_t s)
 {
+    if (b->torn)
+    {
+        return SG_ERR_CUDA; // until clear()
+    }
     const bool insert = op == kOpInsertAos || op == kOpInsertSoa;
     const bool build = insert && b->maybe_empty && in0 != nullptr && b->n_items > 0;
     if (insert && in0 != nullptr)
@@ -1116,6 +1123,7 @@ sg_batch_clear(sg_table_batch* b, void* stream)
     }
     const sg_status st = dispatch_init(b, as_stream(stream));
     b->maybe_empty = b->maybe_empty || st == SG_OK;
+    b->torn = b->torn && st != SG_OK;
     return st;
 }
 

@@ -103,3 +103,29 @@ for kind in (some, 1 - some):
         popped, done = d.ops(big, torch.arange(cap + 100, device="cuda"))
         assert d.size() <= cap and d.size() >= cap - 60
 ''')
+
+
+def test_batched_insert_that_broke_off_is_not_taken_for_tables():
+    """Tables of several regions, whose keys are listed in their own slots before they are built: with the launch that
+    builds them refused the batch answers nothing until clear(); with another one refused it goes on."""
+    _run(r'''
+tables, per = 5, 5000
+k = keys(0, tables * per)
+off = torch.arange(tables + 1, dtype=torch.int64, device="cuda") * per
+b = sg.table_batch.createDeviceObjects([10000] * tables, key="u64")
+for at in (0, 1, 2, 3, 4):  # choose, lists, build, tiles, walk
+    b.clear()
+    assert refused(at, lambda: b.insert(k, off))
+    if at == 2:
+        for call in (lambda: b.contains(k, off), lambda: b.find(k, off), lambda: b.insert(k, off),
+                     lambda: b.erase(k, off)):
+            try:
+                call()
+                raise SystemExit("answered")
+            except N.StdgpuError as e:
+                assert e.status == N.SG_ERR_CUDA
+        b.clear()
+    b.insert(k, off)
+    assert b.sizes().tolist() == [per] * tables and bool(b.contains(k, off).all())
+    assert not bool(b.contains(k + 1, off).any())
+''')
