@@ -452,7 +452,10 @@ SG_API sg_status sg_server_table_size(sg_server* server, int32_t table, int64_t*
 /* Waits for the table's requests (and a grow in flight), then its device view. */
 SG_API sg_status sg_server_table_view(sg_server* server, int32_t table, sg_unordered_view* out);
 
-/* ---------------- vector<T> (T = 4 or 8 bytes) ---------------- */
+/* ---------------- vector<T> (T = 4 or 8 bytes) ----------------
+ * Calls that change a vector or a deque act on the device in the order in which the host makes them, whatever
+ * streams they are given: a call on another stream than the last one waits for it.  (Calls under stream capture
+ * are left to the order of the graphs they go into.) */
 
 typedef struct sg_vector sg_vector;
 
