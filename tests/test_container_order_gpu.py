@@ -96,3 +96,97 @@ def test_deque_calls_on_two_streams_act_in_call_order(cap, n, hold):
     torch.cuda.synchronize()
     assert d.size() == n
     sg.deque.destroyDeviceObject(d)
+
+
+@pytest.mark.parametrize("cap", [5000, 1 << 18])
+def test_container_calls_captured_and_made_eagerly_in_turn(cap):
+    """A graph of vector and deque calls replayed between calls made on the stream."""
+    n = cap // 4
+    v = sg.vector.createDeviceObject(cap, elem_bytes=8)
+    d = sg.deque.createDeviceObject(cap, elem_bytes=8)
+    ids = torch.arange(1, n + 1, device="cuda")
+    buf = torch.zeros_like(ids)
+    mixed = torch.arange(n, device="cuda").remainder(2).to(torch.uint8)
+    out = torch.zeros((3, n), dtype=torch.int64, device="cuda")
+
+    def chain(s):
+        v.clear(stream=s)
+        d.clear(stream=s)
+        buf.copy_(ids)
+        v.push_back(buf, stream=s)
+        d.push_back(buf, stream=s)
+        buf.zero_()
+        out[0].copy_(v.pop_back(n, stream=s)[0])
+        buf.copy_(ids + n)
+        popped, _ = d.ops(mixed, buf, stream=s)
+        buf.zero_()
+        out[1].copy_(popped)
+        out[2].copy_(d.pop_front(n, stream=s)[0])
+
+    def check():
+        torch.cuda.synchronize()
+        pops = n - int(mixed.sum())
+        assert torch.equal(out[0].sort().values, ids)
+        assert torch.equal(out[1][mixed == 0].sort().values, ids[:pops])
+        want = torch.cat([ids[pops:], (ids + n)[mixed == 1]])
+        assert torch.equal(out[2].sort().values, want.sort().values)
+        assert v.size() == 0 and d.size() == 0
+
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        chain(s)
+    check()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        chain(torch.cuda.current_stream())
+    for _ in range(3):
+        out.zero_()
+        g.replay()
+        check()
+        v.push_back(ids)
+        d.push_back(ids)
+        torch.cuda.synchronize()
+        assert v.size() == n and d.size() == n
+    sg.vector.destroyDeviceObject(v)
+    sg.deque.destroyDeviceObject(d)
+
+
+@pytest.mark.parametrize("n", [300, 5000, 1 << 20])
+def test_early_kernels_behind_another_streams_work(n):
+    """Inputs written on another stream directly before an event that the call's stream waits for, with other early
+    calls queued on that stream before: the calls see the inputs."""
+    other, s = torch.cuda.Stream(), torch.cuda.Stream()
+    t = sg.unordered_set.createDeviceObject(2 * n, key="u64")
+    v = sg.vector.createDeviceObject(4 * n, elem_bytes=8)
+    d = sg.deque.createDeviceObject(4 * n, elem_bytes=8)
+    b = sg.table_batch.createDeviceObjects([4 * n] * 3, key="u64")
+    src = torch.arange(1, n + 1, device="cuda") * 0x9E3779B97F4A7C1
+    buf = torch.zeros_like(src)
+    off = torch.tensor([0, 0, n, n], device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(3):
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(1_000_000)
+            buf.copy_(src)
+        done = torch.cuda.Event()
+        done.record(other)
+        with torch.cuda.stream(s):
+            t.clear(stream=s)
+            v.clear(stream=s)
+            d.clear(stream=s)
+            b.clear(stream=s)
+            s.wait_event(done)
+            t.insert(buf, stream=s)
+            v.push_back(buf, stream=s)
+            d.push_back(buf, stream=s)
+            b.insert(buf, off, stream=s)
+            got = t.contains(src, stream=s), b.contains(src, off, stream=s), d.pop_front(n, stream=s)[0]
+            buf.zero_()
+        s.synchronize()
+        assert bool(got[0].all()) and bool(got[1].all()) and torch.equal(got[2], src)
+        assert t.size() == n and v.size() == n and b.sizes().tolist() == [0, n, 0]
+    sg.unordered_set.destroyDeviceObject(t)
+    sg.vector.destroyDeviceObject(v)
+    sg.deque.destroyDeviceObject(d)
+    sg.table_batch.destroyDeviceObjects(b)
