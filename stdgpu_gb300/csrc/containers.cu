@@ -1068,11 +1068,12 @@ k_vector_pop_back(const T* data, long long* size, int64_t cap, int64_t n, T* out
 
 // clear(), and the end of the calls that the host drives (insert, erase).
 __global__ void
-k_vector_call_ends(long long* size, int64_t cap, bool clear, sg_vector_sync* sync, uint32_t epoch)
+k_vector_call_ends(long long* size, int64_t cap, bool clear, sg_vector_sync* sync, uint32_t epoch, vector_control* ctl)
 {
     wait_for_stream();
     if (clear)
     {
+        *ctl = vector_control{}; // whatever launches that overlapped against the rules left there
         *size = 0;
     }
     vector_call_ends(size, cap, 0, sync, epoch);
@@ -1080,7 +1081,8 @@ k_vector_call_ends(long long* size, int64_t cap, bool clear, sg_vector_sync* syn
 
 // keep: the turn words too (slot i is free for ticket i, modulo 2^32)
 __global__ void
-k_deque_reset(unsigned* seq, deque_counters* c, int64_t cap, bool keep, sg_deque_sync* sync, uint32_t epoch)
+k_deque_reset(unsigned* seq, deque_counters* c, int64_t cap, bool keep, sg_deque_sync* sync, uint32_t epoch,
+              deque_control* ctl)
 {
     wait_for_stream();
     if (keep)
@@ -1103,6 +1105,7 @@ k_deque_reset(unsigned* seq, deque_counters* c, int64_t cap, bool keep, sg_deque
     c->end = static_cast<unsigned long long>(cap) << 32;
     c->error = 0;
     c->avail = 0;
+    *ctl = deque_control{};
     deque_call_ends(c, sync, epoch, keep ? 0u : 1u);
 }
 
@@ -1583,7 +1586,8 @@ vector_call_ends(sg_vector* v, bool clear, cudaStream_t s)
     {
         return st;
     }
-    SG_CUDA_TRY(launch_early(k_vector_call_ends, 1, 1, s, v->size, v->capacity, clear, v->sync, v->epoch));
+    SG_CUDA_TRY(launch_early(k_vector_call_ends, 1, 1, s, v->size, v->capacity, clear, v->sync, v->epoch,
+                             control_of(v)));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }
@@ -2025,7 +2029,7 @@ sg_deque_clear(sg_deque* d, void* stream)
     }
     const bool keep = d->capacity <= kTurnsKeptMax;
     SG_CUDA_TRY(launch_early(k_deque_reset, keep ? grid_for(d->capacity, kCThreads, 256) : 1, kCThreads, s, d->seq,
-                             d->counters, d->capacity, keep, d->sync, d->epoch));
+                             d->counters, d->capacity, keep, d->sync, d->epoch, control_of(d)));
     SG_LAUNCH_CHECK();
     return SG_OK;
 }

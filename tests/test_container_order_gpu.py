@@ -190,3 +190,34 @@ def test_early_kernels_behind_another_streams_work(n):
     sg.vector.destroyDeviceObject(v)
     sg.deque.destroyDeviceObject(d)
     sg.table_batch.destroyDeviceObjects(b)
+
+
+@pytest.mark.parametrize("cap", [4096, 1 << 18])
+def test_clear_makes_a_container_whole_whatever_its_launch_words_hold(cap):
+    """A graph replayed while a call runs on the same object can leave the count of arrived blocks behind, and then no
+    later call ends properly: clear() starts it anew.  Here the words are written from the host."""
+    import ctypes
+    from stdgpu_gb300 import _native as N
+    from stdgpu_gb300.containers import _DeviceArray
+    n = cap // 4
+    ids = torch.arange(1, n + 1, device="cuda")
+    v = sg.vector.createDeviceObject(n, elem_bytes=8)
+    d = sg.deque.createDeviceObject(cap, elem_bytes=8)
+    view, dview = N.sg_vector_view(), N.sg_deque_view()
+    N.check(N.load().sg_vector_view_of(v._h, ctypes.byref(view)), "view")
+    N.check(N.load().sg_deque_view_of(d._h, ctypes.byref(dview)), "view")
+    for sync in (view.sync, dview.sync):  # the words of the launches lie behind the device calls' own, at 64
+        torch.as_tensor(_DeviceArray(sync + 64, 16, 4), device="cuda").fill_(3)
+    torch.cuda.synchronize()
+    v.clear()
+    d.clear()
+    v.push_back(torch.cat([ids, ids]))
+    raw = torch.as_tensor(_DeviceArray(view.size, 1, 8), device="cuda")
+    assert int(raw[0].item()) == n  # clamped by the call's last block
+    vals, ok = v.pop_back(n)
+    assert bool(ok.all()) and v.size() == 0
+    d.push_back(ids)
+    d.ops(torch.ones(n, dtype=torch.uint8, device="cuda"), ids)
+    assert d.size() == 2 * n and torch.equal(d.pop_front(n)[0], ids)
+    sg.vector.destroyDeviceObject(v)
+    sg.deque.destroyDeviceObject(d)
