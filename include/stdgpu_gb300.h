@@ -264,7 +264,8 @@ SG_API sg_status sg_unordered_valid(sg_unordered* table, void* stream, int32_t* 
 
 /* device_range(): src/stdgpu/impl/unordered_base_detail.cuh:160-208.  Writes the slot indices of all
  * stored elements to out_slots (capacity >= max_size() + 2 entries) and their count to *out_n
- * (synchronises).  Element i of the range is ((value_type*)view.slots)[out_slots[i]]. */
+ * (synchronises).  Element i of the range is ((value_type*)view.slots)[out_slots[i]].  SG_ERR_RETRY_EXHAUSTED and
+ * a count of 0 if a device wait of this call gave up; what out_slots then holds is not the range. */
 SG_API sg_status sg_unordered_device_range(sg_unordered* table, int32_t* out_slots, void* stream, int64_t* out_n);
 
 /* Copy all stored keys (and mapped values for maps; nullable) out, in slot order.  *out_n gets the count. */

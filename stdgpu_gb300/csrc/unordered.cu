@@ -1404,7 +1404,7 @@ k_popc_words(const uint32_t* w, int64_t n, unsigned long long* out)
 // run of tiles (a tile: 1 or 2 KB of slots, read by a warp), shares it out to its warps, counts the live slots,
 // publishes the count, adds up the counts of the runs before its own, and goes through the run again to write.  Runs
 // are taken in order from a counter, so every count waited for is being made by a resident block; the wait is bounded
-// all the same.  The second time the tiles are read last to first: the ones read last are still in L2.  The last run
+// all the same: a block whose wait gives up writes nothing, and the call reports it.  The second time the tiles are read last to first: the ones read last are still in L2.  The last run
 // appends the out-of-band keys and leaves the total in hdr->count.
 // Bound by reading the slots, up to the size of L2 once, beyond it up to twice.  Calls with their read-back of the
 // count: 13.7 M slots of 16 bytes (219 MB), 3.1 M live, 96 us; 27 M slots of 8 bytes, 8.4 M live, 117 us; 219 M slots
@@ -1412,8 +1412,8 @@ k_popc_words(const uint32_t* w, int64_t n, unsigned long long* out)
 // launch for the out-of-band keys.  A single pass whose tiles look back at one another's counts took 156-207 us for
 // the first: its blocks run in lockstep and wait for one another every 32 KB.  Twice the slots per lane cost the
 // 8-byte case 30 %, 6 or 8 blocks per SM nothing or 5 %; keeping the masks of the first time gave nothing.
-constexpr unsigned int kErrRange = 16u; // a wait for an earlier run gave up (table header error bit)
-constexpr int kRangePolls = 1 << 20;
+constexpr unsigned int kErrRange = 16u; // this call's wait for an earlier run gave up (table header error bit)
+constexpr unsigned long long kRangeWaitNs = 1000000000ull; // 1 s, as the other waits of the library
 
 template <int KIND>
 struct range_tile
@@ -1436,11 +1436,18 @@ k_range(dview t, unsigned int* words, int runs, int64_t tiles, int32_t* out_slot
     constexpr int kWarpCount = kThreads / 32;
     __shared__ unsigned int s_run;
     __shared__ unsigned int s_warp[kWarpCount];
+    __shared__ bool s_gave_up;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0)
     {
         s_run = atomicAdd(words + runs, 1u);
+        s_gave_up = false;
+        if (s_run == 0u)
+        {
+            // the bit is the call's own: what an earlier one left goes before any run can wait for this one's count
+            atomicAnd(&t.hdr->error, ~kErrRange);
+        }
     }
     __syncthreads();
     const int run = static_cast<int>(s_run);
@@ -1497,10 +1504,10 @@ k_range(dview t, unsigned int* words, int runs, int64_t tiles, int32_t* out_slot
     for (int r = static_cast<int>(threadIdx.x); r < run; r += kThreads)
     {
         unsigned int v = 0u;
-        for (int polls = 0; polls < kRangePolls; ++polls)
+        for (const unsigned long long t0 = global_ns();;)
         {
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(words + r) : "memory");
-            if (v != 0u)
+            if (v != 0u || global_ns() - t0 > kRangeWaitNs)
             {
                 break;
             }
@@ -1509,6 +1516,7 @@ k_range(dview t, unsigned int* words, int runs, int64_t tiles, int32_t* out_slot
         if (v == 0u)
         {
             atomicOr(&t.hdr->error, kErrRange);
+            s_gave_up = true;
         }
         else
         {
@@ -1516,6 +1524,10 @@ k_range(dview t, unsigned int* words, int runs, int64_t tiles, int32_t* out_slot
         }
     }
     const unsigned int base = block_sum(earlier, unused);
+    if (s_gave_up) // set before the sum's barriers
+    {
+        return;
+    }
     // position behind the tiles not yet written
     unsigned int end = base + warps_before + live;
     for (int64_t tile = tile_hi - 1; tile >= tile_lo; --tile)
@@ -3050,8 +3062,9 @@ sg_unordered_device_range(sg_unordered* t, int32_t* out_slots, void* stream, int
     {
         return st;
     }
-    *out_n = static_cast<int64_t>(host_header(t).count);
-    return (host_header(t).error & kErrRange) != 0u ? SG_ERR_RETRY_EXHAUSTED : SG_OK;
+    const bool whole = (host_header(t).error & kErrRange) == 0u;
+    *out_n = whole ? static_cast<int64_t>(host_header(t).count) : 0;
+    return whole ? SG_OK : SG_ERR_RETRY_EXHAUSTED;
 }
 
 sg_status
@@ -3073,8 +3086,9 @@ sg_unordered_range_copy(sg_unordered* t, void* out_keys, void* out_mapped, void*
     {
         return st;
     }
-    *out_n = static_cast<int64_t>(host_header(t).count);
-    return (host_header(t).error & kErrRange) != 0u ? SG_ERR_RETRY_EXHAUSTED : SG_OK;
+    const bool whole = (host_header(t).error & kErrRange) == 0u;
+    *out_n = whole ? static_cast<int64_t>(host_header(t).count) : 0;
+    return whole ? SG_OK : SG_ERR_RETRY_EXHAUSTED;
 }
 
 sg_status
