@@ -28,8 +28,10 @@ KINDS = {("u32", None): N.SET_U32, ("u64", None): N.SET_U64, ("u64", "u32"): N.M
 
 # A call on a small table is bound by this module's own time: pointers and streams go to ctypes as plain integers
 # (a c_void_p object each cost 0.3 us), and the current stream's handle is read without the torch.cuda.Stream object
-# around it: a call on 700 keys 4.0 us of host time instead of 8, clear() 2.8 instead of 5.7.
-_raw_stream = torch._C._cuda_getCurrentRawStream
+# around it: a call on 700 keys 4.0 us of host time instead of 8, clear() 2.8 instead of 5.7.  (A torch without that
+# reader, which is not among its public names, gives the object.)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or \
+    (lambda device: torch.cuda.current_stream(device).cuda_stream)
 
 
 def _stream(stream) -> int:
