@@ -738,11 +738,11 @@ struct step_counts
 // ---------------------------------------------------------------- warp steps
 // One step covers 32 consecutive elements (lane l owns element i; valid when i is in range), all on
 // table t, and is called by all 32 lanes of the warp together.  Each tile of 4 lanes loads the home
-// groups of its 4 keys (4 x 128-byte requests per tile, 32 per warp).  Each group is then resolved
-// with full-warp ballots: nibble `tbase` of a ballot is the tile's view of its group (bit q = sector
-// q), so the common case -- the key's fate is decided in its home group -- runs without any branch
-// that differs between tiles.  Only keys whose home group is full of other keys (or whose claim lost
-// to another key) take the tile-cooperative slow path.
+// groups of its 4 keys (4 x 128-byte requests per tile, 32 per warp).  What each lane finds in its sector
+// of the four groups is then transposed within the tile (tile_transpose), so that each lane holds its own
+// key's whole group, and the common case -- the key's fate is decided in its home group -- runs without
+// any branch that differs between tiles.  Only keys whose home group is full of other keys (or whose claim
+// lost to another key) take the tile-cooperative slow path.
 
 // Ends a warp step: the lanes leave it together.  Without this barrier the lanes that lost a claim, or took the
 // slow path, left the step on their own and the compiler let them run into the next step's code in parts, up to
@@ -1114,6 +1114,7 @@ erase_key_step_deferred(const dview& t, const tile_lanes& L, typename kind_const
     {
         pend.old = cas_key<KIND>(t, static_cast<uint32_t>(my_slot), key, C::tomb_key);
     }
+    step_end();
 }
 
 template <int KIND>
