@@ -174,15 +174,18 @@ struct spill_list
 };
 
 // First launch of an insert into a batch that may be empty: build[t] = 1 for a table that holds nothing and gets at
-// least a key per two groups (a region is written whole, so fewer keys are cheaper to insert one by one) and not many more than it has slots; todo[t] = 1 for the others that get keys.  A table of several regions with more
-// keys than slots is left to the walk, since a list would overflow.  A table of one region is built by one block,
-// whatever copies its keys hold, while that block gets at most twice an even share of the call's keys among
-// `resident` blocks: 697 tables of 1000 with 5000 distinct keys each take 6680 us so, 9074 by the walk, and one table
-// of 1000 with 2^22 copies of 500 keys takes 127 us by the walk, 9270 by one block.  Tables of several regions get
-// lists (prefix: their tiles of `tile` elements; item_prefix: the regions of the tables before that are built), which
-// leave no room for an element's index: with per-key flags they go to the probe kernel.  The last block to finish adds
-// up the tables, unless none is built: 3 keys each into 65536 cleared tables of 2100 take 155 us, 520 when one block
-// did all of it and each region had its block, 244 with no table ever built.
+// least a key per group (a region is written whole, so fewer keys are cheaper to insert one by one) and not many more
+// than it has slots; todo[t] = 1 for the others that get keys.  4096 tables of 8192, built and walked: 142 and 105 us
+// at half a key per group, 152 and 150 at one, 179 and 257 at two; of 1000 (one region) 40 and 33, 40 and 49, 43 and
+// 70.  A table of several regions with more keys than slots is left to the walk, since a list would overflow.  A
+// table of one region is built by one block, whatever copies its keys hold, while that block gets at most twice an
+// even share of the call's keys among `resident` blocks: 697 tables of 1000 with 5000 distinct keys each take 6680 us
+// so, 9074 by the walk, and one table of 1000 with 2^22 copies of 500 keys takes 127 us by the walk, 9270 by one
+// block.  Tables of several regions get lists (prefix: their tiles of `tile` elements; item_prefix: the regions of
+// the tables before that are built), which leave no room for an element's index: with per-key flags they go to the
+// probe kernel.  The last block to finish adds up the tables, unless none is built: 3 keys each into 65536 cleared
+// tables of 2100 take 155 us, 520 when one block did all of it and each region had its block, 244 with no table ever
+// built.
 __global__ void __launch_bounds__(1024)
 k_batch_choose(const dview* views, const int64_t* offsets, int32_t n, const int32_t* first_item, bool flags, int tile,
                int resident, uint8_t* build, uint8_t* todo, int64_t* prefix, int64_t* item_prefix, build_words* words)
@@ -197,7 +200,7 @@ k_batch_choose(const dview* views, const int64_t* offsets, int32_t n, const int3
         const dview v = views[t];
         const int64_t cnt = offsets[t + 1] - offsets[t];
         const int32_t regions = first_item[t + 1] - first_item[t];
-        const bool ok = cnt > 0 && 2 * cnt >= v.num_groups &&
+        const bool ok = cnt >= v.num_groups &&
                         (cnt <= v.total || (regions == 1 && cnt * resident <= twice)) && regions > 0 &&
                         (regions == 1 || !flags) && v.hdr->size == 0 && v.hdr->tombstones == 0;
         build[t] = ok ? 1 : 0;
@@ -348,12 +351,12 @@ k_batch_lists(const dview* views, const int64_t* offsets, const int64_t* prefix,
 }
 
 // Third launch: the items that are built, one region at a time per block.  A batch of more items than blocks that are
-// resident at once (ORDERED) gives the built ones in `items`, `built` of them, and the blocks take the next one from a counter: a
-// block for each of its regions, built or not, made an insert of 3 keys each into 4096 cleared tables of 8192 take
-// 46 us, 26 so.  Else each item has its block, which looks whether it is built: two reads less to
-// wait for, 13.2 us against 14.2 for 697 tables of 817 regions.  Spilled keys go to the probe kernel one by one.  A table
-// some of whose keys found no room in a list is marked todo: the probe kernel then runs over all its keys, which
-// changes nothing for those stored here.
+// resident at once (ORDERED) gives the built ones in `items`, `built` of them, and the blocks take the next one from
+// a counter: a block for each of its regions, built or not, made an insert of 3 keys each into 4096 cleared tables of
+// 8192 take 46 us, 26 so.  Else each item has its block, which looks whether it is built: two reads less to wait for,
+// 13.2 us against 14.2 for 697 tables of 817 regions.  Spilled keys go to the probe kernel one by one.  A table some
+// of whose keys found no room in a list is marked todo: the probe kernel then runs over all its keys, which changes
+// nothing for those stored here.
 template <int KIND, bool AOS, bool ORDERED>
 __global__ void __launch_bounds__(kRegionThreads, kRegionBlocks)
 k_batch_build(const dview* views, const int64_t* offsets, const build_item* items, const int64_t* built,

@@ -1439,8 +1439,10 @@ next_epoch(Object* d, cudaStream_t s)
 }
 
 // Rings of at most this many slots keep their turn words from call to call and order every mixed launch by them: two
-// launches instead of four.  4096 mixed operations on a ring of 16384: 23 us in steady state and 19 us from empty
-// (30 and 28 us with the rebuild and the epoch as launches of their own).  Larger rings make the words for the
+// launches instead of four.  Neither route is better for every call there: 16384 mixed operations on a ring of 2^16
+// take 21 us by the turn words and 18 by the plan in steady state, 20 and 24 from empty, where pops follow the call's
+// own pushes; on a ring of 2^14 4096 of them take 21 and 18, 18 and 24.  Above the line the plan wins both as calls
+// grow: 2^18 operations 18 and 23 us, 25 and 39; 2^22 42 and 74, 80 and 155.  Larger rings make the words for the
 // launches that wait on them, those of more elements than the ring has slots.
 constexpr int64_t kTurnsKeptMax = int64_t{ 1 } << 16;
 
@@ -1591,9 +1593,9 @@ vector_call_ends(sg_vector* v, bool clear, cudaStream_t s)
     return SG_OK;
 }
 
-// Launches of at least this many elements reserve once per 8192 of them (k_vector_push_back): from here on they
-// have a block of that size for every SM.  2^20 elements (4 rows) 10.9 us, 2^21 (32 rows) 10.9 us, back to back with
-// the call that ends each (11.9 and 12.9 before).
+// Launches of at least this many elements reserve once per 8192 of them (k_vector_push_back, 32 rows), smaller ones
+// once per 1024 (4 rows): from here on there is a block of that size for every SM.  4-byte elements with flags, 4 and
+// 32 rows: 2^16 elements 7-9 and 9 us, 2^20 10 and 11, 2^21 13 and 11, 2^23 27 and 19, 2^24 46 and 31.
 constexpr int64_t kVecLargeTile = int64_t{ 1 } << 21;
 
 template <typename T, int ROWS>
