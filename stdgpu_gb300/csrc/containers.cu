@@ -1122,7 +1122,8 @@ k_deque_copy_out(const T* data, const deque_counters* c, int64_t cap, T* out)
     }
 }
 
-// Words of device memory into pinned host memory (read_words): size() of a vector or deque.
+// Up to 32 words of device memory into pinned host memory: sooner there than by a copy of a few bytes (size() of a
+// vector or deque).
 __global__ void
 k_read_words(const unsigned long long* src, unsigned long long* host, int words)
 {
@@ -1766,7 +1767,9 @@ sg_vector_size(sg_vector* v, void* stream, int64_t* out_size)
         return SG_ERR_BAD_ARG;
     }
     cudaStream_t s = as_stream(stream);
-    SG_CUDA_TRY(read_words(k_read_words, v->size, v->host, 1, s));
+    SG_CUDA_TRY(launch_early(k_read_words, 1, 32, s, reinterpret_cast<const unsigned long long*>(v->size),
+                             reinterpret_cast<unsigned long long*>(v->host), 1));
+    SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     long long x = *v->host;
     *out_size = x < 0 ? 0 : (x > v->capacity ? v->capacity : x);
@@ -2074,7 +2077,10 @@ sg_deque_size(sg_deque* d, void* stream, int64_t* out_size)
     }
     cudaStream_t s = as_stream(stream);
     static_assert(sizeof(deque_counters) % 8 == 0 && sizeof(deque_counters) <= 32 * 8, "one warp copies the counters");
-    SG_CUDA_TRY(read_words(k_read_words, d->counters, d->host, static_cast<int>(sizeof(deque_counters) / 8), s));
+    SG_CUDA_TRY(launch_early(k_read_words, 1, 32, s, reinterpret_cast<const unsigned long long*>(d->counters),
+                             reinterpret_cast<unsigned long long*>(d->host),
+                             static_cast<int>(sizeof(deque_counters) / 8)));
+    SG_LAUNCH_CHECK();
     SG_CUDA_TRY(cudaStreamSynchronize(s));
     const long long x = d->host->size;
     *out_size = x < 0 ? 0 : (x > d->capacity ? d->capacity : x);

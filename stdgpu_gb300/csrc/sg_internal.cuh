@@ -200,29 +200,6 @@ launch_early(void (*kernel)(Params...), int grid, int block, cudaStream_t s, Arg
     return launch_early_shared(kernel, grid, block, 0, s, args...);
 }
 
-// Up to 32 words of device memory into pinned host memory, for calls that then synchronise and read them there.
-// Behind other work of the stream a kernel's stores are there sooner than a copy of 64 bytes, which another engine
-// starts when the kernels are done: a pass of clear, insert, contains, erase and size() on a set of 2^20 keys took
-// 87.7 us, 90.7 with cudaMemcpyAsync.  On an idle stream the copy is sooner: size() 9.4 us, 10.3 by the kernel.
-template <typename Kernel>
-inline cudaError_t
-read_words(Kernel kernel, const void* src, void* host, int words, cudaStream_t s)
-{
-    const cudaError_t idle = cudaStreamQuery(s);
-    if (idle == cudaSuccess)
-    {
-        return cudaMemcpyAsync(host, src, static_cast<size_t>(words) * 8, cudaMemcpyDeviceToHost, s);
-    }
-    if (idle != cudaErrorNotReady)
-    {
-        return idle;
-    }
-    cudaGetLastError(); // "not ready" is an answer here
-    count_launch();
-    return launch_early(kernel, 1, 32, s, static_cast<const unsigned long long*>(src),
-                        static_cast<unsigned long long*>(host), words);
-}
-
 inline int
 grid_for(int64_t work_items, int items_per_block, int max_grid)
 {

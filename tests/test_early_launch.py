@@ -42,7 +42,6 @@ def test_every_early_launched_kernel_waits_first():
         code = _code(unit)
         early = set(re.findall(r"launch_early(?:_shared)?\(\s*(\w+)", code))
         early |= set(re.findall(r"cudaLaunchKernelEx\(&cfg, (\w+)", code))
-        early |= set(re.findall(r"read_words\((k_\w+)", code))
         for name in sorted(early - {"kernel"}):
             body = re.search(r"__launch_bounds__\([^{;]*\)?\s*" + name + r"\([^{;]*\)\s*\{(.*?)\n\}", code, re.S) or \
                 re.search(r"__global__[^{;]*\b" + name + r"\([^{;]*\)\s*\{(.*?)\n\}", code, re.S)
