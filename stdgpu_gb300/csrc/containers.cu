@@ -542,7 +542,9 @@ k_deque_rebuild_turns(unsigned* seq, const deque_counters* c, const sg_deque_syn
 
 // The launches after the plan: element i moves its element.  Its rank among the pushes (or pops) before it is its
 // tile's count, its warp's and its row's, so tickets follow the element order and a row's pushes and pops go to
-// consecutive slots.  Bound by the bytes: flag, value or popped value, slot and outcome, about 27 bytes an operation.
+// consecutive slots.  An operation moves flag, value or popped value, slot and outcome, 25 bytes: 422 MB in 105 us at
+// 2^24 operations, 0.6 of the measured copy rate, with 68 % of the issue slots taken; neither is full, since each load
+// waits for its rank, which waits for the flags.
 // kMoveFirst: pops of elements stored before the call, every outcome, and the pushes too when they meet no pop
 // at a slot (the other two launches then return at once); else kMovePush and kMoveLate follow, pushes
 // and then the pops of elements that the call pushed.
@@ -1323,8 +1325,10 @@ struct call_order
 };
 
 // Lives from before a call's first launch to after its last one.  Calls under stream capture are left to the order
-// of the graphs they go into.  It costs half a microsecond of the host's time a call, most of it for the event, and
-// nothing on the device: ten push_back and pop_front of 64 elements 67.2 us there with and without.
+// of the graphs they go into.  It costs half a microsecond of the host's time a call, most of it for the event; on the
+// device nothing before a launch_early (ten push_back and pop_front of 64 elements 67.2 us with and without) and a
+// microsecond or so before another kernel (a pass of 2^24 mixed operations, a pop and the caller's own kernels 285 us,
+// 286 with it).
 class ordered_call
 {
 public:

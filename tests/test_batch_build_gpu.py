@@ -1,8 +1,9 @@
-"""Batched inserts into tables that hold nothing, which are built in shared memory a region of probe groups at a
-time, at the sizes where that changes: tables of less than a block's groups, exactly one block's, several blocks.,
-than several blocks., regions than are built, too few keys to be built; keys crowded into the last groups of a
-region (they spill into the next one); tables filled to max_size() and past it; a batch with only some tables empty.
-Sizes, flags per key, contents and lookups equal the oracle's (the tables are independent)."""
+"""Batched inserts with flags per key into tables that hold nothing.  Tables of one region (256 probe groups) are then
+built in shared memory, larger ones take their keys through the probe kernel (without flags they are built from
+lists of their regions' keys: tests/test_batch_lists_gpu.py).  Tables of less than a region's groups, about
+one region's and several; too few keys to be built; keys crowded into a few neighbouring groups and around the table's
+end; tables filled to max_size() and past it; a batch with only some tables empty.  Sizes, flags per key, contents and
+lookups equal a dict's per table."""
 
 import numpy as np
 import pytest
@@ -93,11 +94,11 @@ def _keys_near(bits, groups, total_groups, first, last, count, rng):
 
 
 def test_keys_that_spill_over_a_regions_end():
-    """Three times as many keys as slots in the 8 groups before a cluster region's end: most go on into the next
-    region, through the probe kernel, and some tables of the batch are built as usual."""
+    """Three times as many keys as slots in 8 neighbouring groups: most go on into the next groups, through the probe
+    kernel (the inserts ask for flags), and a small table of the batch is built as usual."""
     cap = 80000
     g = sg.geometry_for(sg.KINDS[("u64", None)], cap)
-    assert g.num_groups > 4096 + 64  # more than one region of 8 x 512 groups
+    assert g.num_groups > 4096 + 64  # room behind the 4096 groups whose end is crowded
     bits = int(g.bucket_count).bit_length() - 1
     rng = np.random.default_rng(5)
     crowd = _keys_near(bits, None, g.num_groups, 4088, 4096, 3 * 8 * 16, rng)

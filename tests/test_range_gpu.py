@@ -1,6 +1,6 @@
 """device_range() and range_copy() against the slot image itself: the stored keys, mapped values and slot indices in
-slot order, then the out-of-band keys, at sizes around the tiles of the compaction (32 KB of slots), for empty, sparse
-and full tables and after erases.  src/stdgpu/impl/unordered_base_detail.cuh:136-208."""
+slot order, then the out-of-band keys, at sizes around the tiles of the compaction (1 or 2 KB of slots), for empty,
+sparse and full tables and after erases.  src/stdgpu/impl/unordered_base_detail.cuh:136-208."""
 
 import numpy as np
 import pytest
