@@ -356,6 +356,7 @@ SG_API sg_status sg_batch_contains(sg_table_batch* batch, const void* keys, cons
 SG_API sg_status sg_batch_sizes(sg_table_batch* batch, void* stream, int64_t* out_sizes);
 /* Device view of table t for native device calls. */
 SG_API sg_status sg_batch_view_of(const sg_table_batch* batch, int32_t table, sg_unordered_view* out);
+/* out_storage_bytes: of the tables' slots (their headers, locks and the calls' own arrays not counted). */
 SG_API sg_status sg_batch_info(const sg_table_batch* batch, int64_t* out_storage_bytes, int32_t* out_n_tables);
 
 /* ---------------- served request stream (no counterpart in the reference) ---------------- */

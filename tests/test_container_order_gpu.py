@@ -221,3 +221,80 @@ def test_clear_makes_a_container_whole_whatever_its_launch_words_hold(cap):
     assert d.size() == 2 * n and torch.equal(d.pop_front(n)[0], ids)
     sg.vector.destroyDeviceObject(v)
     sg.deque.destroyDeviceObject(d)
+
+
+@pytest.mark.parametrize("before", ["nothing", "kernel", "copy", "memset", "fork"])
+@pytest.mark.parametrize("n", [300, 5000, 1 << 20])
+def test_early_kernels_captured_behind(before, n):
+    """The first call of a captured graph behind each kind of work: nothing, a kernel, a copy, a memset, and a kernel
+    together with another stream's that was joined by an event."""
+    t = sg.unordered_map.createDeviceObject(2 * n, key="u64", mapped="u32")
+    v = sg.vector.createDeviceObject(n, elem_bytes=8)
+    d = sg.deque.createDeviceObject(4 * n, elem_bytes=8)
+    b = sg.table_batch.createDeviceObjects([4 * n] * 2, key="u64")
+    src = torch.arange(1, n + 1, device="cuda") * 0x9E3779B97F4A7C1
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    off = torch.tensor([0, n, n], device="cuda")
+    keys, other, spare = torch.empty_like(src), torch.empty_like(vals), torch.empty_like(src)
+    out = torch.empty((5, n), dtype=torch.int64, device="cuda")
+    side = torch.cuda.Stream()
+
+    def work(s):
+        """Writes keys and mapped values; the stream's last piece of work is of the kind asked for."""
+        if before == "nothing":
+            return
+        if before == "fork":
+            side.wait_stream(s)
+            with torch.cuda.stream(side):
+                keys.copy_(src)
+            torch.mul(vals, 1, out=other)
+            s.wait_stream(side)
+            return
+        torch.mul(src, 1, out=keys)
+        torch.mul(vals, 1, out=other)
+        if before == "copy":
+            keys.copy_(src)
+        if before == "memset":
+            spare.zero_()
+
+    def calls(s):
+        steps = [lambda: t.clear(stream=s), lambda: t.insert(keys, other, stream=s),
+                 lambda: out[0].copy_(t.find(keys, stream=s)[0]), lambda: t.erase(keys[: n // 2], stream=s),
+                 lambda: out[1].copy_(t.contains(keys, stream=s)),
+                 lambda: v.clear(stream=s), lambda: v.push_back(keys, stream=s),
+                 lambda: out[2].copy_(v.pop_back(n, stream=s)[0]),
+                 lambda: d.clear(stream=s), lambda: d.push_back(keys, stream=s),
+                 lambda: out[3].copy_(d.pop_front(n, stream=s)[0]),
+                 lambda: b.clear(stream=s), lambda: b.insert(keys, off, stream=s),
+                 lambda: out[4].copy_(b.contains(keys, off, stream=s))]
+        for step in steps:
+            work(s)
+            step()
+
+    keys.copy_(src)
+    other.copy_(vals)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        calls(s)  # warm-up
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        calls(torch.cuda.current_stream())
+    for _ in range(3):
+        if before != "nothing":
+            keys.zero_()
+            other.zero_()
+        out.fill_(-1)
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], vals.long())
+        assert not bool(out[1][: n // 2].any()) and bool((out[1][n // 2:] == 1).all())
+        assert torch.equal(out[2].sort().values, src.sort().values)
+        assert torch.equal(out[3], src) and bool((out[4] == 1).all())
+        assert t.size() == n - n // 2 and b.sizes().tolist() == [n, 0]
+    sg.unordered_map.destroyDeviceObject(t)
+    sg.vector.destroyDeviceObject(v)
+    sg.deque.destroyDeviceObject(d)
+    sg.table_batch.destroyDeviceObjects(b)
