@@ -112,32 +112,42 @@ region_insert(const region& r, uint32_t l, uint32_t rot, typename kind_consts<KI
     return kRegionRefused;
 }
 
-// The region as clear() leaves it: never-used slots, and erased markers at or above total_count.
+// The 16-byte unit whose first slot is s0 as clear() leaves it: never-used slots, and erased markers at or above
+// total_count.
+template <int KIND>
+SG_D uint4
+cleared_unit(const dview& t, uint32_t s0)
+{
+    using C = kind_consts<KIND>;
+    using K = typename C::K;
+    uint4 d = make_uint4(~0u, ~0u, ~0u, ~0u);
+    if (s0 + C::slots_per_lane > t.total)
+    {
+        char* bytes = reinterpret_cast<char*>(&d);
+        for (int s = 0; s < C::slots_per_lane; ++s)
+        {
+            if (s0 + s >= t.total)
+            {
+                *reinterpret_cast<K*>(bytes + s * C::slot_bytes) = C::tomb_key;
+            }
+        }
+    }
+    return d;
+}
+
+// The region as clear() leaves it.
 template <int KIND>
 SG_D void
 region_start(const dview& t, const region& r)
 {
     using C = kind_consts<KIND>;
-    using K = typename C::K;
     uint4* const smem = reinterpret_cast<uint4*>(r.smem);
     const uint32_t first_slot = r.first * C::slots_per_group;
     const bool whole_slots = first_slot + r.count * C::slots_per_group <= t.total;
     for (uint32_t u = threadIdx.x; u < r.count * (kGroupBytes / 16); u += blockDim.x)
     {
-        uint4 d = make_uint4(~0u, ~0u, ~0u, ~0u);
-        const uint32_t s0 = first_slot + u * C::slots_per_lane;
-        if (!whole_slots && s0 + C::slots_per_lane > t.total)
-        {
-            char* bytes = reinterpret_cast<char*>(&d);
-            for (int s = 0; s < C::slots_per_lane; ++s)
-            {
-                if (s0 + s >= t.total)
-                {
-                    *reinterpret_cast<K*>(bytes + s * C::slot_bytes) = C::tomb_key;
-                }
-            }
-        }
-        smem[u] = d;
+        smem[u] = whole_slots ? make_uint4(~0u, ~0u, ~0u, ~0u)
+                              : cleared_unit<KIND>(t, first_slot + u * C::slots_per_lane);
     }
 }
 

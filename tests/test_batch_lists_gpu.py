@@ -250,3 +250,54 @@ def test_a_batch_makes_few_device_allocations(cap):
     assert sg.live_device_allocations() - before <= 7
     sg.table_batch.destroyDeviceObjects(b)
     assert sg.live_device_allocations() == before
+
+
+@pytest.mark.parametrize("kind,size", [(k, "regions") for k in KINDS] + [
+    (O.SET_U64, "many"), (O.SET_U32, "no regions"), (O.MAP_U64_U32, "no regions")])
+def test_clear_leaves_every_slot_and_header_as_new(kind, size):
+    """One launch over the regions clears a batch of up to 256 MB; a fill and a launch a larger one (ten tables of the
+    most regions) and one with a table that has no regions."""
+    most = _cap_with_groups(kind, REGIONS * REGION + 1)
+    caps = {"regions": [_cap_with_groups(kind, 5 * REGION + 3), 1, 300, _cap_with_groups(kind, REGION + 1), 77],
+            "many": [most - 1] * 10 + [5], "no regions": [100, most, 2000]}[size]
+    arena = sum(_geometry(kind, c).num_groups + 1 for c in caps) * 128
+    assert (arena > 1 << 28) == (size == "many")
+    ks, ms = _names(kind)
+    kd, vd = np.dtype(O.KEY_DTYPE[kind]), O.VAL_DTYPE[kind]
+    top = np.iinfo(kd).max
+    rng = np.random.default_rng(kind)
+    keys = [np.concatenate([_random(kind, min(c, 20000), rng), np.array([top, top - 1], kd)]) for c in caps]
+    flat = np.concatenate(keys)
+    off = np.concatenate([[0], np.cumsum([len(k) for k in keys])]).astype(np.int64)
+    vals = _value(kind, flat)
+    b = sg.table_batch.createDeviceObjects(caps, key=ks, mapped=ms)
+    for _ in range(2):
+        b.insert(dev(flat), dev(off), dev(vals) if vals is not None else None)
+        b.erase(dev(flat[: len(keys[0]) // 2]), dev(np.minimum(off, len(keys[0]) // 2)))
+        b.clear()
+        for t in range(len(caps)):
+            assert _stored(b, kind, t) == {}, t
+            v = b.view(t)
+            raw = torch.as_tensor(_DeviceArray(v.slots, (int(v.num_groups) + 1) * 16, 8), device="cuda").cpu().numpy()
+            rows = np.ascontiguousarray(raw.view(np.uint8).reshape(-1, SLOT[kind])[:, : kd.itemsize]).view(kd).ravel()
+            assert (rows[: int(v.total_count)] == top).all(), t
+            assert (rows[int(v.num_groups) * (128 // SLOT[kind]):] == top).all(), t
+            assert not torch.as_tensor(_DeviceArray(v.header, 8, 8), device="cuda").any().item(), t
+        assert not b.contains(dev(flat), dev(off)).any().item() and b.sizes().sum() == 0
+    sg.table_batch.destroyDeviceObjects(b)
+
+
+def test_clearing_a_small_batch_costs_about_what_clearing_a_table_costs():
+    """One launch either way: a fill of the arena and a launch behind it took a small batch several times as long."""
+    def each(clear):
+        def calls():
+            for _ in range(20):
+                clear()
+        return _microseconds(calls, lambda: torch.cuda._sleep(2_000_000)) / 20  # queued behind a sleeping kernel
+
+    b = sg.table_batch.createDeviceObjects([1000] * 64, key="u64")
+    t = sg.unordered_set.createDeviceObject(1000, key="u64")
+    batch, table = each(b.clear), each(t.clear)
+    sg.table_batch.destroyDeviceObjects(b)
+    sg.unordered_set.destroyDeviceObject(t)
+    assert batch < 3 * table, (batch, table)
